@@ -560,16 +560,20 @@ def gpu_object(galsim, p):
 DRAW_STEP_DRAM_READ = 37439488
 DRAW_STEP_DRAM_WRITE = 63917824
 DRAW_STEP_STORES = 285221408
-# FP64 pipe and issue utilisation of the Sersic table kernel (ncu --set full, round 5 of a
-# 4096-table build; profiles/sersic_nodes_pair_kernel_4096_tables.md)
-TABLES_FP64_PIPE = 0.446
-TABLES_ISSUE_ACTIVE = 0.747
+# FP64 pipe and issue utilisation of the Sersic table kernel (ncu, a 4096-table build;
+# profiles/sersic_table_kernel_4096_tables.md)
+TABLES_FP64_PIPE = 0.276
+TABLES_ISSUE_ACTIVE = 0.340
+
+
+TABLE_BUILD_LAUNCHES = 2     # of an untruncated Sersic table build: set-up and tables
 
 
 def table_build_launches(n_values, gsp_kvalue_accuracy=1e-5, table_spacing=1.):
-    """Kernel launches of one Sersic table build (gsb_sersic_tables_build): setup, scan init,
-    one (nodes, scan) pair per round of 64 ln k nodes over the table stride (kTableRound in
-    csrc/gsb_tables.cu), and the finalize.
+    """Kernel launches of a Sersic table build (gsb_sersic_tables_build) with truncated profiles:
+    setup, scan init, one (nodes, scan) pair per round of 64 ln k nodes over the table stride
+    (kTableRound in csrc/gsb_tables.cu), and the tables.  (An untruncated build has no rounds:
+    TABLE_BUILD_LAUNCHES.)
     The stride is the node count of the largest n (sersic_stride in csrc/gsb_tables.cu)."""
     nmax = float(np.max(n_values))
     kderiv6 = math.exp(math.lgamma(8. * nmax) - math.lgamma(2. * nmax)) / 2304.
@@ -1028,12 +1032,12 @@ def run_gpu(args):
         torch.cuda.synchronize(dev)
         t_ms = ts.elapsed_time(te) / reps
         tables_roof = {'bound': 'fp64 issue', 'unit': 'fraction of the FP64 pipe',
-                       'kernel': 'sersic_nodes_pair_kernel (+ scan, setup, finalize): %d FP64 Sersic FT tables'
+                       'kernel': 'sersic_table_kernel (+ setup): %d FP64 Sersic FT tables'
                                  % len(prog.sersic_n),
                        'kernel_ms': t_ms, 'step_share': t_ms / ms,
                        'frac': TABLES_FP64_PIPE, 'issue_active': TABLES_ISSUE_ACTIVE,
-                       'frac_source': 'ncu --set full, round 5 of a 4096-table build '
-                                      '(profiles/sersic_nodes_pair_kernel_4096_tables.md)'}
+                       'frac_source': 'ncu, a 4096-table build '
+                                      '(profiles/sersic_table_kernel_4096_tables.md)'}
 
     # e2e through the public API: host parameters -> draw_batch -> host pixels.  The warm-up
     # steps make the one-time allocations (the page-locked read-back buffer) before timing.
@@ -1167,7 +1171,7 @@ def run_gpu(args):
             'roofline_tables': tables_roof,
             # per step: the Sersic table build, one leaf-prepare launch, the leaf gather into
             # bucket order, one fused draw per FFT-size bucket and the added-flux scatter
-            'gpu_launches': int(args.steps * (table_build_launches(params[:, 0]) + 3 + nb)),
+            'gpu_launches': int(args.steps * (TABLE_BUILD_LAUNCHES + 3 + nb)),
             'fp32_error_vs_reference': fp32_err,
             'mixed_batch': mixed,
             'large_stamps': large,

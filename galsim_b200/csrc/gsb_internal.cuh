@@ -215,8 +215,8 @@ struct gsb_tables {
     int stride = 0;               // nodes per slot
     double* d_header = nullptr;   // count * kSersicHeader
     double4* d_node = nullptr;    // count * stride
-    double* d_val = nullptr;      // scratch: count * stride Hankel values
-    void* d_scan = nullptr;       // scratch: per-slot state of the table's stopping scan
+    double* d_val = nullptr;      // scratch: count * stride Hankel values (truncated tables)
+    void* d_scan = nullptr;       // scratch: per-slot state of the truncated tables' stopping scan
     double* d_n = nullptr;        // Sersic indices of the slots
     double* d_trunc = nullptr;    // truncation radius / r0 of the slots (when any is truncated)
     size_t cap_trunc = 0;
@@ -226,12 +226,7 @@ struct gsb_tables {
     bool has_dn = false;
     double* d_dheader = nullptr;  // count * kSersicDHeader
     double4* d_dnode = nullptr;   // count * stride
-    double* d_dval = nullptr;     // scratch: count * stride d/dn Hankel values
     size_t cap_dn_slots = 0, cap_dn_nodes = 0;
-    // the device part of the last Sersic build as a CUDA graph, and what it was captured for
-    cudaGraphExec_t sersic_exec = nullptr;
-    unsigned char sersic_key[256] = {};
-    cudaStream_t capture_stream = nullptr;
     // truncated Moffat slots (gsb_moffat_tables_build)
     int moffat_count = 0;
     int moffat_stride = 0;            // nodes per slot

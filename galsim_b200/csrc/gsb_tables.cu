@@ -4,13 +4,15 @@
 //                zeros of J0, built once per device (gsb_init).
 //   hankel_*     the reference's adaptive Hankel transform (src/math/Hankel.cpp:179-249),
 //                one warp per transform, terms summed 32 at a time with a warp prefix sum.
+//   ogata_log_*  the quadrature's levels resampled onto a uniform grid in ln x, so that a table
+//                of transforms on a uniform ln k grid is a correlation (sersic_table_kernel).
 //   sersic_*     SersicInfo (src/SBSersic.cpp:301-667): HLR and missing-flux radii by
 //                Brent, the ln k table of the Hankel transform, its high-k fit and maxk,
 //                and the natural cubic spline (src/Table.cpp:634-686).
 //   kolmogorov_* KolmogorovInfo stepk (src/SBKolmogorov.cpp:338-420).
 //   prepare_*    per-leaf derived constants and stepk / maxk.
 #include <algorithm>
-#include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "gsb_internal.cuh"
@@ -21,9 +23,9 @@ namespace gsb {
 namespace {
 
 constexpr int kLevMin = 5;
-constexpr int kMaxRounds = 128;      // rounds of ln k nodes per table build (status flags)
-// ln k nodes per table and round: a table's nodes past its stopping point are integrated only
-// up to the end of the round in which its scan stops (even: the nodes go in pairs)
+constexpr int kMaxRounds = 128;      // rounds of ln k nodes per truncated table build (status flags)
+// ln k nodes per truncated table and round: a table's nodes past its stopping point are integrated
+// only up to the end of the round in which its scan stops
 constexpr int kTableRound = 64;
 constexpr int kLevMax = 20;
 constexpr long long kNroot = 1000000;
@@ -52,11 +54,6 @@ __device__ __forceinline__ double exp_tab256_core(double x, const double* tab)
     p = fma(p, r, 1.);
     const double v = tab[j] * p;
     return __hiloint2double(__double2hiint(v) + (m << 20), __double2loint(v));
-}
-
-__device__ __forceinline__ double exp_tab256_neg(double x, const double* tab)
-{
-    return exp_tab256_core(fmax(x, -708.), tab);
 }
 
 __global__ void ogata_root_kernel(double2* root, long long nroot)
@@ -154,140 +151,116 @@ __device__ double warp_hankel(const OgataTables& og, const F& f, double k, doubl
     return ans1;
 }
 
-// The Sersic integrand exp(-r^(1/n)) is evaluated inline by the node-pair quadrature below, with
-// log r = log x_i - log k; its n-derivative along the table's moving grid (GSB_TABLES_DN): the
-// quadrature sum T(k) = sum_j w_j f(x_j / k) has dT/dn along k = k(n) with d ln k / dn = c equal
-// to sum_j w_j [df/dn - c r df/dr](x_j / k); df/dn = f u ln r / n^2, r df/dr = -f u / n,
-// u = r^(1/n).
+// The quadrature levels on a uniform grid in ln x.  A level-l sum for a radial profile whose
+// transform is wanted on a uniform ln k grid,
+//     S_l(k) = sum_i w_i f(x_i / k) = sum_i w_i G(ln x_i - ln k),     G(y) = f(e^y),
+// samples a smooth G at the scattered ln x_i.  With G band-limited well below pi / h, its value
+// between the points of a grid of spacing h is the windowed-sinc sum
+//     G(u h) = sum_q phi(u - q) G(q h),   phi(t) = sinc(t) exp(beta (sqrt(1 - (2 t / W)^2) - 1)),
+// so the nodes can be spread onto the grid once and for all, A_l[q] = sum_i w_i phi(ln x_i / h - q),
+// and S_l(k) = sum_q A_l[q] G(q h - ln k): one array of G per profile serves every ln k on the
+// grid and every level, and a term costs one multiply-add instead of an exponential.  The A_l
+// depend on the spacing alone.  Against the scattered sums (Sersic n from 0.3 to 6.2, every
+// level): 1e-15 of the flux at n <= 0.5, 5e-12 where the level's own cancellation is largest.
+constexpr int kLogW = 48;                 // window width in grid points
+constexpr double kLogBeta = 34.;
+constexpr double kLogMaxStep = 0.0333;    // largest grid spacing (the spectrum of G at n = 0.3 is
+                                          // 1e-19 at pi / h; larger n decays faster)
+constexpr int kLogLev0 = kLevMin;
+constexpr int kLogLevels = 57;            // levels 5 .. 61: all the halving can reach
 
-// Two adjacent ln k nodes of one Sersic table in one warp (k0 < k1 = k0 e^dlogk): the terms
-// of both sums at one level share the node load (log x_i, w_i) and the inner exponential,
-//   u0 = (x_i / k0)^(1/n) = exp((log x_i - log k0) / n),   u1 = u0 * exp((log k0 - log k1) / n),
-// so a pair of terms costs three exponentials instead of four, and each lane carries two
-// independent outer exponentials.  Each sum keeps warp_ogata_sum's stopping rule on its own
-// running total (the loop runs until both have stopped; a stopped or inactive sum skips its
-// outer exponential, a warp-uniform branch).  Node 0's terms are warp_ogata_sum's; node 1's
-// u differs from a direct exponential by the rounding of one product (~1e-16 relative), the
-// size of the exponential's own rounding.  The inner argument is bounded (|log x_i - log k|
-// / n < 100 for the tabulated nodes and the tables' k range), so it takes no range test.
-// (Groups of four nodes per warp share more, but their state no longer fits the 64 registers
-// that four 256-thread blocks per SM allow, and they measured slower.)
-// DN: also the d/dn integrand on the same nodes, f u / n (log r / n + c) with c = dfront/dn (its
-// sums stop where the value sums stop, the halving follows the values), returned through dout.
-template <bool TAB, bool DN = false>
-__device__ __forceinline__ double2 warp_ogata_sum_pair(const OgataTables& og, double invn, double c1,
-                                                       double logk0, double logk1, int lev, bool act0,
-                                                       bool act1, const double* etab, double dnc = 0.,
-                                                       double2* dout = nullptr)
+struct OgataLog {
+    double h;
+    const double* a;
+    int qmin[kLogLevels], len[kLogLevels], off[kLogLevels];
+};
+
+// A_l[q], one block per grid point q: the nodes within W / 2 grid points of it (the node list is
+// ascending in ln x).
+__global__ void __launch_bounds__(256) ogata_log_kernel(const double2* __restrict__ xw, int n, double h, int qmin,
+                                                        double* __restrict__ a)
 {
-    const int lane = threadIdx.x & 31;
-    const double h = ldexp(1.0, -lev);
-    const int nmax = (int)fmin(kPi / h, 1e6);
-    const double2* xw = TAB ? og.xw + og.off[lev - og.lev_min] : nullptr;
-    double acc0 = 0., acc1 = 0., th0 = 0., th1 = 0.;
-    double dacc0 = 0., dacc1 = 0.;
-    int chunk = 0;
-    for (int base = 0; base < nmax; base += 32, ++chunk) {
-        const int i = base + lane;
-        const bool valid = i < nmax;
-        double s0 = 0., s1 = 0., ds0 = 0., ds1 = 0.;
-        if (valid) {
-            const double2 n = TAB ? xw[i] : ogata_node(og.root, h, i);
-            const double lr0 = n.x - logk0;
-            const double u0 = exp_tab256_core(lr0 * invn, etab);
-            if (act0) {
-                const double f = exp_tab256_neg(-u0, etab);
-                s0 = n.y * f;
-                if (DN) ds0 = s0 * u0 * invn * (lr0 * invn + dnc);
-            }
-            if (act1) {
-                const double u1 = u0 * c1;
-                const double f = exp_tab256_neg(-u1, etab);
-                s1 = n.y * f;
-                if (DN) ds1 = s1 * u1 * invn * ((n.x - logk1) * invn + dnc);
-            }
+    const int q = qmin + int(blockIdx.x);
+    auto lower = [&](double u) {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (xw[mid].x / h < u) lo = mid + 1; else hi = mid;
         }
-        if (act0) {
-            const unsigned m0 = __ballot_sync(0xffffffffu, valid && fabs(s0) < th0);
-            if (m0) {
-                const bool in = lane <= __ffs(m0) - 1;
-                acc0 = warp_total(acc0 + (in ? s0 : 0.));
-                if (DN) dacc0 = warp_total(dacc0 + (in ? ds0 : 0.));
-                act0 = false;
-            } else {
-                acc0 += s0;
-                if (DN) dacc0 += ds0;
-            }
-        }
-        if (act1) {
-            const unsigned m1 = __ballot_sync(0xffffffffu, valid && fabs(s1) < th1);
-            if (m1) {
-                const bool in = lane <= __ffs(m1) - 1;
-                acc1 = warp_total(acc1 + (in ? s1 : 0.));
-                if (DN) dacc1 = warp_total(dacc1 + (in ? ds1 : 0.));
-                act1 = false;
-            } else {
-                acc1 += s1;
-                if (DN) dacc1 += ds1;
-            }
-        }
-        if (!(act0 || act1)) break;
-        if (chunk < kEagerChunks || (chunk % kLazyChunks) == kLazyChunks - 1) {
-            if (act0) th0 = 1e-15 * fabs(warp_total(acc0));
-            if (act1) th1 = 1e-15 * fabs(warp_total(acc1));
-        }
+        return lo;
+    };
+    const int i0 = lower(q - 0.5 * kLogW), i1 = lower(q + 0.5 * kLogW);
+    double sum = 0.;
+    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const double t = xw[i].x / h - q;
+        const double v = 2. * t / kLogW;
+        const double s = fabs(t) < 1e-9 ? 1. : sinpi(t) / (kPi * t);
+        sum += xw[i].y * s * exp(kLogBeta * (sqrt(fmax(1. - v * v, 0.)) - 1.));
     }
-    // sums that ran to nmax without stopping
-    if (act0) { acc0 = warp_total(acc0); if (DN) dacc0 = warp_total(dacc0); }
-    if (act1) { acc1 = warp_total(acc1); if (DN) dacc1 = warp_total(dacc1); }
-    const double k0 = exp(logk0), k1 = exp(logk1);
-    if (DN) *dout = make_double2(dacc0 / (k0 * k0), dacc1 / (k1 * k1));
-    return make_double2(acc0 / (k0 * k0), acc1 / (k1 * k1));
+    sum = warp_total(sum);
+    __shared__ double part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) sum += part[w];
+        a[blockIdx.x] = sum;
+    }
 }
 
-// The reference's halving and stopping rule (AdaptiveHankelIntegrator::integrate,
-// Hankel.cpp:179-219) for both nodes of the pair, advanced over one common level index L:
-// node j starts at its own level s_j (h0 = 1/32 halved while h0 > 100 k_j; s_1 <= s_0 since
-// k_1 > k_0), takes the sum at every level from s_j on (ans0 <- ans1, ans1 <- sum(L)) and
-// stops at the first level where the reference's test passes; a node that has stopped, or has
-// not started, does not contribute to the level's sums.  The running answers live in this
-// warp's shared-memory slot `a` (ans0, ans1 of node 0, then of node 1) rather than in
-// registers across the term loop.  has1 = false integrates node 0 alone.
-template <bool DN = false>
-__device__ double2 warp_hankel_pair(const OgataTables& og, double invn, double logk0, double logk1,
-                                    bool has1, double relerr, double abserr, int* status, double* a,
-                                    const double* etab, double dnc = 0.)
+// The Sersic profile and its n-derivative along the table's moving grid (GSB_TABLES_DN) at
+// y = ln(x / k):  f = exp(-u), u = e^(y/n);  the sum T(k) = sum_j w_j f(x_j / k) has dT/dn along
+// k = k(n) with d ln k / dn = c equal to sum_j w_j [df/dn - c r df/dr](x_j / k), and
+// df/dn = f u ln r / n^2, r df/dr = -f u / n.
+__device__ __forceinline__ double2 sersic_sample(double y, double invn, double dnc)
 {
-    const int lane = threadIdx.x & 31;
-    const double k0 = exp(logk0), k1 = exp(logk1);
-    int s0 = 5, s1 = 5;
-    for (double h0 = 1. / 32.; h0 > 100. * k0 && s0 < 60; h0 *= 0.5) ++s0;
-    for (double h0 = 1. / 32.; h0 > 100. * k1 && s1 < 60; h0 *= 0.5) ++s1;
-    const double c1 = exp((logk0 - logk1) * invn);
-    auto more = [&](double x0, double x1) {
-        const double err = fabs(x1 - x0);
-        return (err > relerr * x1 && (err > abserr || fabs(x1) > 2. * fabs(x0))) || x1 == 0.;
-    };
-    bool run0 = true, run1 = has1;
-    for (int L = has1 ? min(s0, s1) : s0; run0 || run1; ++L) {
-        // the reference halves until its level counter passes 60: the last sum is at 61
-        if (L > 61) { if (status) *status = 1; break; }
-        const bool g0 = run0 && L >= s0, g1 = run1 && L >= s1;
-        double2 d = make_double2(0., 0.);
-        const double2 r = (L >= og.lev_min && L <= og.lev_max)
-                              ? warp_ogata_sum_pair<true, DN>(og, invn, c1, logk0, logk1, L, g0, g1, etab, dnc, &d)
-                              : warp_ogata_sum_pair<false, DN>(og, invn, c1, logk0, logk1, L, g0, g1, etab, dnc, &d);
-        __syncwarp();
-        if (lane == 0) {
-            if (g0) { a[0] = a[1]; a[1] = r.x; if (DN) a[5] = d.x; }
-            if (g1) { a[2] = a[3]; a[3] = r.y; if (DN) a[7] = d.y; }
+    const double v = y * invn;
+    const double u = exp(fmin(v, 7.));
+    const double f = exp(-u);
+    return make_double2(f, f * u * invn * (v + dnc));
+}
+
+// acc[r] += sum_q A[q] g[q - p (m + r)] (and the same with gd for DN), q = qlo .. qhi; g points at
+// the sample of d = 0, and samples from top on are 0.  With p = 1 the array is padded with them and the R nodes of a thread share each sample through a window in
+// registers: one shared-memory read (lane stride R doubles, R odd: no bank conflicts) and one
+// broadcast read feed R multiply-adds.
+template <int R, bool DN, bool P1>
+__device__ __forceinline__ void correlate(const double* __restrict__ A, int qlo, int qhi, const double* g,
+                                          const double* gd, int m, int p, int top, double (&acc)[R],
+                                          double (&dacc)[R])
+{
+    double w[R], wd[R];
+    if (P1) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+            w[r] = g[qlo - m - r];
+            if (DN) wd[r] = gd[qlo - m - r];
         }
-        __syncwarp();
-        if (g0 && L > s0) run0 = more(a[0], a[1]);
-        if (g1 && L > s1) run1 = more(a[2], a[3]);
     }
-    __syncwarp();
-    return make_double2(a[1], a[3]);
+#pragma unroll 6
+    for (int q = qlo; q <= qhi; ++q) {
+        const double a = A[q];
+        if (P1) {
+            w[0] = g[q - m];
+            if (DN) wd[0] = gd[q - m];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                acc[r] = fma(a, w[r], acc[r]);
+                if (DN) dacc[r] = fma(a, wd[r], dacc[r]);
+            }
+#pragma unroll
+            for (int r = R - 1; r > 0; --r) {
+                w[r] = w[r - 1];
+                if (DN) wd[r] = wd[r - 1];
+            }
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int d = min(q - p * (m + r), top);
+                acc[r] = fma(a, g[d], acc[r]);
+                if (DN) dacc[r] = fma(a, gd[d], dacc[r]);
+            }
+        }
+    }
 }
 
 // Truncated Hankel transform (math::hankel_trunc, src/math/Hankel.cpp:249-255) of a radial
@@ -448,91 +421,107 @@ __global__ void sersic_truncation_kernel(const double* in, int count, double* ou
     out[2 * i + 1] = gamma_p(2. * n, pow(trunc / r0, 1. / n));
 }
 
-__global__ void sersic_setup_kernel(const double* n_arr, const double* trunc_arr, int count, gsb_gsparams gsp,
-                                    double* header, int stride, double* dheader)
+// Per-table constants.  A block holds 32 tables and three warps, one per independent part (the
+// low-k series and grid, the half-light radius, the missing-flux radius):
+// each part is a chain of dependent FP64 divisions, so taking them side by side rather than in
+// one thread sets the kernel's time (a few hundred tables: 65-100 us in one thread each).
+__global__ void __launch_bounds__(96) sersic_setup_kernel(const double* n_arr, const double* trunc_arr, int count,
+                                                           gsb_gsparams gsp, double* header, int stride,
+                                                           double* dheader)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= count) return;
-    double* H = header + (size_t)s * kSersicHeader;
-    const double n = n_arr[s];
-    const double trunc = trunc_arr ? trunc_arr[s] : 0.;      // in units of r0
+    __shared__ int bad_b[32], bad_r[32];
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int s = blockIdx.x * 32 + lane;
+    const bool live = s < count;
+    double* H = header + (size_t)(live ? s : 0) * kSersicHeader;
+    const double n = live ? n_arr[s] : 1.;
+    const double trunc = live && trunc_arr ? trunc_arr[s] : 0.;      // in units of r0
     const double gamma2n = tgamma(2. * n);
-    double gamma4n = tgamma(4. * n);
-    double gamma6n = tgamma(6. * n);
-    double gamma8n = tgamma(8. * n);
     // truncated profiles (SBSersic.cpp:332-352, 393-424): the flux fraction inside trunc and the
     // moments of the truncated profile
-    double ff = 1.;
-    if (trunc > 0.) {
-        const double z = pow(trunc, 1. / n);
-        ff = gamma_p(2. * n, z);
-        gamma4n *= gamma_p(4. * n, z);
-        gamma6n *= gamma_p(6. * n, z);
-        gamma8n *= gamma_p(8. * n, z);
+    const double z = trunc > 0. ? pow(trunc, 1. / n) : 0.;
+    const double ff = trunc > 0. ? gamma_p(2. * n, z) : 1.;
+    if (live && part == 0) {
+        double gamma4n = tgamma(4. * n);
+        double gamma6n = tgamma(6. * n);
+        double gamma8n = tgamma(8. * n);
+        if (trunc > 0.) {
+            gamma4n *= gamma_p(4. * n, z);
+            gamma6n *= gamma_p(6. * n, z);
+            gamma8n *= gamma_p(8. * n, z);
+        }
+        // buildFT low-k series (SBSersic.cpp:386-424)
+        const double kderiv2 = -gamma4n / (4. * gamma2n) / ff;
+        const double kderiv4 = gamma6n / (64. * gamma2n) / ff;
+        const double kderiv6 = gamma8n / (2304. * gamma2n) / ff;
+        const double kmin = pow(gsp.kvalue_accuracy / kderiv6, 1. / 6.);
+        const double dlogk = gsp.table_spacing * sqrt(sqrt(gsp.kvalue_accuracy / 10.));
+        int ncand = 0;
+        const double logk_end = log(500.);
+        for (double logk = log(kmin) - 0.001; logk < logk_end && ncand < stride; logk += dlogk)
+            ++ncand;
+        H[kSH_N] = n;
+        H[kSH_NUSED] = 0;
+        H[kSH_FRONT] = log(kmin) - 0.001;
+        H[kSH_DA] = dlogk;
+        H[kSH_KSQMIN] = kmin * kmin;
+        H[kSH_KSQMAX] = 0.;
+        H[kSH_KD2] = kderiv2;
+        H[kSH_KD4] = kderiv4;
+        H[kSH_HIGHA] = 0.;
+        H[kSH_HIGHB] = 0.;
+        H[kSH_MAXK] = kmin;
+        H[kSH_DLOGK] = dlogk;
+        H[kSH_NCAND] = ncand;
+        H[kSH_TRUNC] = trunc;
+        H[kSH_FLUXFRAC] = ff;
+        if (dheader) {
+            // d/dn of the low-k coefficients (ratios of Gamma functions)
+            double* D = dheader + (size_t)s * kSersicDHeader;
+            const double psi2 = digamma(2. * n);
+            D[kSD_DKD2] = kderiv2 * (4. * digamma(4. * n) - 2. * psi2);
+            D[kSD_DKD4] = kderiv4 * (6. * digamma(6. * n) - 2. * psi2);
+            D[kSD_DHIGHA] = 0.;
+            D[kSD_DHIGHB] = 0.;
+            // front = ln k_min - 0.001 with k_min = (kvalue_accuracy / kderiv6)^(1/6)
+            D[kSD_DFRONT] = -(8. * digamma(8. * n) - 2. * psi2) / 6.;
+        }
+    } else if (part == 1) {
+        const RootResult rb = sersic_b(n, gamma2n, ff);
+        bad_b[lane] = !rb.ok;
+        if (live) {
+            const double b = rb.x;
+            H[kSH_RE] = pow(b, n);
+            if (dheader) {
+                // d ln(r_e / r0) / dn, r_e = b^n: db/dn from P(2n, b) = 1/2 by implicit differentiation
+                const double dPdb = exp(-b + (2. * n - 1.) * log(b) - lgamma(2. * n));
+                const double dbdn = -2. * gamma_p_da(2. * n, b) / dPdb;
+                dheader[(size_t)s * kSersicDHeader + kSD_DLNRE] = log(b) + n * dbdn / b;
+            }
+        }
+    } else if (part == 2) {
+        // stepK (SBSersic.cpp:304-318): the untruncated missing-flux radius (its lower bracket falls
+        // back to the profile's own b, :589-592), capped at trunc
+        double b = 0.;
+        if (-log(gsp.folding_threshold * gamma2n) < 0.) b = sersic_b(n, gamma2n, ff).x;
+        const RootResult rr = sersic_missing_flux_radius(n, gamma2n, b, gsp.folding_threshold);
+        bad_r[lane] = !rr.ok;
+        double R = rr.x;
+        if (trunc > 0. && trunc < R) R = trunc;
+        R = fmax(R, gsp.stepk_minimum_hlr);
+        if (live) H[kSH_STEPK] = kPi / R;
     }
-    // buildFT low-k series (SBSersic.cpp:386-424)
-    const double kderiv2 = -gamma4n / (4. * gamma2n) / ff;
-    const double kderiv4 = gamma6n / (64. * gamma2n) / ff;
-    const double kderiv6 = gamma8n / (2304. * gamma2n) / ff;
-    const double kmin = pow(gsp.kvalue_accuracy / kderiv6, 1. / 6.);
-    const double dlogk = gsp.table_spacing * sqrt(sqrt(gsp.kvalue_accuracy / 10.));
-    int ncand = 0;
-    const double logk_end = log(500.);
-    for (double logk = log(kmin) - 0.001; logk < logk_end && ncand < stride; logk += dlogk)
-        ++ncand;
-    int status = 0;
-    RootResult rb = sersic_b(n, gamma2n, ff);
-    if (!rb.ok) status = 2;
-    const double b = rb.x;
-    // stepK (SBSersic.cpp:304-318): the untruncated missing-flux radius (its lower bracket falls
-    // back to the profile's own b, :589-592), capped at trunc
-    RootResult rr = sersic_missing_flux_radius(n, gamma2n, b, gsp.folding_threshold);
-    if (!rr.ok) status = 3;
-    double R = rr.x;
-    if (trunc > 0. && trunc < R) R = trunc;
-    R = fmax(R, gsp.stepk_minimum_hlr);
-    H[kSH_N] = n;
-    H[kSH_NUSED] = 0;
-    H[kSH_FRONT] = log(kmin) - 0.001;
-    H[kSH_DA] = dlogk;
-    H[kSH_KSQMIN] = kmin * kmin;
-    H[kSH_KSQMAX] = 0.;
-    H[kSH_KD2] = kderiv2;
-    H[kSH_KD4] = kderiv4;
-    H[kSH_HIGHA] = 0.;
-    H[kSH_HIGHB] = 0.;
-    H[kSH_MAXK] = kmin;
-    H[kSH_STEPK] = kPi / R;
-    H[kSH_RE] = pow(b, n);
-    H[kSH_DLOGK] = dlogk;
-    H[kSH_NCAND] = ncand;
-    H[kSH_STATUS] = status;
-    H[kSH_TRUNC] = trunc;
-    H[kSH_FLUXFRAC] = ff;
-    if (dheader) {
-        // d/dn of the low-k coefficients (ratios of Gamma functions) and of ln(r_e / r0) =
-        // n ln b, with db/dn from P(2n, b) = 1/2 by implicit differentiation.
-        double* D = dheader + (size_t)s * kSersicDHeader;
-        const double psi2 = digamma(2. * n);
-        D[kSD_DKD2] = kderiv2 * (4. * digamma(4. * n) - 2. * psi2);
-        D[kSD_DKD4] = kderiv4 * (6. * digamma(6. * n) - 2. * psi2);
-        D[kSD_DHIGHA] = 0.;
-        D[kSD_DHIGHB] = 0.;
-        // front = ln k_min - 0.001 with k_min = (kvalue_accuracy / kderiv6)^(1/6)
-        D[kSD_DFRONT] = -(8. * digamma(8. * n) - 2. * psi2) / 6.;
-        const double dPdb = exp(-b + (2. * n - 1.) * log(b) - lgamma(2. * n));
-        const double dbdn = -2. * gamma_p_da(2. * n, b) / dPdb;
-        D[kSD_DLNRE] = log(b) + n * dbdn / b;
-    }
+    __syncthreads();
+    if (live && part == 0) H[kSH_STATUS] = bad_r[lane] ? 3 : bad_b[lane] ? 2 : 0;
 }
 
-// Running state of the serial part of buildFT for one table (SBSersic.cpp:436-509): the
-// maxk bookkeeping and the 10-point high-k least-squares fit, advanced one round of nodes at a
-// time so that nodes past the stopping point are never integrated.
+// Running state of a truncated table's stopping scan (buildFT, SBSersic.cpp:436-509): the 10-point
+// high-k least-squares fit, advanced one round of nodes at a time so that few nodes past the
+// stopping point are integrated.
 struct SersicScan {
-    double sf, skf, sk, sk2, maxk, ksq_max, a, b;
+    double sf, skf, sk, sk2;
     double fit[10];
-    int fit_size, fit_head, n_correct, found, nused, done;
+    int fit_size, fit_head, n_correct, nused, done;
 };
 
 __global__ void sersic_scan_init_kernel(const double* header, int count, SersicScan* scan)
@@ -540,16 +529,13 @@ __global__ void sersic_scan_init_kernel(const double* header, int count, SersicS
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     SersicScan& S = scan[s];
+    const double* H = header + (size_t)s * kSersicHeader;
     S.sf = S.skf = S.sk = S.sk2 = 0.;
-    S.maxk = sqrt(header[(size_t)s * kSersicHeader + kSH_KSQMIN]);
-    S.ksq_max = -1.;
-    S.a = S.b = 0.;
-    S.fit_size = S.fit_head = S.n_correct = S.found = S.nused = 0;
-    S.done = int(header[(size_t)s * kSersicHeader + kSH_NCAND]) < 2 ? 1 : 0;
+    S.fit_size = S.fit_head = S.n_correct = S.nused = 0;
+    S.done = H[kSH_TRUNC] <= 0. || int(H[kSH_NCAND]) < 2 ? 1 : 0;
 }
 
-// One warp per node of this round for the truncated tables (trunc > 0; the pair kernel skips
-// them): the truncated Hankel transform / hankel_norm, hankel_norm = flux fraction n Gamma(2n).
+// One warp per node of this round for the truncated tables (trunc > 0): the truncated Hankel transform / hankel_norm, hankel_norm = flux fraction n Gamma(2n).
 __global__ void __launch_bounds__(256) sersic_trunc_nodes_kernel(const double* header, int count, int i0,
                                     int nround, const __grid_constant__ OgataTables og, const SersicScan* scan,
                                     double* vals, int stride, const int* prev_live, int* status_out)
@@ -573,78 +559,21 @@ __global__ void __launch_bounds__(256) sersic_trunc_nodes_kernel(const double* h
     }
 }
 
-// One warp per pair of adjacent nodes (i, i + 1) of this round: Hankel transform / hankel_norm at
-// k_i, k_{i+1} through warp_hankel_pair; DN: with the d/dn values of the same nodes.
-// prev_live (the previous round's scan flag) is zero once every table has stopped: the launch
-// then returns at once.
-template <bool DN>
-__global__ void __launch_bounds__(256, 4) sersic_nodes_pair_kernel(const double* header, int count, int i0,
-                                    int nround, gsb_gsparams gsp, const __grid_constant__ OgataTables og,
-                                    const SersicScan* scan, double* vals, int stride,
-                                    const int* prev_live, int* status_out, const double* dheader,
-                                    double* dvals)
-{
-    if (prev_live && *prev_live == 0) return;
-    // the exponential's 2^(j/256) table, read three times per pair of terms, from shared memory
-    __shared__ double etab[256];
-    etab[threadIdx.x] = g_exp2_256[threadIdx.x];
-    __syncthreads();
-    const int npair = (nround + 1) / 2;
-    const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    // slots hold ascending n; the costly large-n tables are taken first so that they do not
-    // form the tail of the launch
-    const long long s = count - 1 - warp / npair;
-    const int i = i0 + 2 * int(warp % npair);
-    if (s < 0) return;
-    if (scan[s].done) return;
-    const double* H = header + s * kSersicHeader;
-    if (H[kSH_TRUNC] > 0.) return;          // sersic_trunc_nodes_kernel
-    const int ncand = int(H[kSH_NCAND]);
-    if (i >= ncand) return;
-    const bool has1 = i + 1 < ncand && i + 1 < i0 + nround;
-    const double n = H[kSH_N];
-    const double logk0 = H[kSH_FRONT] + i * H[kSH_DLOGK];
-    const double logk1 = H[kSH_FRONT] + (i + 1) * H[kSH_DLOGK];
-    const double hankel_norm = n * tgamma(2. * n);
-    __shared__ double ans[8][DN ? 8 : 4];  // the running answers of each warp's pair
-    double* a = ans[(threadIdx.x >> 5) & 7];
-    int st = 0;
-    const double dnc = DN ? dheader[s * kSersicDHeader + kSD_DFRONT] : 0.;
-    const double2 v = warp_hankel_pair<DN>(og, 1. / n, logk0, logk1, has1, gsp.integration_relerr,
-                                           gsp.integration_abserr * hankel_norm, &st, a, etab, dnc);
-    if ((threadIdx.x & 31) == 0) {
-        const double v0 = v.x / hankel_norm, v1 = v.y / hankel_norm;
-        vals[s * stride + i] = v0;
-        if (has1) vals[s * stride + i + 1] = v1;
-        if (DN) {
-            // node value y = v k^2 = T(k) / norm with norm = n Gamma(2n) and k = k_i(n):
-            // dy/dn = (dT/dn) / norm - y (1/n + 2 psi(2n)), dT/dn from the second integrand.
-            const double q = 1. / n + 2. * digamma(2. * n);
-            const double k0 = exp(logk0), k1 = exp(logk1);
-            dvals[s * stride + i] = (a[5] / hankel_norm - v0 * q) * k0 * k0;
-            if (has1) dvals[s * stride + i + 1] = (a[7] / hankel_norm - v1 * q) * k1 * k1;
-        }
-        if (st) atomicOr(status_out, 1);
-    }
-}
-
-// live_out is set when a table still needs nodes after this round; a zero prev_live (the
-// previous round's flag) means every table has stopped and the launch returns at once.
+// The stopping scan of the truncated tables, whose nodes are integrated in rounds (the others stop
+// inside sersic_table_kernel).  live_out is set when a table still needs nodes after this round; a
+// zero prev_live (the previous round's flag) means every table has stopped and the launch returns
+// at once.
 __global__ void sersic_scan_kernel(const double* header, int count, int stride, int i0, int nround,
-                                   gsb_gsparams gsp, const double* vals, double4* nodes,
-                                   SersicScan* scan, const double* dvals, double4* dnodes,
+                                   gsb_gsparams gsp, const double* vals, SersicScan* scan,
                                    const int* prev_live, int* live_out)
 {
     if (prev_live && *prev_live == 0) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= count) return;
     if (scan[s].done) return;
-    // the state is advanced in a local copy (the node stores below may alias it as far as the
-    // compiler knows, which would send every field access to global memory) and written back
     SersicScan S = scan[s];
     const double* H = header + (size_t)s * kSersicHeader;
     const double* v = vals + (size_t)s * stride;
-    double4* nd = nodes + (size_t)s * stride;
     const int ncand = int(H[kSH_NCAND]);
     const double front = H[kSH_FRONT], dlogk = H[kSH_DLOGK];
     const int n_fit = 10;
@@ -654,19 +583,17 @@ __global__ void sersic_scan_kernel(const double* header, int count, int stride, 
         const double k = exp(logk), ksq = k * k;
         const double val = v[i];
         const double f0 = val * ksq;
-        nd[i] = make_double4(logk, f0, 0., 0.);
-        if (dnodes) dnodes[(size_t)s * stride + i] = make_double4(logk, dvals[(size_t)s * stride + i], 0., 0.);
-        S.nused = i + 1;
-        if (fabs(val) > gsp.maxk_threshold) { S.maxk = k; S.n_correct = 0; }
+        if (fabs(val) > gsp.maxk_threshold) { S.n_correct = 0; }
         else {
-            S.found = 1;
             const double den = n_fit * S.sk2 - S.sk * S.sk;
-            S.a = (S.sf * S.sk2 - S.sk * S.skf) / den;
-            S.b = (n_fit * S.skf - S.sk * S.sf) / den;
-            const double f0_pred = S.a + S.b / k;
+            const double a = (S.sf * S.sk2 - S.sk * S.skf) / den;
+            const double b = (n_fit * S.skf - S.sk * S.sf) / den;
+            const double f0_pred = a + b / k;
             if (fabs(f0 - f0_pred) / ksq < gsp.kvalue_accuracy) ++S.n_correct;
             else S.n_correct = 0;
-            if (S.n_correct >= 5) { S.ksq_max = ksq; S.done = 1; scan[s] = S; return; }
+            // (one node more than the stop itself: sersic_table_kernel forms its window sums
+            // afresh, and a stop that its rounding moved would read the next node)
+            if (S.n_correct >= 6) { S.done = 1; S.nused = iend; scan[s] = S; return; }
         }
         const double inv_k = 1. / k;
         if (S.fit_size == n_fit) {
@@ -688,11 +615,11 @@ __global__ void sersic_scan_kernel(const double* header, int count, int stride, 
         }
     }
     if (iend >= ncand) S.done = 1;
+    S.nused = iend;
     scan[s] = S;
     if (!S.done && live_out) *live_out = 1;
 }
 
-// End of buildFT (SBSersic.cpp:510-537) and the natural spline (Table.cpp:634-686).
 // Natural cubic spline second derivatives z of nodes (x, y) (Thomas algorithm; c is scratch).
 // TSpline setup, src/Table.cpp:634-686.
 __device__ void natural_spline(const double* x, const double* y, double* z, double* c, int N)
@@ -718,106 +645,331 @@ __device__ void natural_spline(const double* x, const double* y, double* z, doub
     }
 }
 
-// End of buildFT (SBSersic.cpp:510-537) and the natural spline, one warp per table: the warp
-// stages the table's nodes in shared memory (coalesced), lane 0 runs the serial parts there.
-// Dynamic shared memory: 4 * stride doubles.
-__global__ void __launch_bounds__(32) sersic_finalize_kernel(double* header, int count, int stride,
-                                                             gsb_gsparams gsp, const SersicScan* scan,
-                                                             double4* nodes, double4* dnodes, double* dheader)
+// One Sersic table per block: the transforms at the ln k nodes (the reference's adaptive halving,
+// AdaptiveHankelIntegrator::integrate, Hankel.cpp:179-219, on the resampled levels), buildFT's
+// stopping rule, high-k fit and maxk (SBSersic.cpp:436-537) and the natural spline (Table.cpp:634-686).
+//
+// The samples of G (and of its n-derivative) over the whole grid the table can reach are formed
+// once in shared memory; a warp then takes 32 R consecutive nodes, R a thread, through the levels
+// in step: a node starts at its own level (h0 = 1/32 halved while h0 > 100 k), keeps its last two
+// sums and drops out at the first level where the reference's test passes.  After each chunk of
+// THREADS x R nodes every thread tests its own nodes for the stop, so nodes past the stop cost at
+// most the rest of a chunk.  The spline's tridiagonal system on the uniform grid,
+// z_(i-1) + 4 z_i + z_(i+1) = d_i, is solved by its Green's function (-lambda)^|e| / (2 sqrt 3),
+// lambda = 2 - sqrt 3 (2e-18 at |e| = 31), with d continued odd about both ends.
+//
+// Bound by the latency of the multiply-add chains and the shared-memory reads that feed them (R = 3:
+// one read per three).  4096 tables, n in 0.5 .. 4: 1.05 ms, where integrating each node pair by
+// its scattered sums (three exponentials a pair of terms) in rounds with a scan and a spline
+// kernel after them took 10.3 ms; 113 tables 0.31 ms, 1.4 before.
+// R = 1 with 512 threads serves builds of a few tables per SM (kSmallBuild), where a block's
+// latency counts and SMs are idle.
+//
+// Dynamic shared memory: [G samples | (DN) derivative samples | values | (DN) derivative values],
+// gcap + pad doubles a sample array and stride doubles a value array; the spline's right-hand side
+// takes the place of the samples.
+template <int R, int THREADS, bool DN, bool P1>
+__global__ void __launch_bounds__(THREADS, THREADS > 64 ? 1 : 8) sersic_table_kernel(
+    double* header, int count, int stride, gsb_gsparams gsp, const __grid_constant__ OgataLog lg, int p, int gcap,
+    int pad, const SersicScan* scan, const double* tvals, double4* nodes, double4* dnodes, double* dheader,
+    int* status_out)
 {
-    extern __shared__ double fsm[];
-    const int s = blockIdx.x;
-    const int lane = threadIdx.x;
-    if (s >= count) return;
-    double* xs = fsm;
-    double* ys = xs + stride;
-    double* zs = ys + stride;
-    double* cs = zs + stride;
+    extern __shared__ double tsm[];
+    __shared__ int s_stop, s_above, s_below;
+    const int lane = threadIdx.x & 31;
+    // slots hold ascending n; the costly large-n tables are taken first so that they do not form
+    // the tail of the launch
+    const int s = count - 1 - int(blockIdx.x);
     double* H = header + (size_t)s * kSersicHeader;
-    double4* nd = nodes + (size_t)s * stride;
-    const SersicScan& S = scan[s];
-    const int N = S.nused;
-    if (N < 2) {
-        if (lane == 0) { H[kSH_STATUS] = 5; H[kSH_NUSED] = 0; }
+    double* g = tsm;
+    double* gd = g + gcap + pad;
+    double* V = DN ? gd + gcap + pad : gd;
+    double* DV = V + stride;
+    const bool trunc = H[kSH_TRUNC] > 0.;
+    int ncand = int(H[kSH_NCAND]);
+    if (ncand < 2) {
+        if (threadIdx.x == 0) { H[kSH_STATUS] = 5; H[kSH_NUSED] = 0; }
         return;
     }
+    const double n = H[kSH_N], invn = 1. / n;
     const double front = H[kSH_FRONT], dlogk = H[kSH_DLOGK];
-    const int n_fit = 10;
-    for (int i = lane; i < N; i += 32) {
-        const double4 v = nd[i];
-        xs[i] = v.x;
-        ys[i] = v.y;
+    const double norm = n * tgamma(2. * n);
+    const double abserr = gsp.integration_abserr * norm;
+    const double dnc = DN ? dheader[(size_t)s * kSersicDHeader + kSD_DFRONT] : 0.;
+    // samples d = d0 .. dmax at y = d h - front; beyond dmax f = exp(-u) is 0 (u > 745)
+    const int dmax = int(floor((front + 6.6134 * n) / lg.h));
+    const int d0 = dmax - gcap + 1;
+    if (trunc) {
+        ncand = min(ncand, scan[s].nused);
+        for (int i = threadIdx.x; i < ncand; i += THREADS) V[i] = tvals[(size_t)s * stride + i];
+    } else {
+        for (int j = threadIdx.x; j < gcap + pad; j += THREADS) {
+            const double2 v = j < gcap ? sersic_sample((d0 + j) * lg.h - front, invn, dnc) : make_double2(0., 0.);
+            g[j] = v.x;
+            if (DN) gd[j] = v.y;
+        }
     }
-    __syncwarp();
-    double ksq_max = 0., maxk = 0., a = 0., b = 0.;
-    if (lane == 0) {
-        ksq_max = S.ksq_max;
-        maxk = S.maxk;
-        a = S.a;
-        b = S.b;
-        if (ksq_max <= 0.) ksq_max = exp(2. * xs[N - 1]);
-        if (S.found) {
-            maxk *= exp(dlogk);
+    if (threadIdx.x == 0) { s_stop = ncand; s_above = s_below = -1; }
+    __syncthreads();
+
+    const int n_fit = 10;
+    // The fit's four sums (f0, f0 / k, 1 / k, 1 / k^2 over the 10 nodes before node i) are running
+    // sums, as in the reference: they carry the rounding of the first nodes' 1 / k, which at
+    // large n is what the fit consists of, so the order of the additions is kept.  Their steps are
+    // formed by all threads, then four lanes run through the chunk.
+    constexpr int CHUNK = THREADS * R;
+    __shared__ double sums[4][CHUNK];
+    __shared__ double s_end[4], s_fit[2];
+    double carry = 0.;                       // lanes 0-3 of warp 0: the sum before the next chunk
+    auto fit = [&](double sf, double skf, double sk, double sk2, double& a, double& b) {
+        const double den = n_fit * sk2 - sk * sk;
+        a = (sf * sk2 - sk * skf) / den;
+        b = (n_fit * skf - sk * sf) / den;
+    };
+
+    unsigned char* ok = reinterpret_cast<unsigned char*>(DN ? DV + stride : V + stride);
+    for (int c0 = 0; c0 < ncand; c0 += THREADS * R) {
+        const int c1 = min(ncand, c0 + THREADS * R);
+        const int w0 = c0 + int(threadIdx.x >> 5) * 32 * R;      // this warp's nodes w0 .. w0 + 32 R - 1
+        if (!trunc && w0 < c1) {
+            const int m = w0 + lane * R;
+            double prev[R], cur[R], dcur[R], ksq[R];
+            int lev[R];
+            unsigned run = 0;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double k = exp(front + (m + r) * dlogk);
+                ksq[r] = k * k;
+                prev[r] = cur[r] = dcur[r] = 0.;
+                int l = kLogLev0;
+                for (double h0 = 1. / 32.; h0 > 100. * k && l < 60; h0 *= 0.5) ++l;
+                lev[r] = l;
+                if (m + r < c1) run |= 1u << r;
+            }
+            int l = lev[R - 1];                                   // k ascends: the warp's lowest level
+            l = __reduce_min_sync(0xffffffffu, run ? l : 99);
+            const int mlast = min(c1 - 1, w0 + 32 * R - 1);
+            while (__any_sync(0xffffffffu, run != 0u)) {
+                // the reference halves until its level counter passes 60: the last sum is at 61
+                if (l > kLogLev0 + kLogLevels - 1) {
+                    if (lane == 0) atomicOr(status_out, 1);
+                    break;
+                }
+                const int j = l - kLogLev0;
+                const int qmin = lg.qmin[j];
+                const double* A = lg.a + lg.off[j] - qmin;
+                // the nodes still at work in this warp bound the samples that count
+                int mhi = 0;
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if ((run >> r & 1u) && l >= lev[r]) mhi = m + r;
+                mhi = __reduce_max_sync(0xffffffffu, mhi);
+                const int qhi = min(qmin + lg.len[j] - 1, p * mhi + dmax);
+                // samples below d0 (levels far beyond the usual) are formed on the fly
+                const int qlo = max(qmin, d0 + p * mlast + (R - 1) * p);
+                double acc[R], dacc[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) acc[r] = dacc[r] = 0.;
+                for (int q = qmin; q < min(qlo, qhi + 1); ++q) {
+                    const double a = A[q];
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const double2 v = sersic_sample((q - p * (m + r)) * lg.h - front, invn, dnc);
+                        acc[r] = fma(a, v.x, acc[r]);
+                        if (DN) dacc[r] = fma(a, v.y, dacc[r]);
+                    }
+                }
+                // (lanes past mlast read other samples of the array, or its zero padding)
+                if (qlo <= qhi)
+                    correlate<R, DN, P1>(A, qlo, qhi, g - d0, gd - d0, min(m, mlast), p, dmax + 1, acc, dacc);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (!(run >> r & 1u) || l < lev[r]) continue;
+                    prev[r] = cur[r];
+                    cur[r] = acc[r] / ksq[r];
+                    if (DN) dcur[r] = dacc[r] / ksq[r];
+                    if (l == lev[r]) continue;
+                    const double err = fabs(cur[r] - prev[r]);
+                    const bool more = (err > gsp.integration_relerr * cur[r] &&
+                                       (err > abserr || fabs(cur[r]) > 2. * fabs(prev[r]))) || cur[r] == 0.;
+                    if (!more) run &= ~(1u << r);
+                }
+                ++l;
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (m + r >= c1) continue;
+                const double v = cur[r] / norm;
+                V[m + r] = v;
+                // node value y = v k^2 = T(k) / norm with norm = n Gamma(2n) and k = k_i(n):
+                // dy/dn = (dT/dn) / norm - y (1/n + 2 psi(2n)), dT/dn from the second correlation.
+                if (DN) DV[m + r] = (dcur[r] / norm - v * (1. / n + 2. * digamma(2. * n))) * ksq[r];
+            }
+        }
+        __syncthreads();
+        for (int i = c0 + threadIdx.x; i < c1; i += THREADS) {
+            const double logk = front + i * dlogk;
+            const double k = exp(logk), ksq = k * k, f0 = V[i] * ksq, inv_k = 1. / k;
+            const int j = i - c0;
+            if (i >= n_fit) {
+                const double k_back = exp(logk - n_fit * dlogk);
+                const double kb = exp(front + (i - n_fit) * dlogk);
+                const double f_back = V[i - n_fit] * (kb * kb);
+                const double inv_k_back = 1. / k_back;
+                sums[0][j] = f0 - f_back;
+                sums[1][j] = f0 * inv_k - f_back * inv_k_back;
+                sums[2][j] = inv_k - inv_k_back;
+                sums[3][j] = inv_k * inv_k - inv_k_back * inv_k_back;
+            } else {
+                sums[0][j] = f0;
+                sums[1][j] = f0;             // times 1 / k and 1 / k^2 below, fused with the addition
+                sums[2][j] = inv_k;
+                sums[3][j] = inv_k;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < 4) {
+            double* sm = sums[threadIdx.x];
+            int j = 0;
+            for (; j < c1 - c0 && c0 + j < n_fit; ++j) {
+                const double v = sm[j], inv_k = 1. / exp(front + (c0 + j) * dlogk);
+                const double next = threadIdx.x == 1 ? fma(v, inv_k, carry) : threadIdx.x == 3 ? fma(v, v, carry) : carry + v;
+                sm[j] = carry;
+                carry = next;
+            }
+#pragma unroll 8
+            for (; j < c1 - c0; ++j) {
+                const double v = sm[j];
+                sm[j] = carry;
+                carry += v;
+            }
+        }
+        __syncthreads();
+        // the stop: the fifth in a row of the nodes below maxk_threshold that the fit predicts
+        for (int i = c0 + threadIdx.x; i < c1; i += THREADS) {
+            const int j = i - c0;
+            const double k = exp(front + i * dlogk), ksq = k * k;
+            bool good = false;
+            if (!(fabs(V[i]) > gsp.maxk_threshold)) {
+                double a, b;
+                fit(sums[0][j], sums[1][j], sums[2][j], sums[3][j], a, b);
+                good = fabs(V[i] * ksq - (a + b / k)) / ksq < gsp.kvalue_accuracy;
+            }
+            ok[i] = good;
+        }
+        __syncthreads();
+        for (int i = max(c0, 4) + int(threadIdx.x); i < c1; i += THREADS)
+            if (ok[i] && ok[i - 1] && ok[i - 2] && ok[i - 3] && ok[i - 4]) atomicMin(&s_stop, i);
+        __syncthreads();
+        // the last node whose fit was taken (the stop, if any), and the last above the threshold
+        const int end = min(c1, s_stop + 1);
+        for (int i = c0 + threadIdx.x; i < end; i += THREADS)
+            atomicMax(fabs(V[i]) > gsp.maxk_threshold ? &s_above : &s_below, i);
+        __syncthreads();
+        if (threadIdx.x == 0 && s_below >= c0) {
+            const int j = s_below - c0;
+            fit(sums[0][j], sums[1][j], sums[2][j], sums[3][j], s_fit[0], s_fit[1]);
+        }
+        if (s_stop < ncand) break;
+    }
+    if (threadIdx.x < 4) s_end[threadIdx.x] = carry;
+    const bool stopped = s_stop < ncand;
+    const int N = stopped ? s_stop + 1 : ncand;
+    // the spline's right-hand side, in the samples' place
+    double* D = tsm;
+    const double ih2 = 6. / (dlogk * dlogk);
+    auto f0 = [&](int i) { const double k = exp(front + i * dlogk); return V[i] * (k * k); };
+    for (int i = threadIdx.x; i < N; i += THREADS) {
+        const bool in = i > 0 && i < N - 1;
+        D[i] = in ? ih2 * ((f0(i + 1) - f0(i)) - (f0(i) - f0(i - 1))) : 0.;
+    }
+    __syncthreads();
+    const double back = front + (N - 1) * dlogk;
+    if (threadIdx.x == 0) {
+        double a, b, maxk, ksq_max;
+        if (s_below >= 0) {
+            a = s_fit[0];
+            b = s_fit[1];
+            maxk = (s_above >= 0 ? exp(front + s_above * dlogk) : sqrt(H[kSH_KSQMIN])) * exp(dlogk);
         } else {
-            const double den = n_fit * S.sk2 - S.sk * S.sk;
-            a = (S.sf * S.sk2 - S.sk * S.skf) / den;
-            b = (n_fit * S.skf - S.sk * S.sf) / den;
+            fit(s_end[0], s_end[1], s_end[2], s_end[3], a, b);
             maxk = sqrt(a / gsp.maxk_threshold);
             for (int it = 0; it < 3; ++it) maxk = sqrt((a - b / maxk) / gsp.maxk_threshold);
         }
-        natural_spline(xs, ys, zs, cs, N);
+        if (stopped) {
+            const double k = exp(back);
+            ksq_max = k * k;
+        } else {
+            ksq_max = exp(2. * back);
+        }
+        H[kSH_NUSED] = N;
+        H[kSH_DA] = (back - front) / (N - 1);
+        H[kSH_KSQMAX] = ksq_max;
+        H[kSH_HIGHA] = a;
+        H[kSH_HIGHB] = b;
+        H[kSH_MAXK] = maxk;
     }
-    __syncwarp();
+    // z_i = sum_e G(e) d_(i + e), d odd about nodes 0 and N - 1 (period 2 (N - 1))
+    auto green = [&](const double* d, int i) {
+        const int L = N - 1;
+        const double lam = -0.26794919243112270647;        // sqrt 3 - 2
+        if (N < 3) return 0.;
+        auto at = [&](int j) {
+            j %= 2 * L;
+            if (j < 0) j += 2 * L;
+            return j <= L ? d[j] : -d[2 * L - j];
+        };
+        double w = 1., sum = d[i];
+        if (i >= 31 && i + 31 <= L) {
+            for (int e = 1; e <= 31; ++e) { w *= lam; sum = fma(w, d[i - e] + d[i + e], sum); }
+        } else {
+            for (int e = 1; e <= 31; ++e) { w *= lam; sum = fma(w, at(i - e) + at(i + e), sum); }
+        }
+        return sum * 0.28867513459481288225;               // 1 / (2 sqrt 3)
+    };
+    double4* nd = nodes + (size_t)s * stride;
     // .w: k^2 at the node, for the evaluators' spline offset 0.5 ln(k_i^2 / k^2)
-    for (int i = lane; i < N; i += 32) nd[i] = make_double4(xs[i] - front, ys[i], zs[i], exp(2. * xs[i]));
-    const double back = xs[N - 1];
-    if (dnodes) {
+    for (int i = threadIdx.x; i < N; i += THREADS) {
+        const double x = front + i * dlogk;
+        nd[i] = make_double4(x - front, f0(i), (i == 0 || i == N - 1) ? 0. : green(D, i), exp(2. * x));
+    }
+    if (DN) {
         // The spline is linear in its node values, so d/dn of the interpolant is the spline of
         // the node derivatives on the same grid.  Likewise the high-k fit is linear in the f0
         // values of its window: the 10 nodes before the stopping node, or the last 10 nodes
         // when the scan ran to the end of the candidate grid.
         double4* dn = dnodes + (size_t)s * stride;
-        __syncwarp();
-        for (int i = lane; i < N; i += 32) cs[i] = ys[i];     // keep f0 for the fit window
-        __syncwarp();
-        for (int i = lane; i < N; i += 32) ys[i] = dn[i].y;
-        __syncwarp();
-        double* f0s = zs;   // reuse: z of the main table is already written out
-        if (lane == 0) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < N; i += THREADS)
+            D[i] = i > 0 && i < N - 1 ? ih2 * ((DV[i + 1] - DV[i]) - (DV[i] - DV[i - 1])) : 0.;
+        __syncthreads();
+        for (int i = threadIdx.x; i < N; i += THREADS)
+            dn[i] = make_double4(front + i * dlogk - front, DV[i], (i == 0 || i == N - 1) ? 0. : green(D, i), 0.);
+        if (threadIdx.x == 0) {
             // The fit's 1/k_i move too: d(1/k_i)/dn = -c / k_i with c = dfront/dn.
-            double* D = dheader + (size_t)s * kSersicDHeader;
-            const double c = D[kSD_DFRONT];
-            const int wend = S.ksq_max > 0. ? N - 1 : N;
+            double* Dh = dheader + (size_t)s * kSersicDHeader;
+            const double c = dnc;
+            const int wend = stopped ? N - 1 : N;
             const int wbeg = wend - n_fit > 0 ? wend - n_fit : 0;
             double sk = 0., sk2 = 0., sf = 0., skf = 0., dsf = 0., dskf = 0.;
             for (int i = wbeg; i < wend; ++i) {
                 const double inv_k = exp(-(front + i * dlogk));
-                const double f0 = cs[i], df0 = ys[i];
+                const double f = f0(i), df = DV[i];
                 sk += inv_k;
                 sk2 += inv_k * inv_k;
-                sf += f0;
-                skf += f0 * inv_k;
-                dsf += df0;
-                dskf += (df0 - c * f0) * inv_k;
+                sf += f;
+                skf += f * inv_k;
+                dsf += df;
+                dskf += (df - c * f) * inv_k;
             }
             const double dsk = -c * sk, dsk2 = -2. * c * sk2;
             const double den = n_fit * sk2 - sk * sk, dden = n_fit * dsk2 - 2. * sk * dsk;
             const double na = sf * sk2 - sk * skf, dna = dsf * sk2 + sf * dsk2 - dsk * skf - sk * dskf;
             const double nb = n_fit * skf - sk * sf, dnb = n_fit * dskf - dsk * sf - sk * dsf;
-            D[kSD_DHIGHA] = (dna * den - na * dden) / (den * den);
-            D[kSD_DHIGHB] = (dnb * den - nb * dden) / (den * den);
-            natural_spline(xs, ys, f0s, cs, N);
+            Dh[kSD_DHIGHA] = (dna * den - na * dden) / (den * den);
+            Dh[kSD_DHIGHB] = (dnb * den - nb * dden) / (den * den);
         }
-        __syncwarp();
-        for (int i = lane; i < N; i += 32) dn[i] = make_double4(xs[i] - front, ys[i], f0s[i], 0.);
     }
-    if (lane != 0) return;
-    H[kSH_NUSED] = N;
-    H[kSH_DA] = (back - front) / (N - 1);
-    H[kSH_KSQMAX] = ksq_max;
-    H[kSH_HIGHA] = a;
-    H[kSH_HIGHB] = b;
-    H[kSH_MAXK] = maxk;
 }
 
 // Truncated Moffat FT tables (SBMoffat::setupFT, src/SBMoffat.cpp:565-625).  Per slot
@@ -1273,6 +1425,118 @@ static int sersic_stride(const double* h_n, int count, const gsb_gsparams* gsp)
     return int(span / dlogk) + 4;
 }
 
+// The resampled quadrature levels of each device and spacing, kept while they are among the last
+// few spacings used (a spacing is a GSParams setting: a program has one or two; 0.4 MB each).
+namespace {
+struct LogEntry {
+    double* a = nullptr;
+    OgataLog lg{};
+    unsigned long long used = 0;
+};
+constexpr int kLogEntries = 4;
+LogEntry g_log[64][kLogEntries];
+unsigned long long g_log_clock = 0;
+std::mutex g_log_mutex;
+}  // namespace
+
+// The levels for grid spacing h (g_log_mutex held).
+static int ogata_log_levels(DeviceState* st, double h, cudaStream_t stream, OgataLog* out)
+{
+    int dev = 0;
+    cudaGetDevice(&dev);
+    LogEntry* slots = g_log[dev & 63];
+    LogEntry* e = slots;
+    for (int i = 0; i < kLogEntries; ++i) {
+        if (slots[i].a && slots[i].lg.h == h) {
+            slots[i].used = ++g_log_clock;
+            *out = slots[i].lg;
+            return GSB_OK;
+        }
+        if (slots[i].used < e->used) e = &slots[i];
+    }
+    OgataLog lg{};
+    lg.h = h;
+    int total = 0, cnt[kLogLevels];
+    auto psi = [](double t) { return t * std::tanh(0.5 * M_PI * std::sinh(t)); };
+    for (int j = 0; j < kLogLevels; ++j) {
+        const double hl = std::ldexp(1.0, -(kLogLev0 + j));
+        cnt[j] = int(std::min(M_PI / hl, double(kNroot)));
+        // the first and last node: J0's first zero, and its cnt-th to McMahon's leading term
+        const double t0 = hl * 2.404825557695773 / M_PI, t1 = hl * (cnt[j] - 0.25);
+        const double x0 = M_PI / hl * psi(t0), x1 = M_PI / hl * psi(t1);
+        lg.qmin[j] = int(std::floor(std::log(x0) / h)) - kLogW / 2 - 1;
+        lg.len[j] = int(std::ceil(std::log(x1) / h)) + kLogW / 2 + 1 - lg.qmin[j] + 1;
+        lg.off[j] = total;
+        total += lg.len[j];
+    }
+    cudaFree(e->a);
+    e->a = nullptr;
+    e->lg.h = 0.;
+    GSB_CUDA_CHECK(cudaMalloc(&e->a, sizeof(double) * total));
+    double2* d_tmp = nullptr;
+    int rc = GSB_OK;
+    cudaError_t ce = cudaMallocAsync(&d_tmp, sizeof(double2) * kNroot, stream);
+    for (int j = 0; j < kLogLevels && ce == cudaSuccess; ++j) {
+        const int lev = kLogLev0 + j;
+        const double2* xw = d_tmp;
+        if (lev <= kLevMax) xw = st->d_xw + st->og.off[lev - kLevMin];
+        else ogata_level_kernel<<<(cnt[j] + 255) / 256, 256, 0, stream>>>(d_tmp, st->d_root, std::ldexp(1.0, -lev), cnt[j]);
+        ogata_log_kernel<<<lg.len[j], 256, 0, stream>>>(xw, cnt[j], h, lg.qmin[j], e->a + lg.off[j]);
+        ce = cudaGetLastError();
+    }
+    if (d_tmp) cudaFreeAsync(d_tmp, stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);
+    if (ce != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(e->a);
+        e->a = nullptr;
+        return set_error(GSB_ERR_CUDA, std::string("resampled quadrature levels: ") + cudaGetErrorString(ce));
+    }
+    lg.a = e->a;
+    e->lg = lg;
+    e->used = ++g_log_clock;
+    *out = lg;
+    return rc;
+}
+
+// Builds of at most this many tables per SM take one 512-thread block of single nodes a table.
+constexpr int kSmallBuild = 4;
+
+template <int R, int THREADS>
+static int launch_sersic_tables(gsb_tables* t, int count, int stride, double nmax, const gsb_gsparams* gsp,
+                                const OgataLog& lg, int p, const SersicScan* scan, double4* dnode, double* dheader,
+                                int* d_status, cudaStream_t stream)
+{
+    // the samples a table of index nmax reaches from its level-12 sums down to its last node; smaller
+    // n reach less far up
+    const double kderiv6 = std::exp(std::lgamma(8. * nmax) - std::lgamma(2. * nmax)) / 2304.;
+    const double front = std::log(gsp->kvalue_accuracy / kderiv6) / 6.;
+    const int reach = std::max(0, int((front + 6.6134 * nmax) / lg.h)) + 1 - std::min(0, lg.qmin[12 - kLogLev0]);
+    const int pad = p == 1 ? 33 * R : 1;
+    const bool dn = dheader != nullptr;
+    // per table: the samples (or the spline's right-hand side), the values, one flag byte a node
+    const size_t fixed = (size_t)stride * (dn ? 2 : 1) * sizeof(double) + stride + 16;
+    const size_t room = 226 * 1024 - sizeof(double) * 4 * THREADS * R;
+    const size_t per = sizeof(double) * (dn ? 2 : 1);
+    // as many samples as the tables need, at least the right-hand side's room (samples that do not
+    // fit are formed on the fly)
+    size_t gcap = ((size_t)reach + (size_t)p * stride + 63) / 64 * 64;
+    const size_t least = std::max<size_t>(64, dn ? stride / 2 + 1 : stride);
+    if (fixed + per * (least + pad) > room) return set_error(GSB_ERR_UNSUPPORTED, "Sersic table too long");
+    gcap = std::max(std::min(gcap, (room - fixed) / per - pad), least);
+    const size_t sm = fixed + per * (gcap + pad);
+    auto go = [&](auto kernel) -> int {
+        if (sm + sizeof(double) * 4 * THREADS * R > 47 * 1024)
+            GSB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+        kernel<<<count, THREADS, sm, stream>>>(t->d_header, count, stride, *gsp, lg, p, int(gcap), pad, scan, t->d_val,
+                                               t->d_node, dnode, dheader, d_status);
+        GSB_CUDA_CHECK(cudaGetLastError());
+        return GSB_OK;
+    };
+    if (p == 1) return dn ? go(sersic_table_kernel<R, THREADS, true, true>) : go(sersic_table_kernel<R, THREADS, false, true>);
+    return dn ? go(sersic_table_kernel<R, THREADS, true, false>) : go(sersic_table_kernel<R, THREADS, false, false>);
+}
+
 int sersic_tables_build(gsb_tables* t, const double* h_n, const double* h_trunc, int count,
                         const gsb_gsparams* gsp, bool with_dn, cudaStream_t stream)
 {
@@ -1305,18 +1569,16 @@ int sersic_tables_build(gsb_tables* t, const double* h_n, const double* h_trunc,
         GSB_CUDA_CHECK(cudaMalloc(&t->d_status, sizeof(int) * (1 + kMaxRounds)));
     }
     if (with_dn && ((size_t)count > t->cap_dn_slots || (size_t)count * stride > t->cap_dn_nodes)) {
-        cudaFree(t->d_dheader); cudaFree(t->d_dnode); cudaFree(t->d_dval);
-        t->d_dheader = nullptr; t->d_dnode = nullptr; t->d_dval = nullptr;
+        cudaFree(t->d_dheader); cudaFree(t->d_dnode);
+        t->d_dheader = nullptr; t->d_dnode = nullptr;
         t->cap_dn_slots = std::max<size_t>(count, t->cap_dn_slots);
         t->cap_dn_nodes = std::max<size_t>((size_t)count * stride, t->cap_dn_nodes);
         GSB_CUDA_CHECK(cudaMalloc(&t->d_dheader, sizeof(double) * kSersicDHeader * t->cap_dn_slots));
         GSB_CUDA_CHECK(cudaMalloc(&t->d_dnode, sizeof(double4) * t->cap_dn_nodes));
-        GSB_CUDA_CHECK(cudaMalloc(&t->d_dval, sizeof(double) * t->cap_dn_nodes));
     }
     t->has_dn = with_dn;
     double* dheader = with_dn ? t->d_dheader : nullptr;
     double4* dnode = with_dn ? t->d_dnode : nullptr;
-    double* dval = with_dn ? t->d_dval : nullptr;
     t->count = count;
     t->stride = stride;
     double* d_n = t->d_n;
@@ -1334,96 +1596,48 @@ int sersic_tables_build(gsb_tables* t, const double* h_n, const double* h_trunc,
         GSB_CUDA_CHECK(cudaMemcpyAsync(d_trunc, h_trunc, sizeof(double) * count, cudaMemcpyHostToDevice, stream));
     }
     if ((stride + kTableRound - 1) / kTableRound > kMaxRounds) return set_error(GSB_ERR_UNSUPPORTED, "Sersic table too long");
-    const size_t fsm = sizeof(double) * 4 * (size_t)stride;
-    if (fsm > 227 * 1024) return set_error(GSB_ERR_UNSUPPORTED, "Sersic table too long");
-    if (fsm > 48 * 1024)
-        GSB_CUDA_CHECK(cudaFuncSetAttribute(sersic_finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            int(std::min<size_t>(fsm, 227 * 1024))));
-    // the device part of the build: set-up, the rounds of nodes and their stopping scans, the
-    // finalisation (no host synchronisation inside)
-    auto enqueue = [&](cudaStream_t stream) -> int {
-        // d_status[0]: convergence status; d_status[1 + r]: some table still needs nodes after round r
-        GSB_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int) * (1 + kMaxRounds), stream));
-        sersic_setup_kernel<<<(count + 127) / 128, 128, 0, stream>>>(d_n, d_trunc, count, *gsp, t->d_header, stride,
-                                                                     dheader);
-        GSB_CUDA_CHECK(cudaGetLastError());
-        sersic_scan_init_kernel<<<(count + 127) / 128, 128, 0, stream>>>(t->d_header, count, static_cast<SersicScan*>(t->d_scan));
-        GSB_CUDA_CHECK(cudaGetLastError());
-        // Rounds of kRound ln k nodes: integrate, then advance each table's stopping scan.
-        constexpr int kRound = kTableRound;
-        const int threads = 256;
-        for (int i0 = 0, r = 0; i0 < stride; i0 += kRound, ++r) {
-            const int* prev_live = r > 0 ? d_status + r : nullptr;
-            const long long nwarps = (long long)count * ((kRound + 1) / 2);
-            const long long blocks = (nwarps * 32 + threads - 1) / threads;
-            if (with_dn)
-                sersic_nodes_pair_kernel<true><<<(unsigned)blocks, threads, 0, stream>>>(
-                    t->d_header, count, i0, kRound, *gsp, st->og, static_cast<const SersicScan*>(t->d_scan),
-                    t->d_val, stride, prev_live, d_status, dheader, dval);
-            else
-                sersic_nodes_pair_kernel<false><<<(unsigned)blocks, threads, 0, stream>>>(
-                    t->d_header, count, i0, kRound, *gsp, st->og, static_cast<const SersicScan*>(t->d_scan),
-                    t->d_val, stride, prev_live, d_status, nullptr, nullptr);
-            GSB_CUDA_CHECK(cudaGetLastError());
-            if (has_trunc) {
-                const long long tw = (long long)count * kRound;
-                sersic_trunc_nodes_kernel<<<(unsigned)((tw * 32 + threads - 1) / threads), threads, 0, stream>>>(
-                    t->d_header, count, i0, kRound, st->og, static_cast<const SersicScan*>(t->d_scan), t->d_val, stride,
-                    prev_live, d_status);
-                GSB_CUDA_CHECK(cudaGetLastError());
-            }
-            sersic_scan_kernel<<<(count + 63) / 64, 64, 0, stream>>>(t->d_header, count, stride, i0, kRound,
-                                                                     *gsp, t->d_val, t->d_node, static_cast<SersicScan*>(t->d_scan),
-                                                                     dval, dnode, prev_live, d_status + 1 + r);
-            GSB_CUDA_CHECK(cudaGetLastError());
-        }
-        sersic_finalize_kernel<<<count, 32, fsm, stream>>>(t->d_header, count, stride, *gsp,
-                                                            static_cast<const SersicScan*>(t->d_scan), t->d_node,
-                                                            dnode, dheader);
-        GSB_CUDA_CHECK(cudaGetLastError());
-        return GSB_OK;
-    };
-    // The launches are captured once as a CUDA graph and replayed while the build's shape is
-    // unchanged (table count, node stride, flags, GSParams and buffers: the captured launches
-    // hold them); the captured early-exit rounds then cost a graph node each instead of a launch.
-    struct Key {
-        int count, stride, with_dn, has_trunc;
-        gsb_gsparams gsp;
-        const void* ptr[12];
-    } key;
-    std::memset(&key, 0, sizeof(key));
-    key.count = count;
-    key.stride = stride;
-    key.with_dn = with_dn;
-    key.has_trunc = has_trunc;
-    key.gsp = *gsp;
-    const void* ptrs[12] = {t->d_header, t->d_node, t->d_val, t->d_scan, d_n, d_status, d_trunc, dheader,
-                            dnode, dval, st->og.xw, st->og.root};
-    for (int k = 0; k < 12; ++k) key.ptr[k] = ptrs[k];
-    static_assert(sizeof(Key) <= sizeof(t->sersic_key), "graph key too large");
-    if (!(t->sersic_exec && std::memcmp(t->sersic_key, &key, sizeof(key)) == 0)) {
-        if (t->sersic_exec) { cudaGraphExecDestroy(t->sersic_exec); t->sersic_exec = nullptr; }
-        // captured on a private stream (the caller's may be the legacy default stream, which
-        // cannot be captured); capturing runs nothing
-        if (!t->capture_stream) GSB_CUDA_CHECK(cudaStreamCreateWithFlags(&t->capture_stream, cudaStreamNonBlocking));
-        GSB_CUDA_CHECK(cudaStreamBeginCapture(t->capture_stream, cudaStreamCaptureModeThreadLocal));
-        const int rc = enqueue(t->capture_stream);
-        cudaGraph_t graph = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(t->capture_stream, &graph);
-        if (rc || ce != cudaSuccess) {
-            if (graph) cudaGraphDestroy(graph);
-            cudaGetLastError();
-            return rc ? rc : set_error(GSB_ERR_CUDA, std::string("table-build capture: ") + cudaGetErrorString(ce));
-        }
-        const cudaError_t ie = cudaGraphInstantiate(&t->sersic_exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) {
-            t->sersic_exec = nullptr;
-            return set_error(GSB_ERR_CUDA, std::string("table-build graph: ") + cudaGetErrorString(ie));
-        }
-        std::memcpy(t->sersic_key, &key, sizeof(key));
+    OgataLog lg;
+    const double dlogk = gsp->table_spacing * std::sqrt(std::sqrt(gsp->kvalue_accuracy / 10.));
+    const int p = std::max(1, int(std::ceil(dlogk / kLogMaxStep)));
+    // held until the launch that reads the resampled levels is queued: an eviction frees only
+    // after the device has finished it
+    std::unique_lock<std::mutex> lock(g_log_mutex);
+    {
+        const int rc = ogata_log_levels(st, dlogk / p, stream, &lg);
+        if (rc) return rc;
     }
-    GSB_CUDA_CHECK(cudaGraphLaunch(t->sersic_exec, stream));
+    // truncated tables: rounds of kTableRound ln k nodes, each followed by the stopping scan
+    const int rounds = has_trunc ? (stride + kTableRound - 1) / kTableRound : 0;
+    if (rounds > kMaxRounds) return set_error(GSB_ERR_UNSUPPORTED, "Sersic table too long");
+    // d_status[0]: convergence status; d_status[1 + r]: some table still needs nodes after round r
+    GSB_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int) * (1 + rounds), stream));
+    sersic_setup_kernel<<<(count + 31) / 32, 96, 0, stream>>>(d_n, d_trunc, count, *gsp, t->d_header, stride, dheader);
+    GSB_CUDA_CHECK(cudaGetLastError());
+    SersicScan* scan = static_cast<SersicScan*>(t->d_scan);
+    if (has_trunc) {
+        sersic_scan_init_kernel<<<(count + 127) / 128, 128, 0, stream>>>(t->d_header, count, scan);
+        GSB_CUDA_CHECK(cudaGetLastError());
+        for (int r = 0; r < rounds; ++r) {
+            const int* prev_live = r > 0 ? d_status + r : nullptr;
+            const long long tw = (long long)count * kTableRound;
+            sersic_trunc_nodes_kernel<<<(unsigned)((tw * 32 + 255) / 256), 256, 0, stream>>>(
+                t->d_header, count, r * kTableRound, kTableRound, st->og, scan, t->d_val, stride, prev_live, d_status);
+            GSB_CUDA_CHECK(cudaGetLastError());
+            sersic_scan_kernel<<<(count + 63) / 64, 64, 0, stream>>>(t->d_header, count, stride, r * kTableRound,
+                                                                     kTableRound, *gsp, t->d_val, scan, prev_live,
+                                                                     d_status + 1 + r);
+            GSB_CUDA_CHECK(cudaGetLastError());
+        }
+    }
+    double nmax = 0.;
+    for (int i = 0; i < count; ++i) nmax = std::max(nmax, h_n[i]);
+    {
+        const int rc = count <= kSmallBuild * st->sm_count
+                           ? launch_sersic_tables<1, 512>(t, count, stride, nmax, gsp, lg, p, scan, dnode, dheader, d_status, stream)
+                           : launch_sersic_tables<3, 64>(t, count, stride, nmax, gsp, lg, p, scan, dnode, dheader, d_status, stream);
+        if (rc) return rc;
+    }
+    lock.unlock();
     int h_status = 0;
     GSB_CUDA_CHECK(cudaMemcpyAsync(&h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, stream));
     GSB_CUDA_CHECK(cudaStreamSynchronize(stream));
