@@ -61,6 +61,7 @@ int adjoint_images(const gsb_template* tpl, int n_stamps, const gsb_leaf* d_leav
         return set_error(GSB_ERR_INVALID, "the adjoint of Sersic leaves needs tables built with n-derivatives");
     AdjArgs args;
     args.tpl = *tpl;
+    plan_factors(args.tpl, args.fac);
     args.n_stamps = n_stamps;
     args.leaves = d_leaves;
     args.phases = d_phases;

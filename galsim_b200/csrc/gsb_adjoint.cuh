@@ -32,6 +32,7 @@ __host__ __device__ inline int grad_count(const gsb_template& tpl)
 
 struct AdjArgs {
     gsb_template tpl;
+    FactorPlan fac;
     int n_stamps;
     const gsb_leaf* leaves;
     const gsb_phase* phases;
@@ -232,7 +233,7 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
                     ld[a] = leaf_grad<T>(S.leaf[l], S.sersic, A.dn, kx, ky, g, i - g.x0, j - g.y0);
                     val[a] = cx<T>(ld[a].v, T(0));
                 } else {
-                    val[a] = leaf_cfast<T, II>(S, cache, l, kx, ky, i, j, g);
+                    val[a] = leaf_cfast<T, II>(S, cache, l, i, j, g);
                 }
             } else {
                 val[a] = eval_range<T, II>(tpl, S, cache, dk, i, j, g, o0, o1);
@@ -346,7 +347,7 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32) adjoint_fused_kernel(c
         const int Nk = G.Nk;
         const int hk = Nk / 2;
         const GridRef g{dk, 0, -hk, hk + 1, Nk + 1};
-        if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, Nk, a.want);
+        if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, a.want);
         __syncthreads();
         fill_caches<T, II>(S, a.tpl, cache, dk, Nk);
         __syncthreads();

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_col_kernel(const __grid_con
     const gsb_stamp& G = S.geom;
     const int Nk = G.Nk, hk = Nk / 2;
     const GridRef g{dk, 0, -hk, hk + 1, Nk + 1};
-    if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, Nk, a.want, la.cache_bytes);
+    if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, a.want, la.cache_bytes);
     __syncthreads();
     fill_caches<T, II>(S, a.tpl, cache, dk, Nk);
     __syncthreads();

@@ -121,6 +121,7 @@ int draw_images(const gsb_template* tpl, int n_stamps, const gsb_leaf* d_leaves,
 {
     DrawArgs args;
     args.tpl = *tpl;
+    plan_factors(args.tpl, args.fac);
     args.n_stamps = n_stamps;
     args.leaves = d_leaves;
     args.phases = d_phases;

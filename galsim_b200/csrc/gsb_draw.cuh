@@ -27,10 +27,27 @@
 namespace gsb {
 
 
-constexpr int kWarps = 16;          // warps per CTA (fewer where their FFT scratch does not fit)
+constexpr int kWarps = 16;          // most warps per CTA
+
+// How a leaf's value is formed at a wave vector.  The named kinds read constants of type T formed
+// once per stamp (LeafT); kLeafGeneric goes through leaf_kvalue.
+enum LeafKind { kLeafGeneric = 0, kLeafSep, kLeafExp, kLeafSersic, kLeafMoffat1, kLeafMoffat2, kLeafMoffat3,
+                kLeafMoffatSum, kLeafKolm, kLeafAiry };
+
+// A leaf's constants in the working precision: (u, v) = (a i + c j, b i + d j) is the wave vector of
+// grid point (i, j) in the leaf's own units (Jacobian, dk and size in one factor each), so a point
+// costs a multiply-add an axis and no conversion from the FP64 records.
+template <typename T>
+struct __align__(16) LeafT {
+    T a, b, c, d;
+    T flux;
+    int kind, cache, n;
+    T q[10];
+};
 
 struct StampSmem {
     LeafParams leaf[GSB_MAX_LEAVES];
+    LeafT<double> leaf_t[GSB_MAX_LEAVES];   // holds LeafT<T> of the kernel's T (leaf_const)
     SersicTableView sersic[GSB_MAX_LEAVES];
     gsb_phase phase[GSB_MAX_PHASES];
     double phase_ax[GSB_MAX_PHASES];   // phase turns per k index, x and y
@@ -44,6 +61,7 @@ struct StampSmem {
     int phase_cache[GSB_MAX_PHASES];
     int sersic_cache[GSB_MAX_LEAVES];
     int ii_cache[GSB_MAX_LEAVES];      // InterpolatedImage taps per column / row (IITaps)
+    int aux_cache[GSB_MAX_LEAVES];     // Exponential: kept columns per row; Moffat: quadrature nodes
     int regstack;      // the program fits the 4-deep register stack
     // Factored form of the program (see plan_factored): the root is a product of atoms; the
     // separable atoms (diagonal Box / Gaussian leaves, phases, scales) are folded into
@@ -55,6 +73,10 @@ struct StampSmem {
     short atom_o1[GSB_MAX_OPS];
     unsigned char atom_kind[GSB_MAX_OPS];      // kAtomRange, kAtomPhase (arg), kAtomScale (arg)
     unsigned char atom_arg[GSB_MAX_OPS];
+    // evaluation list: the leaves of the atoms that are real leaves or sums of them, real_last marking
+    // the last of an atom; the other atoms follow by index
+    int n_real, n_other;
+    unsigned char real_leaf[GSB_MAX_OPS], real_last[GSB_MAX_OPS], other[GSB_MAX_OPS];
     unsigned char leaf_sep[GSB_MAX_LEAVES];    // leaf folded into XS / YS
     unsigned char phase_sep[GSB_MAX_PHASES];   // phase folded into XS / YS
     unsigned char scale_sep[GSB_MAX_SCALES];   // scale folded into XS / YS
@@ -68,15 +90,33 @@ constexpr size_t kSmemLimit = 227 * 1024;
 // Warps per CTA of the fused kernels for (T, N): 16, or 8 where 16 per-warp FFT buffers of N
 // complex T (plus twiddles, stamp state and caches) exceed the 227 KB of shared memory
 // (double at N >= 768).
+//
+// In float, 8 warps of up to 128 registers where the shared memory leaves room for two CTAs on an
+// SM (N <= 128, and N >= 256, whose W is in global memory): the evaluator takes four wave
+// vectors a lane at a time, which needs the registers, and two CTAs cover one another's set-up.
+// N = 192 fills an SM's shared memory with one CTA: 16 warps.
 template <typename T, int N>
 __host__ __device__ constexpr int fused_warps()
 {
+    if (sizeof(T) == 4 && N != 192) return kWarps / 2;
     return ((sizeof(StampSmem) + 15) / 16 * 16 + sizeof(Cx<T>) * N * (1 + kWarps) + kCacheBytes + 4096 <=
             kSmemLimit) ? kWarps : kWarps / 2;
 }
 
+// The factors of the program's root product, found once per launch on the host (plan_factors): MUL
+// nodes are flattened, PHASE and SCALE nodes give a separable factor and pass their child on, and
+// every other LEAF and every ADD subtree is a factor of its own.
+enum { kFactorLeaf = 0, kFactorTree, kFactorSum, kFactorPhase, kFactorScale };
+struct FactorPlan {
+    int n;
+    int depth;                                    // of the evaluation stack
+    short o0[GSB_MAX_OPS], o1[GSB_MAX_OPS];       // ops of a leaf or subtree
+    unsigned char kind[GSB_MAX_OPS], arg[GSB_MAX_OPS];
+};
+
 struct DrawArgs {
     gsb_template tpl;
+    FactorPlan fac;
     int n_stamps;
     const gsb_leaf* leaves;
     const gsb_phase* phases;
@@ -90,6 +130,7 @@ struct DrawArgs {
     int add;
     double* added_flux;
     void* work;          // per-CTA W slabs when W does not fit in shared memory
+    int max_grid = 0;    // when > 0: CTAs for which `work` has a slab
 };
 
 __device__ inline int floor_div(int a, int n) { return a >= 0 ? a / n : -((-a + n - 1) / n); }
@@ -191,106 +232,124 @@ __device__ __forceinline__ bool want_leaf(unsigned want, int l) { return (want >
 __device__ __forceinline__ bool want_phase(unsigned want, int p) { return (want >> (8 + p)) & 1u; }
 __device__ __forceinline__ bool want_scale(unsigned want, int q) { return (want >> (16 + q)) & 1u; }
 
-// Split the program's root product into atoms (thread 0).  MUL nodes are flattened; PHASE and
-// SCALE nodes contribute a separable factor and pass their child on; a LEAF is separable when
-// its value is X(i) Y(j) (Box or Gaussian with a diagonal Jacobian: the reference's 1-d fill);
-// every other LEAF and every ADD subtree is an atom evaluated per point.  Factors named in
-// `want` (the adjoint's differentiated records) are not folded: a wanted separable leaf stays a
-// leaf atom, a wanted phase or scale becomes an atom of its own.  Returns false when the atoms
-// do not fit the fixed arrays (the program is then evaluated unfactored).
-__device__ inline bool plan_factored(StampSmem& S, const gsb_template& tpl, unsigned want = 0u)
+// The factor list of a template (host).
+inline void plan_factors(const gsb_template& tpl, FactorPlan& P)
 {
-    short c1[GSB_MAX_OPS], c2[GSB_MAX_OPS], start[GSB_MAX_OPS];
-    short st[GSB_MAX_OPS];
+    short c1[GSB_MAX_OPS], c2[GSB_MAX_OPS], start[GSB_MAX_OPS], st[GSB_MAX_OPS];
     int sp = 0;
+    P.n = 0;
+    P.depth = 0;
     for (int o = 0; o < tpl.n_ops; ++o) {
         const int code = tpl.op_code[o];
         c1[o] = c2[o] = -1;
         if (code == GSB_OP_LEAF) {
-            start[o] = o;
-            st[sp++] = o;
+            start[o] = short(o);
+            st[sp++] = short(o);
         } else if (code == GSB_OP_MUL || code == GSB_OP_ADD) {
             c2[o] = st[--sp];
             c1[o] = st[sp - 1];
             start[o] = start[c1[o]];
-            st[sp - 1] = o;
+            st[sp - 1] = short(o);
         } else {
             c1[o] = st[sp - 1];
             start[o] = start[c1[o]];
-            st[sp - 1] = o;
+            st[sp - 1] = short(o);
         }
+        P.depth = std::max(P.depth, sp);
     }
-    for (int l = 0; l < GSB_MAX_LEAVES; ++l) S.leaf_sep[l] = 0;
-    for (int p = 0; p < GSB_MAX_PHASES; ++p) S.phase_sep[p] = 0;
-    for (int q = 0; q < GSB_MAX_SCALES; ++q) S.scale_sep[q] = 0;
-    S.n_atoms = 0;
     sp = 0;
-    st[sp++] = tpl.n_ops - 1;
+    st[sp++] = short(tpl.n_ops - 1);
     while (sp > 0) {
         const int o = st[--sp];
-        const int code = tpl.op_code[o], arg = tpl.op_arg[o];
+        const int code = tpl.op_code[o];
         if (code == GSB_OP_MUL) {
             st[sp++] = c1[o];
             st[sp++] = c2[o];
-        } else if (code == GSB_OP_PHASE || code == GSB_OP_SCALE) {
-            const bool ph = code == GSB_OP_PHASE;
-            if (ph ? want_phase(want, arg) : want_scale(want, arg)) {
-                S.atom_o0[S.n_atoms] = o;
-                S.atom_o1[S.n_atoms] = o + 1;
-                S.atom_kind[S.n_atoms] = ph ? kAtomPhase : kAtomScale;
-                S.atom_arg[S.n_atoms] = (unsigned char)arg;
-                ++S.n_atoms;
-            } else if (ph) {
-                S.phase_sep[arg] = 1;
-            } else {
-                S.scale_sep[arg] = 1;
-            }
+            continue;
+        }
+        const int f = P.n++;
+        P.o0[f] = short(o);
+        P.o1[f] = short(o + 1);
+        P.arg[f] = (unsigned char)tpl.op_arg[o];
+        if (code == GSB_OP_PHASE || code == GSB_OP_SCALE) {
+            P.kind[f] = code == GSB_OP_PHASE ? kFactorPhase : kFactorScale;
             st[sp++] = c1[o];
+        } else if (code == GSB_OP_LEAF) {
+            P.kind[f] = kFactorLeaf;
         } else {
-            if (code == GSB_OP_LEAF && !want_leaf(want, arg)) {
-                const LeafParams& L = S.leaf[arg];
-                if ((L.type == GSB_BOX || L.type == GSB_GAUSSIAN) && !(L.flags & GSB_LEAF_JAC_GENERAL)) {
-                    S.leaf_sep[arg] = 1;
-                    continue;
-                }
-            }
-            bool sum = code == GSB_OP_ADD;
+            bool sum = true;
             for (int q = start[o]; q <= o && sum; ++q)
                 sum = tpl.op_code[q] == GSB_OP_LEAF || tpl.op_code[q] == GSB_OP_ADD;
-            S.atom_o0[S.n_atoms] = start[o];
-            S.atom_o1[S.n_atoms] = o + 1;
-            S.atom_kind[S.n_atoms] = sum ? kAtomSum : kAtomRange;
-            S.atom_arg[S.n_atoms] = (unsigned char)(code == GSB_OP_LEAF ? arg : 0);
-            ++S.n_atoms;
+            P.o0[f] = start[o];
+            P.kind[f] = sum ? kFactorSum : kFactorTree;
         }
     }
-    return true;
 }
 
+// Sort the factors into atoms and folded separable ones (thread 0).  A leaf is separable when its
+// value is X(i) Y(j) (Box or Gaussian with a diagonal Jacobian: the reference's 1-d fill).  Factors
+// named in `want` (the adjoint's differentiated records) are not folded: a wanted separable leaf
+// stays a leaf atom, a wanted phase or scale becomes an atom of its own.
+__device__ inline void plan_factored(StampSmem& S, const gsb_template& tpl, const FactorPlan& P, unsigned want = 0u)
+{
+    int n = 0, nl = 0, no = 0;
+    for (int f = 0; f < P.n; ++f) {
+        const int kind = P.kind[f], arg = P.arg[f];
+        if (kind == kFactorPhase && !want_phase(want, arg)) { S.phase_sep[arg] = 1; continue; }
+        if (kind == kFactorScale && !want_scale(want, arg)) { S.scale_sep[arg] = 1; continue; }
+        if (kind == kFactorLeaf && !want_leaf(want, arg)) {
+            const LeafParams& L = S.leaf[arg];
+            if ((L.type == GSB_BOX || L.type == GSB_GAUSSIAN) && !(L.flags & GSB_LEAF_JAC_GENERAL)) {
+                S.leaf_sep[arg] = 1;
+                continue;
+            }
+        }
+        S.atom_o0[n] = P.o0[f];
+        S.atom_o1[n] = P.o1[f];
+        S.atom_kind[n] = kind == kFactorPhase ? kAtomPhase : kind == kFactorScale ? kAtomScale
+                         : kind == kFactorSum ? kAtomSum : kAtomRange;
+        S.atom_arg[n] = (unsigned char)(kind == kFactorTree || kind == kFactorSum ? 0 : arg);
+        bool real = kind == kFactorSum || kind == kFactorLeaf;
+        for (int o = P.o0[f]; o < P.o1[f] && real; ++o)
+            real = !(tpl.op_code[o] == GSB_OP_LEAF && tpl.leaf_type[tpl.op_arg[o]] == GSB_INTERPOLATED);
+        if (real) {
+            for (int o = P.o0[f]; o < P.o1[f]; ++o)
+                if (tpl.op_code[o] == GSB_OP_LEAF) {
+                    S.real_leaf[nl] = tpl.op_arg[o];
+                    S.real_last[nl++] = 0;
+                }
+            S.real_last[nl - 1] = 1;
+        } else {
+            S.other[no++] = (unsigned char)n;
+        }
+        ++n;
+    }
+    S.n_atoms = n;
+    S.n_real = nl;
+    S.n_other = no;
+}
+
+// Trapezoid nodes of the Moffat sum (moffat_nodes).
+constexpr int kMoffatNodes = 64;
+constexpr double kMoffatTau = 0.25;
+
 template <typename T, bool II = true>
-__device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, int Nk, unsigned want = 0u,
-                                   int budget = kCacheBytes)
+__device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, const FactorPlan& fac, int Nk,
+                                   unsigned want = 0u, int budget = kCacheBytes)
 {
     const int hk = Nk / 2;
     int used = 0;
-    int depth = 0, maxd = 0;
-    for (int o = 0; o < tpl.n_ops; ++o) {
-        const int c = tpl.op_code[o];
-        if (c == GSB_OP_LEAF) ++depth;
-        else if (c == GSB_OP_MUL || c == GSB_OP_ADD) --depth;
-        maxd = depth > maxd ? depth : maxd;
-    }
-    S.regstack = maxd <= 4;
+    S.regstack = fac.depth <= 4;
     S.xy_cache = -1;
+    for (int l = 0; l < tpl.n_leaves; ++l) S.leaf_sep[l] = 0;
+    for (int p = 0; p < tpl.n_phases; ++p) S.phase_sep[p] = 0;
+    for (int q = 0; q < tpl.n_scales; ++q) S.scale_sep[q] = 0;
     {
         const int bytes = ((hk + 1 + Nk + 1) * (int)sizeof(Cx<T>) + 15) & ~15;
-        if (S.regstack && bytes <= budget && plan_factored(S, tpl, want)) {
+        if (S.regstack && bytes <= budget) {
+            plan_factored(S, tpl, fac, want);
             S.xy_cache = used;
             used += bytes;
-        } else {
-            for (int l = 0; l < GSB_MAX_LEAVES; ++l) S.leaf_sep[l] = 0;
-            for (int p = 0; p < GSB_MAX_PHASES; ++p) S.phase_sep[p] = 0;
-            for (int q = 0; q < GSB_MAX_SCALES; ++q) S.scale_sep[q] = 0;
         }
     }
     for (int l = 0; l < tpl.n_leaves; ++l) {
@@ -324,14 +383,165 @@ __device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, int Nk
         const int bytes = ((hk + 1 + Nk + 1) * (int)sizeof(T) + 15) & ~15;
         if (used + bytes <= budget) { S.leaf_cache[l] = used; used += bytes; }
     }
+    for (int l = 0; l < tpl.n_leaves; ++l) {
+        S.aux_cache[l] = -1;
+        const LeafParams& L = S.leaf[l];
+        int bytes = 0;
+        if (L.type == GSB_EXPONENTIAL) bytes = ((Nk + 1) * (int)sizeof(ushort2) + 15) & ~15;
+        else if (L.type == GSB_MOFFAT && sizeof(T) == 4 && int(L.d[2]) == 0) bytes = kMoffatNodes * (int)sizeof(float2);
+        else continue;
+        if (hk < 65535 && used + bytes <= budget) { S.aux_cache[l] = used; used += bytes; }
+    }
+}
+
+template <typename T>
+__device__ __forceinline__ LeafT<T>& leaf_const(StampSmem& S, int l)
+{ return *reinterpret_cast<LeafT<T>*>(&S.leaf_t[l]); }
+template <typename T>
+__device__ __forceinline__ const LeafT<T>& leaf_const(const StampSmem& S, int l)
+{ return *reinterpret_cast<const LeafT<T>*>(&S.leaf_t[l]); }
+
+// The constants of leaf l in the working precision (one thread per leaf, after plan_caches).
+//
+// Float arithmetic drawn into a double image (drawImage's default precision with an ImageD) keeps
+// the general path for the profiles whose fast form rounds differently: the double image shows the
+// last bit of every operation, and its users compare such images across versions.
+template <typename T>
+__device__ __noinline__ void set_leaf_const(StampSmem& S, int l, double dk, bool mixed)
+{
+    const LeafParams& L = S.leaf[l];
+    LeafT<T>& t = leaf_const<T>(S, l);
+    t.kind = kLeafGeneric;
+    t.cache = -1;
+    t.n = 0;
+    t.flux = T(L.flux);
+    double size = 1.;
+    if (S.leaf_cache[l] >= 0) {
+        t.kind = kLeafSep;
+        t.cache = S.leaf_cache[l];
+    } else if (L.type == GSB_EXPONENTIAL && S.aux_cache[l] >= 0) {
+        // (the general path's own order of operations: k = (i dk, j dk), then r0 squared)
+        t.kind = kLeafExp;
+        t.cache = S.aux_cache[l];
+        t.q[0] = T(L.d[0]);
+        t.q[1] = T(dk);
+        t.a = T(L.jac[0]);
+        t.b = T(L.jac[1]);
+        t.c = T(L.jac[2]);
+        t.d = T(L.jac[3]);
+        return;
+    } else if (L.type == GSB_SERSIC && S.sersic_cache[l] >= 0) {
+        const SersicTableView& v = S.sersic[l];
+        t.kind = kLeafSersic;
+        t.cache = S.sersic_cache[l];
+        t.n = v.n;
+        size = L.d[0];
+        t.q[0] = T(v.ksq_min);
+        t.q[1] = T(v.ksq_max);
+        t.q[2] = T(v.kderiv2);
+        t.q[3] = T(v.kderiv4);
+        t.q[4] = T(v.highk_a);
+        t.q[5] = T(v.highk_b);
+        t.q[6] = T(v.da);
+        t.q[7] = T(1. / v.da);
+        t.q[8] = T(0.34657359027997264 / v.da);          // node coordinate + 1/2: log2(k^2) q8 + q9
+        t.q[9] = T(0.5 - v.front / v.da);
+    } else if (L.type == GSB_MOFFAT) {
+        const int mode = int(L.d[2]);
+        size = L.d[0];
+        t.flux = T(L.d[1]);
+        if (mode >= 1 && mode <= 3 && sizeof(T) == 4 && !mixed) {
+            t.kind = kLeafMoffat1 + mode - 1;
+        } else if (mode == 0 && S.aux_cache[l] >= 0) {
+            // terms a point at x needs: up to cosh t = 1 + B / x, B = 19 + nu ln 2B bounding the rest by 2e-9 of
+            // the sum.  The smallest x of the grid sets the node count.
+            const float nu = float(L.d[3]);
+            float B = 20.f;
+            for (int it = 0; it < 6; ++it) B = 19.f + nu * __logf(2.f * B);
+            const float j0 = float(L.jac[0]), j1 = float(L.jac[1]), j2 = float(L.jac[2]), j3 = float(L.jac[3]);
+            const float det = fabsf(j0 * j3 - j1 * j2);
+            const float fro = sqrtf(j0 * j0 + j1 * j1 + j2 * j2 + j3 * j3);
+            const float xmin = float(dk * size) * det / fro;      // <= dk rD times the smaller singular value
+            const float tend = __logf(2.f + 2.f * B / xmin);
+            const int need = int(tend * float(1. / kMoffatTau)) + 2;
+            // the weights cosh(nu t) stay within FP32, and the nodes within the cache
+            if (!mixed && xmin > 0.f && need <= kMoffatNodes && nu * tend < 80.f) {
+                t.kind = kLeafMoffatSum;
+                t.cache = S.aux_cache[l];
+                t.n = need;
+                t.q[0] = T(nu);
+                t.q[1] = T(2.f * B);
+            }
+        }
+    } else if (L.type == GSB_KOLMOGOROV && sizeof(T) == 4 && !mixed) {
+        t.kind = kLeafKolm;
+        size = L.d[0];
+    } else if (L.type == GSB_AIRY && sizeof(T) == 4 && !mixed) {
+        t.kind = kLeafAiry;
+        size = L.d[0];
+        t.flux = T(L.d[1]);
+        t.q[0] = T(L.d[2]);
+        t.q[1] = T(L.d[3]);
+    }
+    size *= dk;
+    t.a = T(L.jac[0] * size);
+    t.b = T(L.jac[1] * size);
+    t.c = T(L.jac[2] * size);
+    t.d = T(L.jac[3] * size);
+}
+
+// Columns [lo, hi) of row j that survive the Exponential's clip (exponential_keep, which keeps a
+// range of columns in every row).
+static __device__ __noinline__ ushort2 exponential_columns(const LeafParams& L, double dk, int hk, int j)
+{
+    const double r0 = L.d[0], ksqmax = L.d[1], kmax = L.d[2];
+    int i1, i2;
+    if (!(L.flags & GSB_LEAF_JAC_GENERAL)) {
+        const double A = L.jac[0], D = L.jac[3];
+        const int jq = j < 0 ? -j : j;
+        kvalue_range_1d(hk + 1, kmax, ksqmax, 0., dk * A * r0, jq * (dk * D * r0), i1, i2);
+    } else {
+        const double A = L.jac[0], B = L.jac[1], C = L.jac[2], D = L.jac[3];
+        const double y0 = -hk * dk;
+        const double kx0 = (C * y0) * r0 + (j + hk) * (C * dk * r0);
+        const double ky0 = (D * y0) * r0 + (j + hk) * (D * dk * r0);
+        kvalue_range_2d(hk + 1, kmax, ksqmax, kx0, A * dk * r0, ky0, B * dk * r0, i1, i2);
+    }
+    if (i1 >= i2) return make_ushort2(0, 0);
+    return make_ushort2((unsigned short)(i1 < 0 ? 0 : i1), (unsigned short)(i2 > hk + 1 ? hk + 1 : i2));
+}
+
+// Node j of the Moffat sum: (log2(e) cosh t_j, w_j).
+static __device__ __noinline__ float2 moffat_node(double nu, double lognorm, int j)
+{
+    const double t = j * kMoffatTau;
+    const double w = 0.5 * kMoffatTau * (exp(lognorm + nu * t) + exp(lognorm - nu * t));
+    return make_float2(float(cosh(t) * 1.4426950408889634), float(j == 0 ? 0.5 * w : w));
 }
 
 // Fill the planned caches (whole block).
 template <typename T, bool II = true>
-__device__ inline void fill_caches(const StampSmem& S, const gsb_template& tpl, unsigned char* cache,
-                                   double dk, int Nk)
+__device__ inline void fill_caches(StampSmem& S, const gsb_template& tpl, unsigned char* cache,
+                                   double dk, int Nk, bool mixed = false)
 {
     const int hk = Nk / 2;
+    // (the last warp forms the constants and the one before it the Moffat nodes, while the first
+    // ones start on the tables)
+    const int back = int(blockDim.x) - 1 - int(threadIdx.x);
+    if (back < tpl.n_leaves) set_leaf_const<T>(S, back, dk, mixed);
+    for (int l = 0; l < tpl.n_leaves; ++l) {
+        if (S.aux_cache[l] < 0) continue;
+        const LeafParams& L = S.leaf[l];
+        if (L.type == GSB_EXPONENTIAL) {
+            ushort2* R = reinterpret_cast<ushort2*>(cache + S.aux_cache[l]);
+            for (int t = threadIdx.x; t < Nk + 1; t += blockDim.x) R[t] = exponential_columns(L, dk, hk, t - hk);
+        } else {
+            // c_nu x^nu K_nu(x) = x^nu sum_j w_j exp(-x cosh t_j)  (moffat_kv), w_j = e^lognorm tau cosh(nu t_j)
+            float2* E = reinterpret_cast<float2*>(cache + S.aux_cache[l]);
+            for (int t = back - 32; t < kMoffatNodes; t += blockDim.x)
+                if (t >= 0) E[t] = moffat_node(L.d[3], L.d[4], t);
+        }
+    }
     for (int l = 0; l < tpl.n_leaves; ++l) {
         if (II && S.ii_cache[l] >= 0) {
             const LeafParams& L = S.leaf[l];
@@ -442,32 +652,200 @@ __device__ inline T sersic_kvalue_smem(const SersicTableView& tb, const typename
     return num / h / ksq;
 }
 
+// Flush-to-zero hardware approximations (one instruction each: the accurate forms' scaling for
+// denormal arguments and results is not needed, a k-value below 1e-38 being 0 of the flux).
+__device__ __forceinline__ float fast_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float fast_log2(float x) { float y; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float fast_rcp(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float fast_rsqrt(float x) { float y; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+__device__ __forceinline__ float fast_sqrt(float x) { float y; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+
+// Sersic FT at V points from the shared-memory nodes (FP32).  One reciprocal of k^2 serves the node
+// offset and both divisions; the offset's logarithm is a series in the ratio's excess over 1 (an
+// exact difference) where the table is fine enough for its degree; the interval comes from the
+// hardware logarithm (a point within rounding of a node may take the neighbouring cubic, which
+// agrees there to third order).
+template <int V>
+__device__ __forceinline__ void sersic_points(const LeafT<float>& L, const unsigned char* cache,
+                                              const float (&ksq)[V], float (&out)[V])
+{
+    const float4* node = reinterpret_cast<const float4*>(cache + L.cache);
+    const float kmin = L.q[0], kmax = L.q[1], h = L.q[6], inv_h = L.q[7], is = L.q[8], io = L.q[9];
+    const int last = L.n - 1;
+    const bool fine = h < 0.04f;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const float k2 = ksq[v];
+        const float inv = fast_rcp(k2);
+        // i = ceil of the node coordinate: the coordinate + 1/2 rounded by adding 1.5 * 2^23
+        const int i = max(1, min(__float_as_int(fmaf(fast_log2(k2), is, io) + 12582912.f) - 0x4b400000, last));
+        const float4 n0 = node[i - 1], n1 = node[i];
+        const float e = (n1.w - k2) * inv;       // k_i^2 / k^2 - 1
+        float aa;
+        if (fine) {
+            // ln(1 + e) / 2, |e| < 0.084: the series to e^8 (next term 1.2e-11)
+            float p = fmaf(e, -1.f / 16.f, 1.f / 14.f);
+            p = fmaf(e, p, -1.f / 12.f);
+            p = fmaf(e, p, 0.1f);
+            p = fmaf(e, p, -0.125f);
+            p = fmaf(e, p, 1.f / 6.f);
+            p = fmaf(e, p, -0.25f);
+            p = fmaf(e, p, 0.5f);
+            aa = e * p;
+        } else {
+            aa = 0.5f * logf(n1.w * inv);
+        }
+        const float bb = h - aa;
+        const float cub = aa * bb * fmaf(aa + h, n0.z, (bb + h) * n1.z);
+        float r = fmaf(cub, -1.f / 6.f, fmaf(aa, n0.y, bb * n1.y)) * inv_h * inv;
+        if (!(k2 >= kmin && k2 < kmax)) {
+            if (k2 >= kmax) r = fmaf(L.q[5], fast_rsqrt(k2), L.q[4]) * inv;
+            else r = fmaf(k2, fmaf(k2, L.q[3], L.q[2]), 1.f);
+        }
+        out[v] = r;
+    }
+}
+
+// x^nu sum_j w_j exp(-x cosh t_j) at V points, x^2 given (1 at x = 0).
+template <int V>
+__device__ __forceinline__ void moffat_sum_points(const LeafT<float>& L, const unsigned char* cache,
+                                                  const float (&xsq)[V], float (&out)[V])
+{
+    const float2* E = reinterpret_cast<const float2*>(cache + L.cache);
+    float sum[V], x[V], xs = 1e30f;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        sum[v] = 0.f;
+        x[v] = sqrtf(xsq[v]);
+        if (x[v] > 0.f) xs = fminf(xs, x[v]);
+    }
+    // the smallest x of the V needs the most nodes: cosh t up to 1 + B / x
+    const float need = fast_log2(fmaf(L.q[1], fast_rcp(xs), 2.f)) * float(0.6931471805599453 / kMoffatTau);
+    const int nj = min(L.n, int(need) + 2);
+    for (int j = 0; j < nj; ++j) {
+        const float2 e = E[j];
+#pragma unroll
+        for (int v = 0; v < V; ++v) sum[v] = fmaf(e.y, fast_exp2(-x[v] * e.x), sum[v]);
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) out[v] = x[v] > 0.f ? sum[v] * exp2f(L.q[0] * log2f(x[v])) : 1.f;
+}
+
+// Real leaf l at the V points (i, j0 + v js) with the shared-memory caches, the leaf's flux included.
+template <typename T, int V>
+__device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned char* cache, int l, int i, int j0,
+                                            int js, int hk, double dk, T (&out)[V])
+{
+    const LeafT<T>& L = leaf_const<T>(S, l);
+    const int kind = L.kind;
+    if (kind == kLeafGeneric) {
+        const GridRef g{dk, 0, -hk, hk + 1, 2 * hk + 1};
+        const T kx = T(i) * T(dk);
+#pragma unroll 1
+        for (int v = 0; v < V; ++v) {
+            const int j = j0 + v * js;
+            const T val = leaf_kvalue<T>(S.leaf[l], S.sersic, kx, T(j) * T(dk), g, i, j + hk);
+#pragma unroll
+            for (int w = 0; w < V; ++w) if (w == v) out[w] = val;
+        }
+        return;
+    }
+    const T flux = L.flux;
+    if (kind == kLeafSep) {
+        const T* X = reinterpret_cast<const T*>(cache + L.cache);
+        const T x = flux * X[i];
+#pragma unroll
+        for (int v = 0; v < V; ++v) out[v] = x * X[hk + 1 + hk + j0 + v * js];
+        return;
+    }
+    const T jf = T(j0), jd = T(js);
+    if constexpr (sizeof(T) == 8) {
+        // (double: the remaining kinds gain nothing over the general path but its conversions)
+        if (kind == kLeafSersic) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const T j = jf + T(v) * jd, u = L.a * T(i) + L.c * j, w = L.b * T(i) + L.d * j;
+                out[v] = flux * sersic_kvalue_smem<T>(
+                                    S.sersic[l], reinterpret_cast<const typename NodeT<T>::type*>(cache + L.cache), u * u + w * w);
+            }
+            return;
+        }
+    }
+    if (kind == kLeafExp) {
+        // flux / (1 + k^2 r0^2)^(3/2) where the clip keeps it
+        const ushort2* R = reinterpret_cast<const ushort2*>(cache + L.cache) + hk + j0;
+        const T r0 = L.q[0], tdk = L.q[1], kx = T(i) * tdk;
+        const T A = L.a, B = L.b, C = L.c, D = L.d;
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            const ushort2 r = R[v * js];
+            const T ky = (jf + T(v) * jd) * tdk;
+            const T u = A * kx + C * ky;
+            const T w = B * kx + D * ky;
+            const T q = T(1) + (u * u + w * w) * r0 * r0;
+            const T val = flux / (q * sqrt(q));
+            out[v] = i >= int(r.x) && i < int(r.y) ? val : T(0);
+        }
+        return;
+    }
+    if constexpr (sizeof(T) == 4) {
+        float ksq[V];
+        {
+            const float ui = L.a * float(i), wi = L.b * float(i), c = L.c, d = L.d;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const float j = jf + float(v) * jd;
+                const float u = ui + c * j, w = wi + d * j;
+                ksq[v] = u * u + w * w;
+            }
+        }
+        if (kind == kLeafSersic) {
+            sersic_points<V>(L, cache, ksq, out);
+        } else if (kind == kLeafKolm) {
+            // exp(-(k^2)^(5/6)); log2 of 0 is -inf, and its power 0
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                out[v] = fast_exp2(-1.44269504f * fast_exp2(fast_log2(ksq[v]) * (5.f / 6.f)));
+        } else if (kind == kLeafMoffatSum) {
+            moffat_sum_points<V>(L, cache, ksq, out);
+        } else if (kind == kLeafAiry) {
+#pragma unroll 1
+            for (int v = 0; v < V; ++v) {
+                float k2 = ksq[0];
+#pragma unroll
+                for (int w = 1; w < V; ++w) if (w == v) k2 = ksq[w];
+                const float val = airy_kvalue<float>(k2, L.q[0], L.q[1]);
+#pragma unroll
+                for (int w = 0; w < V; ++w) if (w == v) out[w] = val;
+            }
+        } else {
+            // Moffat beta = 1.5, 2.5, 3.5: exp(-k) times 1, 1 + k, 1 + k + k^2 / 3
+            const float c1 = kind == kLeafMoffat1 ? 0.f : 1.f, c2 = kind == kLeafMoffat3 ? 1.f / 3.f : 0.f;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const float k = sqrtf(ksq[v]);
+                out[v] = expf(-k) * (1.f + k * (c1 + k * c2));
+            }
+        }
+#pragma unroll
+        for (int v = 0; v < V; ++v) out[v] *= flux;
+    }
+}
+
 // One leaf at k index (i, j) with the shared-memory caches.
 template <typename T>
-__device__ __forceinline__ T leaf_fast(const StampSmem& S, const unsigned char* cache, int arg, T kx, T ky,
-                                       int i, int j, const GridRef& g)
+__device__ __noinline__ T leaf_fast(const StampSmem& S, const unsigned char* cache, int arg, int i, int j, int hk,
+                                    double dk)
 {
-    const int hk = g.n / 2;
-    const LeafParams& L = S.leaf[arg];
-    if (S.leaf_cache[arg] >= 0) {
-        const T* X = reinterpret_cast<const T*>(cache + S.leaf_cache[arg]);
-        return T(L.flux) * X[i] * X[hk + 1 + j + hk];
-    }
-    if (S.sersic_cache[arg] >= 0) {
-        const T A = T(L.jac[0]), B = T(L.jac[1]), C = T(L.jac[2]), D = T(L.jac[3]);
-        const T kxp = A * kx + C * ky, kyp = B * kx + D * ky;
-        const T r0 = T(L.d[0]);
-        return T(L.flux) * sersic_kvalue_smem<T>(
-                   S.sersic[arg], reinterpret_cast<const typename NodeT<T>::type*>(cache + S.sersic_cache[arg]),
-                   (kxp * kxp + kyp * kyp) * r0 * r0);
-    }
-    return leaf_kvalue<T>(L, S.sersic, kx, ky, g, i - g.x0, j - g.y0);
+    T out[1];
+    leaf_points<T, 1>(S, cache, arg, i, j, 0, hk, dk, out);
+    return out[0];
 }
 
 // One leaf as a complex value: InterpolatedImage leaves are complex, the others real.
 template <typename T, bool II = true>
-__device__ __forceinline__ Cx<T> leaf_cfast(const StampSmem& S, const unsigned char* cache, int arg, T kx, T ky,
-                                            int i, int j, const GridRef& g)
+__device__ __forceinline__ Cx<T> leaf_cfast(const StampSmem& S, const unsigned char* cache, int arg, int i, int j,
+                                            const GridRef& g)
 {
     if (II && S.leaf[arg].type == GSB_INTERPOLATED) {
         if (S.ii_cache[arg] >= 0) {
@@ -477,24 +855,23 @@ __device__ __forceinline__ Cx<T> leaf_cfast(const StampSmem& S, const unsigned c
         }
         return ii_kvalue<T>(S.leaf[arg], g.dk, i, j);
     }
-    return cx<T>(leaf_fast<T>(S, cache, arg, kx, ky, i, j, g), T(0));
+    return cx<T>(leaf_fast<T>(S, cache, arg, i, j, g.n / 2, g.dk), T(0));
 }
 
 // Evaluation of the ops [o0, o1) (a complete subtree, or the whole program) with the caches and
 // a 4-deep register stack (warp-uniform branches).
 template <typename T, bool II = true>
-__device__ __forceinline__ Cx<T> eval_range(const gsb_template& tpl, const StampSmem& S,
+__device__ __noinline__ Cx<T> eval_range(const gsb_template& tpl, const StampSmem& S,
                                             const unsigned char* cache, double dk, int i, int j,
                                             const GridRef& g, int o0, int o1)
 {
     const int hk = g.n / 2;
     Cx<T> s0 = cx<T>(T(0), T(0)), s1 = s0, s2 = s0, s3 = s0;
     int sp = 0;
-    const T kx = T(i) * T(dk), ky = T(j) * T(dk);
     for (int o = o0; o < o1; ++o) {
         const int code = tpl.op_code[o], arg = tpl.op_arg[o];
         if (code == GSB_OP_LEAF) {
-            const Cx<T> c = leaf_cfast<T, II>(S, cache, arg, kx, ky, i, j, g);
+            const Cx<T> c = leaf_cfast<T, II>(S, cache, arg, i, j, g);
             if (sp == 0) s0 = c; else if (sp == 1) s1 = c; else if (sp == 2) s2 = c; else s3 = c;
             ++sp;
         } else if (code == GSB_OP_MUL || code == GSB_OP_ADD) {
@@ -529,38 +906,94 @@ __device__ __forceinline__ Cx<T> eval_range(const gsb_template& tpl, const Stamp
     return s0;
 }
 
-template <typename T, bool II = true>
-__device__ __forceinline__ Cx<T> eval_fast(const gsb_template& tpl, const StampSmem& S,
-                                           const unsigned char* cache, double dk, int i, int j,
-                                           const GridRef& g)
-{
-    return eval_range<T, II>(tpl, S, cache, dk, i, j, g, 0, tpl.n_ops);
-}
+// The factored program at the V points (i, j0 + v js): the folded separable factors XS[i] YS[j + hk]
+// times the atoms.  Taking V points through each atom at a time shares the program's control flow
+// and the atoms' constants, and gives the latencies V independent chains to overlap.  (A function
+// call per V points, so that the kernels of all sizes share one compiled body.)
+template <typename T, int V> struct Values { Cx<T> v[V]; };
 
-// The factored program at (i, j): product of the per-point atoms (real leaves, complex
-// subtrees) times the folded separable factors XS[i] YS[j + hk].
-template <typename T, bool II = true>
-__device__ __forceinline__ Cx<T> eval_factored(const gsb_template& tpl, const StampSmem& S,
-                                               const unsigned char* cache, double dk, int i, int j,
-                                               const GridRef& g)
+template <typename T, bool II, int V>
+__device__ __forceinline__ Values<T, V> eval_points_inline(const gsb_template& tpl, const StampSmem& S,
+                                                           const unsigned char* cache, int i, int j0, int js, int hk,
+                                                           double dk)
 {
-    const int hk = g.n / 2;
-    const T kx = T(i) * T(dk), ky = T(j) * T(dk);
-    T r = T(1);
-    Cx<T> c = cx<T>(T(1), T(0));
-    for (int a = 0; a < S.n_atoms; ++a) {
-        const int o0 = S.atom_o0[a], o1 = S.atom_o1[a];
-        if (o1 - o0 == 1) {
-            const int l = tpl.op_arg[o0];
-            if (II && S.leaf[l].type == GSB_INTERPOLATED) c = cmul<T>(c, leaf_cfast<T, II>(S, cache, l, kx, ky, i, j, g));
-            else r *= leaf_fast<T>(S, cache, l, kx, ky, i, j, g);
-        } else {
-            c = cmul<T>(c, eval_range<T, II>(tpl, S, cache, dk, i, j, g, o0, o1));
+    Values<T, V> res;
+    T r[V], sum[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) { r[v] = T(1); sum[v] = T(0); }
+    const int nr = S.n_real;
+#pragma unroll 1
+    for (int q = 0; q < nr; ++q) {
+        T t[V];
+        leaf_points<T, V>(S, cache, S.real_leaf[q], i, j0, js, hk, dk, t);
+        const bool last = S.real_last[q];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            sum[v] += t[v];
+            if (last) { r[v] *= sum[v]; sum[v] = T(0); }
         }
     }
     const Cx<T>* XS = reinterpret_cast<const Cx<T>*>(cache + S.xy_cache);
-    const Cx<T> xy = cmul<T>(XS[i], XS[hk + 1 + j + hk]);
-    return cscale<T>(cmul<T>(c, xy), r);
+    const Cx<T>* YS = XS + hk + 1 + hk + j0;
+    const Cx<T> x = XS[i];
+    const int no = S.n_other;
+    if (no == 0) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) res.v[v] = cscale<T>(cmul<T>(x, YS[v * js]), r[v]);
+        return res;
+    }
+    const GridRef g{dk, 0, -hk, hk + 1, 2 * hk + 1};
+#pragma unroll 1
+    for (int v = 0; v < V; ++v) {
+        const int j = j0 + v * js;
+        Cx<T> c = cx<T>(T(1), T(0));
+        for (int q = 0; q < no; ++q) {
+            const int a = S.other[q], o0 = S.atom_o0[a], o1 = S.atom_o1[a];
+            c = cmul<T>(c, o1 - o0 == 1 ? leaf_cfast<T, II>(S, cache, S.atom_arg[a], i, j, g)
+                                        : eval_range<T, II>(tpl, S, cache, dk, i, j, g, o0, o1));
+        }
+        T rv = r[0];
+#pragma unroll
+        for (int w = 1; w < V; ++w) if (w == v) rv = r[w];
+        const Cx<T> z = cscale<T>(cmul<T>(c, cmul<T>(x, YS[v * js])), rv);
+#pragma unroll
+        for (int w = 0; w < V; ++w) if (w == v) res.v[w] = z;
+    }
+    return res;
+}
+
+template <typename T, bool II, int V>
+__device__ __noinline__ Values<T, V> eval_points(const gsb_template& tpl, const StampSmem& S,
+                                                 const unsigned char* cache, int i, int j0, int js, int hk, double dk)
+{
+    return eval_points_inline<T, II, V>(tpl, S, cache, i, j0, js, hk, dk);
+}
+
+// V points of the program, by the best of its three forms.  INL: compiled into the caller.
+template <typename T, bool II, int V, bool INL = false>
+__device__ __forceinline__ Values<T, V> eval_any(const gsb_template& tpl, const StampSmem& S,
+                                                 const unsigned char* cache, int i, int j0, int js, int hk, double dk)
+{
+    if (S.xy_cache >= 0)
+        return INL ? eval_points_inline<T, II, V>(tpl, S, cache, i, j0, js, hk, dk)
+                   : eval_points<T, II, V>(tpl, S, cache, i, j0, js, hk, dk);
+    const GridRef g{dk, 0, -hk, hk + 1, 2 * hk + 1};
+    Values<T, V> res;
+#pragma unroll 1
+    for (int v = 0; v < V; ++v) {
+        const Cx<T> z = S.regstack ? eval_range<T, II>(tpl, S, cache, dk, i, j0 + v * js, g, 0, tpl.n_ops)
+                                   : eval_program<T, II>(tpl, S, dk, i, j0 + v * js, g);
+#pragma unroll
+        for (int w = 0; w < V; ++w) if (w == v) res.v[w] = z;
+    }
+    return res;
+}
+
+template <typename T, bool II, bool INL = false>
+__device__ __forceinline__ Cx<T> eval_point(const gsb_template& tpl, const StampSmem& S, const unsigned char* cache,
+                                            int i, int j, int hk, double dk)
+{
+    return eval_any<T, II, 1, INL>(tpl, S, cache, i, j, 0, hk, dk).v[0];
 }
 
 // acc += v with Kahan's compensation term comp (componentwise).
@@ -613,6 +1046,12 @@ __host__ __device__ constexpr int fused_min_blocks()
     return kSmemPerSM / (smem_bytes<T, N>(w_fits_smem<T, N>()) + 1024) >= 2 ? 2 : 1;
 }
 
+// Bound by instruction issue and its latencies: of ~94 K warp instructions of a 64 x 64 stamp at
+// N = 128 the k-space evaluation takes half, the FFTs a sixth; issue slots 35 % active with the 16
+// warps that 128 registers leave.  Against one wave vector a lane with constants converted from the
+// FP64 records at each (179 K warp instructions): catalog stamps (Sersic x Kolmogorov) N = 128 1.36 ->
+// 1.11 ms, N = 192 1.00 -> 0.85; bulge + disk x Moffat (general beta) N = 128 5.4 -> 2.9, N = 192
+// 14.6 -> 6.0 ms, 16384 stamps.
 template <typename T, int N, bool WSMEM, bool II = true>
 __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, N>()) draw_fused_kernel(const __grid_constant__ DrawArgs a)
 {
@@ -644,41 +1083,110 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
         __syncthreads();
         const int Nk = S.geom.Nk;
         const int hk = Nk / 2;
-        const GridRef g{dk, 0, -hk, hk + 1, Nk + 1};
-        if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, Nk);
+        if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk);
         __syncthreads();
-        fill_caches<T, II>(S, a.tpl, cache, dk, Nk);
+        fill_caches<T, II>(S, a.tpl, cache, dk, Nk, sizeof(T) == 4 && a.out_dtype == GSB_F64);
         __syncthreads();
-        const bool fast = S.regstack;
-        const bool factored = S.xy_cache >= 0;
 
         // ---- column phase: wrapped k-values, inverse DFT along ky ----
-        for (int c = warp; c < H; c += NW) {
-            const int alo = ceil_div(-hk - c, N), ahi = floor_div(hk - c, N);
-            for (int r = lane; r < N; r += 32) {
-                const int kyc = r < N / 2 ? r : r - N;
-                const int blo = ceil_div(-hk - kyc, N), bhi = floor_div(hk - kyc, N);
-                // the fold (wrap) of the aliases, with Kahan compensation
-                Cx<T> acc = cx<T>(T(0), T(0)), comp = acc;
-                for (int ia = alo; ia <= ahi; ++ia) {
-                    const int kx = c + ia * N;
-                    for (int ib = blo; ib <= bhi; ++ib) {
-                        const int ky = kyc + ib * N;
-                        const bool pos = kx >= 0;
-                        const int ii = pos ? kx : -kx, jj = pos ? ky : -ky;
-                        Cx<T> v = factored ? eval_factored<T, II>(a.tpl, S, cache, dk, ii, jj, g)
-                                  : fast ? eval_fast<T, II>(a.tpl, S, cache, dk, ii, jj, g)
-                                         : eval_program<T, II>(a.tpl, S, dk, ii, jj, g);
-                        if (!pos) v = cconj<T>(v);
-                        kahan_add<T>(acc, comp, v);
+        if constexpr (N % 32 == 0) {
+            // A column's Nk + 1 rows ky = -hk .. hk go to the lanes in order, 32 a slot.  N is a multiple
+            // of 32, so slots s, s + N/32, ... of a lane are the aliases of one wrapped row: the lane
+            // folds them (with Kahan compensation) in registers, and a column costs
+            // ceil((Nk + 1) / 32) slots.  When Nk is a multiple of 32 (Nk = N above all) the last slot
+            // would hold the single point ky = hk: those points of all the warp's columns are taken
+            // together, one column a lane, before its columns.
+            constexpr int NS = N / 32;
+            constexpr int V = sizeof(T) == 8 ? (NS % 2 == 0 ? 2 : 1) : NS % 4 == 0 ? 4 : NS % 3 == 0 ? 3 : NS;
+            constexpr int COLS = (H + NW - 1) / NW;
+            const bool edge = COLS <= 32 && Nk % 32 == 0;
+            const int top = edge ? hk - 1 : hk;
+            const int edge_slot = edge ? (Nk % N) / 32 : -1;
+            Cx<T> edge_val = cx<T>(T(0), T(0));
+            if (edge) {
+                const int c = warp + lane * NW;
+                if (c < H) {
+                    for (int kx = c + ceil_div(-hk - c, N) * N; kx <= hk; kx += N) {
+                        const Cx<T> v = eval_point<T, II>(a.tpl, S, cache, kx >= 0 ? kx : -kx, kx >= 0 ? hk : -hk, hk, dk);
+                        edge_val = cadd<T>(edge_val, kx >= 0 ? v : cconj<T>(v));
                     }
                 }
-                buf[r] = acc;
+                __syncwarp();
             }
-            __syncwarp();
-            warp_fft<T, N, +1>(buf, tw);
-            for (int r = lane; r < N; r += 32) W[(size_t)c * WS + r] = buf[r];
-            __syncwarp();
+            int q = 0;
+            for (int c = warp; c < H; c += NW, ++q) {
+                const int kx0 = c + ceil_div(-hk - c, N) * N;
+                for (int s0 = 0; s0 < NS; s0 += V) {
+                    Cx<T> acc[V], comp[V];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) acc[v] = comp[v] = cx<T>(T(0), T(0));
+                    if (edge && edge_slot >= s0 && edge_slot < s0 + V) {
+                        const Cx<T> e = cx<T>(__shfl_sync(0xffffffffu, edge_val.x, q), __shfl_sync(0xffffffffu, edge_val.y, q));
+#pragma unroll
+                        for (int v = 0; v < V; ++v)
+                            if (lane == 0 && s0 + v == edge_slot) acc[v] = e;
+                    }
+                    // a lane's first value needs no compensation
+                    bool first = !(edge && edge_slot >= s0 && edge_slot < s0 + V);
+                    for (int kx = kx0; kx <= hk; kx += N) {
+                        const bool pos = kx >= 0;
+                        const int ii = pos ? kx : -kx;
+                        for (int e0 = -hk + 32 * s0; e0 <= top; e0 += N) {
+                            if (e0 + 32 * V - 1 <= top) {
+                                const int ky = e0 + lane;
+                                const Values<T, V> z = eval_any<T, II, V>(a.tpl, S, cache, ii, pos ? ky : -ky,
+                                                                          pos ? 32 : -32, hk, dk);
+#pragma unroll
+                                for (int v = 0; v < V; ++v) {
+                                    const Cx<T> w = pos ? z.v[v] : cconj<T>(z.v[v]);
+                                    if (first) acc[v] = w;
+                                    else kahan_add<T>(acc[v], comp[v], w);
+                                }
+                                first = false;
+                            } else {
+                                // the last, partial slots of the column (lanes beyond it repeat its end)
+#pragma unroll 1
+                                for (int u = 0; u < V && e0 + 32 * u <= top; ++u) {
+                                    const int ky = e0 + 32 * u + lane, kc = min(ky, top);
+                                    Cx<T> z = eval_point<T, II>(a.tpl, S, cache, ii, pos ? kc : -kc, hk, dk);
+                                    if (!pos) z = cconj<T>(z);
+                                    if (ky > top) z = cx<T>(T(0), T(0));
+#pragma unroll
+                                    for (int v = 0; v < V; ++v)
+                                        if (v == u) kahan_add<T>(acc[v], comp[v], z);
+                                }
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int v = 0; v < V; ++v) buf[pmod(-hk + 32 * (s0 + v) + lane, N)] = acc[v];
+                }
+                __syncwarp();
+                warp_fft<T, N, +1>(buf, tw);
+                for (int r = lane; r < N; r += 32) W[(size_t)c * WS + r] = buf[r];
+                __syncwarp();
+            }
+        } else {
+            for (int c = warp; c < H; c += NW) {
+                const int kx0 = c + ceil_div(-hk - c, N) * N;
+                for (int r = lane; r < N; r += 32) {
+                    const int kyc = r < N / 2 ? r : r - N;
+                    // the fold (wrap) of the aliases, with Kahan compensation
+                    Cx<T> acc = cx<T>(T(0), T(0)), comp = acc;
+                    for (int kx = kx0; kx <= hk; kx += N) {
+                        const bool pos = kx >= 0;
+                        for (int ky = kyc + ceil_div(-hk - kyc, N) * N; ky <= hk; ky += N) {
+                            const Cx<T> v = eval_point<T, II>(a.tpl, S, cache, pos ? kx : -kx, pos ? ky : -ky, hk, dk);
+                            kahan_add<T>(acc, comp, pos ? v : cconj<T>(v));
+                        }
+                    }
+                    buf[r] = acc;
+                }
+                __syncwarp();
+                warp_fft<T, N, +1>(buf, tw);
+                for (int r = lane; r < N; r += 32) W[(size_t)c * WS + r] = buf[r];
+                __syncwarp();
+            }
         }
         __syncthreads();
 
@@ -796,8 +1304,9 @@ int launch_fused(const DrawArgs& args, size_t work_bytes, cudaStream_t stream)
 {
     constexpr bool wsmem = w_fits_smem<T, N>();
     constexpr size_t sm = smem_bytes<T, N>(wsmem);
-    const int grid = draw_grid<T, N>(args.n_stamps);
-    if (!wsmem && (args.work == nullptr || work_bytes < workspace_bytes_for<T, N>(args.n_stamps)))
+    int grid = draw_grid<T, N>(args.n_stamps);
+    if (!wsmem && args.max_grid > 0) grid = std::min(grid, args.max_grid);
+    else if (!wsmem && (args.work == nullptr || work_bytes < workspace_bytes_for<T, N>(args.n_stamps)))
         return set_error(GSB_ERR_INVALID, "draw workspace too small");
     // programs without image leaves run the instance compiled without their code
     if (has_image_leaves(args.tpl)) {

@@ -78,32 +78,65 @@ __global__ void __launch_bounds__(THREADS) large_col_kernel(const __grid_constan
                a.sersic_stride, 1. / N);
     __syncthreads();
     const int Nk = S.geom.Nk, hk = Nk / 2;
-    const GridRef g{dk, 0, -hk, hk + 1, Nk + 1};
-    if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, Nk, 0u, la.cache_bytes);
+    if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, 0u, la.cache_bytes);
     __syncthreads();
-    fill_caches<T, II>(S, a.tpl, cache, dk, Nk);
+    fill_caches<T, II>(S, a.tpl, cache, dk, Nk, sizeof(T) == 4 && a.out_dtype == GSB_F64);
     __syncthreads();
-    const bool factored = S.xy_cache >= 0, fast = S.regstack;
     Cx<T>* W = reinterpret_cast<Cx<T>*>(la.W) + (size_t)s * H * N;
     for (int c = blockIdx.x; c < H; c += gridDim.x) {
-        const int alo = ceil_div(-hk - c, N), ahi = floor_div(hk - c, N);
-        for (int r = threadIdx.x; r < N; r += blockDim.x) {
-            const int kyc = r < N / 2 ? r : r - N;
-            const int blo = ceil_div(-hk - kyc, N), bhi = floor_div(hk - kyc, N);
-            Cx<T> acc = cx<T>(T(0), T(0)), comp = acc;     // Kahan-compensated fold
-            for (int ia = alo; ia <= ahi; ++ia) {
-                const int kx = c + ia * N;
-                for (int ib = blo; ib <= bhi; ++ib) {
-                    const int ky = kyc + ib * N;
+        const int kx0 = c + ceil_div(-hk - c, N) * N;
+        if (sizeof(T) == 4 && N % THREADS == 0) {
+            // the column's rows ky = -hk .. hk in order over the threads: a thread's slots s, s + NS, ...
+            // are the aliases of one wrapped row, V slots at a time (as in draw_fused_kernel)
+            constexpr int V = 4;
+            const int NS = N / THREADS;
+            for (int s0 = 0; s0 < NS; s0 += V) {
+                const int nv = min(V, NS - s0);
+                Cx<T> acc[V], comp[V];
+#pragma unroll
+                for (int v = 0; v < V; ++v) acc[v] = comp[v] = cx<T>(T(0), T(0));
+                for (int kx = kx0; kx <= hk; kx += N) {
                     const bool pos = kx >= 0;
-                    const int ii = pos ? kx : -kx, jj = pos ? ky : -ky;
-                    const Cx<T> v = factored ? eval_factored<T, II>(a.tpl, S, cache, dk, ii, jj, g)
-                                    : fast ? eval_fast<T, II>(a.tpl, S, cache, dk, ii, jj, g)
-                                           : eval_program<T, II>(a.tpl, S, dk, ii, jj, g);
-                    kahan_add<T>(acc, comp, pos ? v : cconj<T>(v));
+                    const int ii = pos ? kx : -kx;
+                    for (int e0 = -hk + THREADS * s0; e0 <= hk; e0 += N) {
+                        const int ky = e0 + int(threadIdx.x);
+                        if (nv == V && e0 + THREADS * V - 1 <= hk) {
+                            const Values<T, V> z = eval_any<T, II, V>(a.tpl, S, cache, ii, pos ? ky : -ky,
+                                                                      pos ? THREADS : -THREADS, hk, dk);
+#pragma unroll
+                            for (int v = 0; v < V; ++v) kahan_add<T>(acc[v], comp[v], pos ? z.v[v] : cconj<T>(z.v[v]));
+                        } else {
+#pragma unroll 1
+                            for (int u = 0; u < nv; ++u) {
+                                const int ku = ky + THREADS * u;
+                                if (ku > hk) break;
+                                const Cx<T> z = eval_point<T, II>(a.tpl, S, cache, ii, pos ? ku : -ku, hk, dk);
+#pragma unroll
+                                for (int v = 0; v < V; ++v)
+                                    if (v == u) kahan_add<T>(acc[v], comp[v], pos ? z : cconj<T>(z));
+                            }
+                        }
+                    }
                 }
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+                    if (v < nv) buf[pmod(-hk + THREADS * (s0 + v) + int(threadIdx.x), N)] = acc[v];
             }
-            buf[r] = acc;
+        } else {
+            // (double: one point at a time, compiled in place -- 1024 threads leave 64 registers, which
+            // a call's saved registers would spill: 9.2 ms in place, 13.7 as calls, two stamps of 8192)
+            for (int r = threadIdx.x; r < N; r += blockDim.x) {
+                const int kyc = r < N / 2 ? r : r - N;
+                Cx<T> acc = cx<T>(T(0), T(0)), comp = acc;     // Kahan-compensated fold
+                for (int kx = kx0; kx <= hk; kx += N) {
+                    const bool pos = kx >= 0;
+                    for (int ky = kyc + ceil_div(-hk - kyc, N) * N; ky <= hk; ky += N) {
+                        const Cx<T> v = eval_point<T, II, sizeof(T) == 8>(a.tpl, S, cache, pos ? kx : -kx, pos ? ky : -ky, hk, dk);
+                        kahan_add<T>(acc, comp, pos ? v : cconj<T>(v));
+                    }
+                }
+                buf[r] = acc;
+            }
         }
         __syncthreads();
         block_fft<T, +1>(buf, N, la.tw);

@@ -70,7 +70,7 @@ __device__ __forceinline__ void stockham_pass(Cx<T>* buf, const Cx<T>* tw, int l
 #pragma unroll
             for (int r = 0; r < R; ++r) v[t][r] = buf[b + r * NB];
 #pragma unroll
-            for (int r = 1; r < R; ++r) {
+            for (int r = 1; r < R && NS > 1; ++r) {      // (the first pass's twiddles are 1)
                 // r k TSTEP <= (R - 1)(NS - 1) N / (NS R) < N: no reduction mod N needed
                 const int idx = r * k * TSTEP;
                 Cx<T> w = tw[idx];

@@ -35,6 +35,12 @@
 
 namespace gsb {
 
+int fused_launch_f32_small(int N, const DrawArgs& args, size_t work_bytes, cudaStream_t stream, bool* handled);
+int fused_launch_f32_large(int N, const DrawArgs& args, size_t work_bytes, cudaStream_t stream, bool* handled);
+int fused_launch_f64_small(int N, const DrawArgs& args, size_t work_bytes, cudaStream_t stream, bool* handled);
+int fused_launch_f64_large(int N, const DrawArgs& args, size_t work_bytes, cudaStream_t stream, bool* handled);
+
+
 namespace {
 
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;
@@ -100,61 +106,31 @@ int noalloc_check_stamps(const gsb_stamp* d_stamps, int n_stamps, int N, int* d_
     return GSB_OK;
 }
 
-template <typename T, int N, bool II>
-int launch_noalloc_ii(const DrawArgs& args, int grid, cudaStream_t stream)
+int launch_noalloc(int N, DrawArgs args, int precision, cudaStream_t stream)
 {
-    constexpr bool wsmem = w_fits_smem<T, N>();
-    constexpr size_t sm = smem_bytes<T, N>(wsmem);
-    GSB_CUDA_CHECK(cudaFuncSetAttribute(draw_fused_kernel<T, N, wsmem, II>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-    draw_fused_kernel<T, N, wsmem, II><<<grid, fused_warps<T, N>() * 32, sm, stream>>>(args);
-    GSB_CUDA_CHECK(cudaGetLastError());
-    return GSB_OK;
-}
-
-template <typename T, int N>
-int launch_noalloc(DrawArgs args, cudaStream_t stream)
-{
-    constexpr bool wsmem = w_fits_smem<T, N>();
-    int grid = draw_grid<T, N>(args.n_stamps);
     void* p = nullptr;
     int* status = nullptr;
     int rc = noalloc_scratch(&p, &status);
     if (rc) return rc;
+    const size_t slab = (precision == GSB_F64 ? sizeof(double2) : sizeof(float2)) * (size_t)(N / 2 + 1) * (N + 1);
+    if (N > 1024 || !good_fft_size_ok(N) || N < 32)
+        return set_error(GSB_ERR_UNSUPPORTED, "gsb_draw_images_noalloc supports FFT sizes 2^a or 3*2^a "
+                                              "from 32 to 1024; got " + std::to_string(N));
     rc = noalloc_check_stamps(args.stamps, args.n_stamps, N, status, stream);
     if (rc) return rc;
-    if (!wsmem) {
-        constexpr size_t slab = sizeof(Cx<T>) * (size_t)(N / 2 + 1) * (N + 1);
-        static_assert(slab <= kNoAllocScratchBytes, "one slab must fit the no-alloc scratch");
-        const int fit = int(kNoAllocScratchBytes / slab);
-        if (grid > fit) grid = fit;
-        args.work = p;
+    // as many CTAs as have a slab in the static scratch
+    static_assert(sizeof(double2) * 513 * 1025 <= kNoAllocScratchBytes, "one slab must fit the no-alloc scratch");
+    args.work = p;
+    args.max_grid = int(kNoAllocScratchBytes / slab);
+    bool handled = false;
+    if (precision == GSB_F64) {
+        rc = fused_launch_f64_small(N, args, kNoAllocScratchBytes, stream, &handled);
+        if (!handled) rc = fused_launch_f64_large(N, args, kNoAllocScratchBytes, stream, &handled);
     } else {
-        args.work = nullptr;
+        rc = fused_launch_f32_small(N, args, kNoAllocScratchBytes, stream, &handled);
+        if (!handled) rc = fused_launch_f32_large(N, args, kNoAllocScratchBytes, stream, &handled);
     }
-    // programs without image leaves run the instance compiled without their code
-    return has_image_leaves(args.tpl) ? launch_noalloc_ii<T, N, true>(args, grid, stream)
-                                      : launch_noalloc_ii<T, N, false>(args, grid, stream);
-}
-
-template <typename T>
-int dispatch_noalloc(int N, const DrawArgs& args, cudaStream_t stream)
-{
-    switch (N) {
-      case 32: return launch_noalloc<T, 32>(args, stream);
-      case 48: return launch_noalloc<T, 48>(args, stream);
-      case 64: return launch_noalloc<T, 64>(args, stream);
-      case 96: return launch_noalloc<T, 96>(args, stream);
-      case 128: return launch_noalloc<T, 128>(args, stream);
-      case 192: return launch_noalloc<T, 192>(args, stream);
-      case 256: return launch_noalloc<T, 256>(args, stream);
-      case 384: return launch_noalloc<T, 384>(args, stream);
-      case 512: return launch_noalloc<T, 512>(args, stream);
-      case 768: return launch_noalloc<T, 768>(args, stream);
-      case 1024: return launch_noalloc<T, 1024>(args, stream);
-    }
-    return set_error(GSB_ERR_UNSUPPORTED, "gsb_draw_images_noalloc supports FFT sizes 2^a or 3*2^a "
-                                          "from 32 to 1024; got " + std::to_string(N));
+    return rc;
 }
 
 }  // namespace
@@ -181,6 +157,7 @@ extern "C" int gsb_draw_images_noalloc(const gsb_template* tpl, int n_stamps, co
     if (precision != GSB_F32 && precision != GSB_F64) return set_error(GSB_ERR_INVALID, "bad precision");
     DrawArgs args;
     args.tpl = *tpl;
+    plan_factors(args.tpl, args.fac);
     args.n_stamps = n_stamps;
     args.leaves = d_leaves;
     args.phases = d_phases;
@@ -194,6 +171,5 @@ extern "C" int gsb_draw_images_noalloc(const gsb_template* tpl, int n_stamps, co
     args.add = add_to_image;
     args.added_flux = d_added_flux;
     args.work = nullptr;
-    return precision == GSB_F64 ? dispatch_noalloc<double>(N, args, (cudaStream_t)stream)
-                                : dispatch_noalloc<float>(N, args, (cudaStream_t)stream);
+    return launch_noalloc(N, args, precision, (cudaStream_t)stream);
 }

@@ -1,0 +1,56 @@
+"""GPU: the draw kernels' evaluation of several wave vectors a lane (leaf kinds with constants in the
+working precision, the fold over a column's aliases, the last point of columns with Nk a multiple of
+32) against the FP64 path, which takes the general form, over FFT sizes, aliasing and profile types."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+pytest.importorskip('torch')
+
+import galsim_b200 as galsim  # noqa: E402
+
+
+def _profiles(gsp, B):
+    rng = np.random.default_rng(11)
+    g1, g2 = rng.uniform(-0.2, 0.2, B), rng.uniform(-0.2, 0.2, B)
+    ones = np.ones(B)
+    return {
+        'exponential': galsim.Exponential(scale_radius=1.2 * ones, gsparams=gsp).shear(g1=g1, g2=g2),
+        'sersic': galsim.Sersic(n=rng.uniform(0.6, 4., B), half_light_radius=1.5 * ones, gsparams=gsp).shear(g1=g1, g2=g2),
+        'moffat': galsim.Moffat(beta=rng.uniform(1.6, 6., B), fwhm=1.7 * ones, gsparams=gsp).shear(g1=g1, g2=g2),
+        'moffat_half': galsim.Moffat(beta=np.where(np.arange(B) % 2, 2.5, 3.5), fwhm=1.7 * ones, gsparams=gsp),
+        'kolmogorov': galsim.Kolmogorov(fwhm=1.7 * ones, gsparams=gsp).shear(g1=g1, g2=g2),
+        'airy': galsim.Airy(lam_over_diam=1.1 * ones, obscuration=0.3, gsparams=gsp).shear(g1=g1, g2=g2),
+        'gaussian': galsim.Gaussian(sigma=0.8 * ones, gsparams=gsp).shear(g1=g1, g2=g2),
+    }
+
+
+@pytest.mark.parametrize('min_n,scale', [(32, 1.), (48, 1.), (64, 0.6), (96, 1.7), (128, 1.3), (192, 1.), (256, 2.2),
+                                         (384, 1.), (1024, 1.)])
+@pytest.mark.parametrize('kind', ['exponential', 'sersic', 'moffat', 'moffat_half', 'kolmogorov', 'airy', 'gaussian',
+                                  'sum'])
+def test_float_draws_against_double(kind, min_n, scale):
+    B = 3
+    gsp = galsim.GSParams(minimum_fft_size=min_n, folding_threshold=0.05, stepk_minimum_hlr=1.)
+    p = _profiles(gsp, B)
+    obj = p[kind] if kind != 'sum' else galsim.Add(p['sersic'] * 0.4, p['exponential'] * 0.6)
+    obj = galsim.Convolve(obj, galsim.Gaussian(sigma=0.4, gsparams=gsp)).shift(0.3, -0.2)
+    lo, hi = [galsim.draw_batch(obj, nx=25, ny=18, scale=scale, dtype=np.float64 if q == 'fp64' else np.float32, precision=q)
+              for q in ('fp32', 'fp64')]
+    assert np.array_equal(lo.N, hi.N) and np.array_equal(lo.Nk, hi.Nk)
+    a, b = lo.flat.cpu().numpy().reshape(B, 18, 25).astype(float), hi.flat.cpu().numpy().reshape(B, 18, 25)
+    # single precision: a few 1e-7 of the value a wave vector, summed over the image with random signs
+    for x, y in zip(a, b):
+        assert np.abs(x - y).max() <= 3e-6 * np.abs(y).max()
+
+
+def test_double_image_keeps_the_general_path():
+    """drawImage into a double image at the default precision: one object and a batch agree bit for bit."""
+    obj = galsim.Convolve(galsim.Exponential(flux=3., half_light_radius=0.8).shear(g1=0.1, g2=-0.05),
+                          galsim.Moffat(beta=3., fwhm=0.7), galsim.Pixel(0.2))
+    im = obj.drawImage(galsim.ImageD(48, 40), scale=0.2, method='fft')
+    many = galsim.Convolve(galsim.Exponential(flux=np.full(3, 3.), half_light_radius=0.8).shear(g1=0.1, g2=-0.05),
+                           galsim.Moffat(beta=3., fwhm=0.7), galsim.Pixel(0.2))
+    sb = galsim.draw_batch(many, nx=48, ny=40, scale=0.2, dtype=np.float64, precision='fp32')
+    for a in sb.flat.cpu().numpy().reshape(3, 40, 48):
+        assert np.array_equal(a, im.array)
