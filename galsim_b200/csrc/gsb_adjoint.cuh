@@ -169,11 +169,114 @@ __device__ __noinline__ void adjoint_range(const gsb_template& tpl, const AdjSme
     }
 }
 
+// The n-derivative nodes (value, second derivative) of the wanted Sersic leaves, in shared memory
+// (whole block, with fill_caches).
+__device__ inline void fill_dn_cache(const AdjSmem& A, const gsb_template& tpl, unsigned char* cache, bool have_dn)
+{
+    const StampSmem& S = A.S;
+    for (int l = 0; l < tpl.n_leaves; ++l) {
+        if (S.leaf[l].type != GSB_SERSIC || S.aux_cache[l] < 0 || !have_dn) continue;
+        float2* dst = reinterpret_cast<float2*>(cache + S.aux_cache[l]);
+        const double4* src = A.dn[l].node;
+        for (int t = threadIdx.x; t < S.sersic[l].n; t += blockDim.x) dst[t] = make_float2(float(src[t].y), float(src[t].z));
+    }
+}
+
+// leaf_grad with the shared-memory constants and nodes, for the kinds that have them (float): the
+// same forms as leaf_points' values.
+template <typename T>
+__device__ __forceinline__ LeafD<T> leaf_grad_fast(const AdjSmem& A, const unsigned char* cache, int l, int i, int j,
+                                                   int hk, const GridRef& g, T kx, T ky)
+{
+    const StampSmem& S = A.S;
+    if constexpr (sizeof(T) == 4) {
+        const LeafT<float>& L = leaf_const<float>(S, l);
+        if (L.kind == kLeafSersic && S.aux_cache[l] >= 0) {
+            const float u = L.a * float(i) + L.c * float(j), w = L.b * float(i) + L.d * float(j);
+            const float k2 = u * u + w * w, flux = L.flux;
+            const float inv = fast_rcp(k2);
+            const float h = L.q[6], inv_h = L.q[7];
+            float phi, dphi, dphin;
+            if (k2 >= L.q[0] && k2 < L.q[1]) {
+                const float4* node = reinterpret_cast<const float4*>(cache + L.cache);
+                const float2* dnode = reinterpret_cast<const float2*>(cache + S.aux_cache[l]);
+                const int q = max(1, min(__float_as_int(fmaf(fast_log2(k2), L.q[8], L.q[9]) + 12582912.f) - 0x4b400000, L.n - 1));
+                const float4 n0 = node[q - 1], n1 = node[q];
+                const float2 d0 = dnode[q - 1], d1 = dnode[q];
+                const float e = (n1.w - k2) * inv;
+                float aa;
+                if (h < 0.04f) {
+                    float p = fmaf(e, -1.f / 16.f, 1.f / 14.f);      // ln(1 + e) / 2, as sersic_points
+                    p = fmaf(e, p, -1.f / 12.f);
+                    p = fmaf(e, p, 0.1f);
+                    p = fmaf(e, p, -0.125f);
+                    p = fmaf(e, p, 1.f / 6.f);
+                    p = fmaf(e, p, -0.25f);
+                    p = fmaf(e, p, 0.5f);
+                    aa = e * p;
+                } else {
+                    aa = 0.5f * logf(n1.w * inv);
+                }
+                const float bb = h - aa, P = aa * bb;
+                const float Q = fmaf(aa + h, n0.z, (bb + h) * n1.z);
+                const float f = fmaf(P * Q, -1.f / 6.f, fmaf(aa, n0.y, bb * n1.y)) * inv_h;
+                const float fl = fmaf(fmaf(aa - bb, Q, P * (n1.z - n0.z)), -1.f / 6.f, n1.y - n0.y) * inv_h;
+                const float Qn = fmaf(aa + h, d0.y, (bb + h) * d1.y);
+                const float fn = fmaf(P * Qn, -1.f / 6.f, fmaf(aa, d0.x, bb * d1.x)) * inv_h;
+                phi = f * inv;
+                dphi = (0.5f * fl - f) * inv * inv;
+                dphin = (fn - float(A.dn[l].dfront) * fl) * inv;     // the argument moves with the grid origin
+            } else {
+                sersic_phi_grad<float>(S.sersic[l], A.dn[l], k2, phi, dphi, dphin);
+            }
+            LeafD<float> r;
+            r.unit = phi;
+            r.v = flux * phi;
+            r.gn = flux * dphin;
+            const float d2 = 2.f * flux * dphi * L.size;              // dv/dk' = 2 k' dv/d|k'|^2
+            r.gx = d2 * u;
+            r.gy = d2 * w;
+            return r;
+        }
+    }
+    if (leaf_const<T>(S, l).kind == kLeafExp) {
+        const LeafT<T>& L = leaf_const<T>(S, l);
+        const ushort2 c = reinterpret_cast<const ushort2*>(cache + L.cache)[hk + j];
+        LeafD<T> r{T(0), T(0), T(0), T(0), T(0)};
+        if (i < int(c.x) || i >= int(c.y)) return r;
+        const T u = L.a * kx + L.c * ky, w = L.b * kx + L.d * ky, r0 = L.q[0];
+        const T p = T(1) + (u * u + w * w) * r0 * r0;
+        const T phi = T(1) / (p * sqrt(p));
+        r.unit = phi;
+        r.v = L.flux * phi;
+        const T d2 = T(-3) * r.v / p * r0 * r0;
+        r.gx = d2 * u;
+        r.gy = d2 * w;
+        return r;
+    }
+    return leaf_grad<T>(S.leaf[l], S.sersic, A.dn, kx, ky, g, i - g.x0, j - g.y0);
+}
+
+// The unit phasor of phase p at (i, j): the product of its cached axis factors, or directly.
+template <typename T>
+__device__ __forceinline__ Cx<T> phase_unit(const StampSmem& S, const unsigned char* cache, int p, int i, int j, int hk)
+{
+    if (S.phase_cache[p] >= 0) {
+        const Cx<T>* PX = reinterpret_cast<const Cx<T>*>(cache + S.phase_cache[p]);
+        return cmul<T>(PX[i], PX[hk + 1 + j + hk]);
+    }
+    double tt = i * S.phase_ax[p] + j * S.phase_ay[p];
+    tt -= rint(tt);
+    T sn, cs;
+    sincospi(T(-2. * tt), &sn, &cs);
+    return cx<T>(cs, sn);
+}
+
 // Gradients of the leaves of a Sum atom (LEAF and ADD ops [o0, o1)) with cotangent w: each
 // leaf receives w unchanged.
 template <typename T>
-__device__ __noinline__ void sum_atom_grads(const gsb_template& tpl, const AdjSmem& A, unsigned want,
-                                            T kx, T ky, int i, int j, const GridRef& g, Cx<T> w, T* acc,
+__device__ __noinline__ void sum_atom_grads(const gsb_template& tpl, const AdjSmem& A, const unsigned char* cache,
+                                            unsigned want, T kx, T ky, int i, int j, const GridRef& g, Cx<T> w, T* acc,
                                             int o0, int o1)
 {
     const T ar = w.x;
@@ -181,7 +284,7 @@ __device__ __noinline__ void sum_atom_grads(const gsb_template& tpl, const AdjSm
         if (tpl.op_code[o] != GSB_OP_LEAF) continue;
         const int l = tpl.op_arg[o];
         if (!want_leaf(want, l)) continue;
-        const LeafD<T> d = leaf_grad<T>(A.S.leaf[l], A.S.sersic, A.dn, kx, ky, g, i - g.x0, j - g.y0);
+        const LeafD<T> d = leaf_grad_fast<T>(A, cache, l, i, j, g.n / 2, g, kx, ky);
         T* gl = acc + kGradPerLeaf * l;
         gl[0] += ar * d.unit;
         gl[1] += ar * d.gx * kx;
@@ -218,19 +321,16 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
             const int o0 = S.atom_o0[a], o1 = S.atom_o1[a];
             if (kind == kAtomPhase) {
                 const int p = S.atom_arg[a];
-                double tt = i * S.phase_ax[p] + j * S.phase_ay[p];
-                tt -= rint(tt);
-                T sn, cs;
-                sincospi(T(-2. * tt), &sn, &cs);
-                ld[a].gx = cs;
-                ld[a].gy = sn;
-                val[a] = cscale<T>(cx<T>(cs, sn), T(S.phase[p].flux_scaling));
+                const Cx<T> e = phase_unit<T>(S, cache, p, i, j, hk);
+                ld[a].gx = e.x;
+                ld[a].gy = e.y;
+                val[a] = cscale<T>(e, T(S.phase[p].flux_scaling));
             } else if (kind == kAtomScale) {
                 val[a] = cx<T>(T(S.scale[S.atom_arg[a]]), T(0));
             } else if (o1 - o0 == 1) {
                 const int l = tpl.op_arg[o0];
                 if (want_leaf(want, l) && !(II && S.leaf[l].type == GSB_INTERPOLATED)) {
-                    ld[a] = leaf_grad<T>(S.leaf[l], S.sersic, A.dn, kx, ky, g, i - g.x0, j - g.y0);
+                    ld[a] = leaf_grad_fast<T>(A, cache, l, i, j, hk, g, kx, ky);
                     val[a] = cx<T>(ld[a].v, T(0));
                 } else {
                     val[a] = leaf_cfast<T, II>(S, cache, l, i, j, g);
@@ -274,7 +374,7 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
                 ga[a][4] += ar * ld[a].gy * ky;
                 ga[a][5] += ar * ld[a].gn;
             } else if (kind == kAtomSum) {
-                sum_atom_grads<T>(tpl, A, want, kx, ky, i, j, g, w, acc, o0, o1);
+                sum_atom_grads<T>(tpl, A, cache, want, kx, ky, i, j, g, w, acc, o0, o1);
             } else {
                 adjoint_range<T, II>(tpl, A, dk, i, j, g, w, acc, o0, o1);
             }
@@ -291,15 +391,17 @@ __device__ inline T load_cot(const void* p, int dtype, long long idx)
 }
 
 // Warps per CTA: 16, or 8 where 16 FFT buffers of N complex T do not fit (double, N >= 768).
+// In float at N <= 128, 8 warps of up to 128 registers, two CTAs an SM, as the forward.
 template <typename T, int N>
 __host__ __device__ constexpr int adj_warps()
 {
+    if (sizeof(T) == 4 && N <= 128) return kWarps / 2;
     return ((sizeof(AdjSmem) + 15) / 16 * 16 + sizeof(Cx<T>) * N * (1 + kWarps) + kCacheBytes + 4096 <=
             kSmemLimit) ? kWarps : kWarps / 2;
 }
 
 template <typename T, int N, bool WSMEM, bool II>
-__global__ void __launch_bounds__(adj_warps<T, N>() * 32) adjoint_fused_kernel(const __grid_constant__ AdjArgs a)
+__global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <= 128 ? 2 : 1) adjoint_fused_kernel(const __grid_constant__ AdjArgs a)
 {
     constexpr int NW = adj_warps<T, N>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -350,6 +452,7 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32) adjoint_fused_kernel(c
         if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, a.want);
         __syncthreads();
         fill_caches<T, II>(S, a.tpl, cache, dk, Nk);
+        fill_dn_cache(A, a.tpl, cache, a.sersic_dheader != nullptr);
         __syncthreads();
         const bool factored = S.xy_cache >= 0 && S.n_atoms <= kAdjAtoms;
         bool subtree = !factored;
@@ -400,24 +503,19 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32) adjoint_fused_kernel(c
             __syncwarp();
             warp_fft<T, N, +1>(buf, tw);
             const T wc = (c == 0 || 2 * c == N) ? inv_n2 : T(2) * inv_n2;
-            const int alo = ceil_div(-hk - c, N), ahi = floor_div(hk - c, N);
-            for (int r = lane; r < N; r += 32) {
-                const Cx<T> gh = cscale<T>(buf[r], wc);
-                const int kyc = r < N / 2 ? r : r - N;
-                const int blo = ceil_div(-hk - kyc, N), bhi = floor_div(hk - kyc, N);
-                for (int ia = alo; ia <= ahi; ++ia) {
-                    const int kx = c + ia * N;
-                    for (int ib = blo; ib <= bhi; ++ib) {
-                        const int ky = kyc + ib * N;
-                        const bool pos = kx >= 0;
-                        // an alias taken as conj(F(-k)) contributes Re(Ghat conj(dF)) = Re(conj(Ghat) dF)
-                        if (factored)
-                            adjoint_point_factored<T, II>(a.tpl, A, cache, a.want, dk, pos ? kx : -kx,
-                                                      pos ? ky : -ky, g, pos ? gh : cconj<T>(gh), ga, acc);
-                        else
-                            adjoint_range<T, II>(a.tpl, A, dk, pos ? kx : -kx, pos ? ky : -ky, g,
-                                             pos ? gh : cconj<T>(gh), acc, 0, a.tpl.n_ops);
-                    }
+            const int kx0 = c + ceil_div(-hk - c, N) * N;
+            // the column's rows ky = -hk .. hk in order, every alias once, as the forward takes them
+            for (int ky = -hk + lane; ky <= hk; ky += 32) {
+                const Cx<T> gh = cscale<T>(buf[pmod(ky, N)], wc);
+                for (int kx = kx0; kx <= hk; kx += N) {
+                    const bool pos = kx >= 0;
+                    // an alias taken as conj(F(-k)) contributes Re(Ghat conj(dF)) = Re(conj(Ghat) dF)
+                    if (factored)
+                        adjoint_point_factored<T, II>(a.tpl, A, cache, a.want, dk, pos ? kx : -kx,
+                                                  pos ? ky : -ky, g, pos ? gh : cconj<T>(gh), ga, acc);
+                    else
+                        adjoint_range<T, II>(a.tpl, A, dk, pos ? kx : -kx, pos ? ky : -ky, g,
+                                         pos ? gh : cconj<T>(gh), acc, 0, a.tpl.n_ops);
                 }
             }
             __syncwarp();

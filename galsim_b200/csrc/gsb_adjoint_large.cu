@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_col_kernel(const __grid_con
     if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, a.want, la.cache_bytes);
     __syncthreads();
     fill_caches<T, II>(S, a.tpl, cache, dk, Nk);
+    fill_dn_cache(A, a.tpl, cache, a.sersic_dheader != nullptr);
     __syncthreads();
     const bool factored = S.xy_cache >= 0 && S.n_atoms <= kAdjAtoms;
     bool subtree = !factored;

@@ -42,6 +42,7 @@ struct __align__(16) LeafT {
     T a, b, c, d;
     T flux;
     int kind, cache, n;
+    T size;             // the leaf's size (in the units of its Jacobian's source), for derivatives
     T q[10];
 };
 
@@ -61,7 +62,8 @@ struct StampSmem {
     int phase_cache[GSB_MAX_PHASES];
     int sersic_cache[GSB_MAX_LEAVES];
     int ii_cache[GSB_MAX_LEAVES];      // InterpolatedImage taps per column / row (IITaps)
-    int aux_cache[GSB_MAX_LEAVES];     // Exponential: kept columns per row; Moffat: quadrature nodes
+    // Exponential: kept columns per row; Moffat: quadrature nodes; Sersic: n-derivative nodes (adjoint)
+    int aux_cache[GSB_MAX_LEAVES];
     int regstack;      // the program fits the 4-deep register stack
     // Factored form of the program (see plan_factored): the root is a product of atoms; the
     // separable atoms (diagonal Box / Gaussian leaves, phases, scales) are folded into
@@ -389,6 +391,8 @@ __device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, const 
         int bytes = 0;
         if (L.type == GSB_EXPONENTIAL) bytes = ((Nk + 1) * (int)sizeof(ushort2) + 15) & ~15;
         else if (L.type == GSB_MOFFAT && sizeof(T) == 4 && int(L.d[2]) == 0) bytes = kMoffatNodes * (int)sizeof(float2);
+        else if (L.type == GSB_SERSIC && sizeof(T) == 4 && want_leaf(want, l) && S.sersic_cache[l] >= 0)
+            bytes = (S.sersic[l].n * (int)sizeof(float2) + 15) & ~15;
         else continue;
         if (hk < 65535 && used + bytes <= budget) { S.aux_cache[l] = used; used += bytes; }
     }
@@ -415,6 +419,7 @@ __device__ __noinline__ void set_leaf_const(StampSmem& S, int l, double dk, bool
     t.cache = -1;
     t.n = 0;
     t.flux = T(L.flux);
+    t.size = T(L.d[0]);
     double size = 1.;
     if (S.leaf_cache[l] >= 0) {
         t.kind = kLeafSep;
@@ -532,7 +537,9 @@ __device__ inline void fill_caches(StampSmem& S, const gsb_template& tpl, unsign
     for (int l = 0; l < tpl.n_leaves; ++l) {
         if (S.aux_cache[l] < 0) continue;
         const LeafParams& L = S.leaf[l];
-        if (L.type == GSB_EXPONENTIAL) {
+        if (L.type == GSB_SERSIC) {
+            // (filled by the adjoint, which knows the derivative tables)
+        } else if (L.type == GSB_EXPONENTIAL) {
             ushort2* R = reinterpret_cast<ushort2*>(cache + S.aux_cache[l]);
             for (int t = threadIdx.x; t < Nk + 1; t += blockDim.x) R[t] = exponential_columns(L, dk, hk, t - hk);
         } else {
