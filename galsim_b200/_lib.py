@@ -110,6 +110,7 @@ def lib():
             'gsb_add_noise': (i, [i, vp, vp, i, i, vp, i, vp, vp, vp]),
             'gsb_fits_pack': (i, [vp, i, vp, ctypes.c_longlong, vp, ctypes.c_longlong, i, vp,
                                   ctypes.c_longlong, vp]),
+            'gsb_expand_leaves': (i, [vp, i, i, vp, ctypes.c_int64, vp, vp, vp, vp]),
             'gsb_permute_records': (i, [vp, vp, vp, ctypes.c_int64, ctypes.c_int64, i, vp]),
             'gsb_adjoint_grad_count': (i, [ctypes.POINTER(TemplateC)]),
             'gsb_adjoint_workspace_size': (sz, [i, i, i]),
@@ -170,8 +171,13 @@ class Device(object):
     _index = 0
     _ready = set()
 
+    _torch = {}
+
     @classmethod
     def torch_device(cls):
+        dev = cls._torch.get(cls._index)
+        if dev is not None:
+            return dev
         import torch
         if not torch.cuda.is_available():
             raise GalSimError("galsim_b200 draws on a CUDA device (B200) and none is available; "
@@ -182,6 +188,7 @@ class Device(object):
             torch.cuda.init()
             check(lib().gsb_init(cls._index))
             cls._ready.add(cls._index)
+        cls._torch[cls._index] = dev
         return dev
 
     @classmethod

@@ -185,7 +185,7 @@ class RecordPlan(object):
         size = rec['leaf_size']
         gsize = torch.zeros_like(size)
         for l, t in enumerate(self.types):
-            if t == _lib.INTERPOLATED:
+            if t == _lib.INTERPOLATED or not (self.want >> l) & 1:      # (no entries, or zeros)
                 continue
             if t == _lib.BOX:
                 gsize[:, l, 0] = (jac[:, l, 0] * gjac[:, l, 0] + jac[:, l, 2] * gjac[:, l, 2]) / size[:, l, 0]
@@ -317,7 +317,7 @@ class GalaxyModel(object):
         phase_cen = rec['phase_cen'].clone()
         phase_cen[:, 0] = torch.stack([dx, dy], -1)     # the program keeps its shift op (see build)
         phase_fs = rec['phase_fs'].clone()
-        phase_fs[:, 0] = torch.abs(torch.linalg.det(S))
+        phase_fs[:, 0] = torch.abs(S[:, 0, 0] * S[:, 1, 1] - S[:, 0, 1] * S[:, 1, 0])
         return draw_records(plan, leaf_flux, leaf_jac, leaf_size, leaf_n, phase_cen, phase_fs,
                             rec['phase_jac'], rec['scales'])
 

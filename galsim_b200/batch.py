@@ -76,7 +76,18 @@ class StampBatch(object):
         self.Nk = Nk
         self.dtype = dtype
         self.scale = scale
-        self.bounds = bounds
+        self._bounds = bounds
+
+    @property
+    def bounds(self):
+        """(xmin, xmax, ymin, ymax) of every stamp's image, a list of tuples."""
+        if self._bounds is None and self.nx is not None:
+            self._bounds = [(1, x, 1, y) for x, y in zip(np.asarray(self.nx).tolist(), np.asarray(self.ny).tolist())]
+        return self._bounds
+
+    @bounds.setter
+    def bounds(self, value):
+        self._bounds = value
 
     @property
     def added_flux(self):
@@ -352,9 +363,8 @@ def run_batch(plan, recompute=True, graph=True):
     dt = _lib.F32 if np.dtype(plan.dtype) == np.float32 else _lib.F64
     prec = _lib.F64 if plan.precision == 'fp64' else _lib.F32
     flat, offsets, flux = prog.draw_stamps(N, Nk, xmin, ymin, nxs, nys, dt, precision=prec, graph=graph)
-    bounds = [(1, int(x), 1, int(y)) for x, y in zip(nxs, nys)]
     return StampBatch(flat, offsets, nxs, nys, xmin, ymin, N, Nk, flux, plan.dtype, plan.scale,
-                      bounds, plan.flux_scale)
+                      None, plan.flux_scale)
 
 
 def _run_real(plan):
@@ -375,10 +385,9 @@ def _run_real(plan):
     xmin = -(nxs // 2)
     ymin = -(nys // 2)
     flat, offsets, flux = draw_real_stamps(plan.prof, B, prog.gsparams, xmin, ymin, nxs, nys, plan.dtype)
-    bounds = [(1, int(x), 1, int(y)) for x, y in zip(nxs, nys)]
     zero = np.zeros(B, np.int64)
     return StampBatch(flat, offsets, nxs, nys, xmin, ymin, zero, zero, flux, plan.dtype, plan.scale,
-                      bounds, plan.flux_scale)
+                      None, plan.flux_scale)
 
 
 def draw_batch(obj, nx=None, ny=None, scale=None, dtype=np.float32, method='fft', area=1.,

@@ -93,10 +93,10 @@ class _ImageLeaf(GSObject):
                 "GPU (x: Delta, Nearest, Linear, Cubic, Quintic, Lanczos, Sinc; k: Nearest, Linear, "
                 "Cubic, Quintic, Lanczos(n <= 3))" % (xi, ki))
         bld.add_leaf(_lib.INTERPOLATED, jac, 1., (float(xi._code), float(ki._code), 0.))
-        bld.image_sources[len(bld.leaves) - 1] = self._sources
+        bld.image_sources[bld.n_leaves - 1] = self._sources
         # a Lanczos k interpolant's coefficient block goes into p[2] when the records are
         # uploaded (Program.upload), where the device exists
-        bld.image_kinterp[len(bld.leaves) - 1] = ki if isinstance(ki, Lanczos) else None
+        bld.image_kinterp[bld.n_leaves - 1] = ki if isinstance(ki, Lanczos) else None
 
     def withGSParams(self, gsparams=None, **kwargs):
         return self

@@ -44,7 +44,9 @@ class Builder(object):
         self.gsparams = gsparams
         self.ops = []
         self.leaf_types = []
-        self.leaves = []
+        self.columns = []         # per leaf: its nine parameter columns (add_leaf)
+        self.leaf_flags = []
+        self._leaves = None       # the same as records, once asked for
         self.phases = []
         self.scales = []
         self.image_sources = {}   # InterpolatedImage leaf -> its _ImageSource list (1 or B)
@@ -61,36 +63,55 @@ class Builder(object):
         return np.broadcast_to(j, (self.B, 2, 2))
 
     def add_leaf(self, ltype, jac, flux, params, flags=0):
-        if len(self.leaves) >= _lib.MAX_LEAVES:
+        """A leaf of the tree, kept as its nine parameter columns (jac 0-3, flux, p 0-2, table slot):
+        a float where all stamps share the value, else one float64 per stamp (see `leaves`)."""
+        if self.n_leaves >= _lib.MAX_LEAVES:
             raise GalSimError("profile tree has more than %d leaves" % _lib.MAX_LEAVES)
-        # the record as 17 float64 words (jac 0-3, flux 4, p 5-7, d 8-15, flags / table in 16),
-        # filled column by column with broadcasting, then viewed as LEAF_DTYPE
-        B = self.B
-        w = np.empty((B, 17), dtype=np.float64)
-        iw = w.view(np.int32)                      # (B, 34): flags at 32, table at 33
         if jac is None:
-            w[:, 0:4] = (1., 0., 0., 1.)
-            general = 0
+            cols = [1., 0., 0., 1.]
         else:
             j = np.asarray(jac, dtype=np.float64)
             if j.ndim == 2:
-                w[:, 0:4] = j.reshape(4)
-                general = _lib.LEAF_JAC_GENERAL if (j[0, 1] != 0. or j[1, 0] != 0.) else 0
+                cols = [float(v) for v in j.reshape(4)]
             else:
-                j = j.reshape(B, 4)
-                w[:, 0:4] = j
-                general = np.where((j[:, 1] != 0.) | (j[:, 2] != 0.), _lib.LEAF_JAC_GENERAL, 0)
-        w[:, 4] = flux
-        w[:, 5:8] = 0.
-        for i, p in enumerate(params):
-            w[:, 5 + i] = np.asarray(p, dtype=np.float64).reshape(-1) if np.ndim(p) else p
-        w[:, 8:16] = 0.
-        iw[:, 32] = np.bitwise_or(general, flags)
-        iw[:, 33] = 0
-        rec = w.view(_lib.LEAF_DTYPE).reshape(B)
-        self.ops.append((_lib.OP_LEAF, len(self.leaves)))
+                cols = list(np.ascontiguousarray(j.reshape(self.B, 4).T)) if self.B > 1 else \
+                    [float(v) for v in j.reshape(4)]
+        cols.append(self._column(flux))
+        cols += [self._column(p) for p in params] + [0.] * (3 - len(params)) + [0.]
+        self.ops.append((_lib.OP_LEAF, self.n_leaves))
         self.leaf_types.append(ltype)
-        self.leaves.append(rec)
+        self.columns.append(cols)
+        self.leaf_flags.append(int(flags))
+
+    def _column(self, v):
+        if np.ndim(v) == 0:
+            return float(v)
+        a = np.array(v, dtype=np.float64).reshape(-1)
+        if a.size == 1:
+            return float(a[0])
+        if a.size != self.B:
+            raise ValueError("could not broadcast a parameter of %d values to %d stamps" % (a.size, self.B))
+        return a
+
+    n_leaves = property(lambda self: len(self.columns))
+
+    @property
+    def leaves(self):
+        """The leaves as structured records (LEAF_DTYPE, one array of B per leaf), made from the
+        columns when first asked for; from then on they are what is uploaded, so that a caller
+        may change them in place."""
+        if self._leaves is None:
+            recs = []
+            for cols, flags in zip(self.columns, self.leaf_flags):
+                # the record as 17 float64 words (jac 0-3, flux 4, p 5-7, d 8-15, flags / table in 16)
+                w = np.zeros((self.B, 17), dtype=np.float64)
+                for i, c in enumerate(cols[:8]):
+                    w[:, i] = c
+                iw = w.view(np.int32)                      # (B, 34): flags at 32, table at 33
+                iw[:, 32] = np.where((w[:, 1] != 0.) | (w[:, 2] != 0.), _lib.LEAF_JAC_GENERAL, 0) | flags
+                recs.append(w.view(_lib.LEAF_DTYPE).reshape(self.B))
+            self._leaves = recs
+        return self._leaves
 
     def add_op(self, code):
         self.ops.append((code, 0))
@@ -118,7 +139,7 @@ class Builder(object):
             raise GalSimError("profile tree needs more than %d program ops" % _lib.MAX_OPS)
         t = _lib.TemplateC()
         t.n_ops = len(self.ops)
-        t.n_leaves = len(self.leaves)
+        t.n_leaves = self.n_leaves
         t.n_phases = len(self.phases)
         t.n_scales = len(self.scales)
         for i, (c, a) in enumerate(self.ops):
@@ -145,17 +166,113 @@ class Program(object):
         obj._flatten(bld, None)
         self.bld = bld
         self.tpl = bld.template()
-        self.L = len(bld.leaves)
+        self.L = bld.n_leaves
         self.gsp_c = _lib.gsparams_c(self.gsparams)
         self._prepared = False
         self.need_dn = False      # build the Sersic d/dn tables (for the adjoint)
 
     # -- device preparation ------------------------------------------------------------------
     def upload(self):
-        """Pack the leaf records, assign Sersic table slots and copy the leaves to the device."""
+        """Assign the table slots and put the leaf records on the device: from the parameter
+        columns, or from the host records where a caller has taken them (Builder.leaves) or a
+        truncated Moffat needs its table slots per stamp."""
         if getattr(self, 'd_leaves', None) is not None:
             return
         import torch
+        bld = self.bld
+        if bld._leaves is None and not any(t == _lib.MOFFAT and np.any(np.asarray(c[7]) > 0.)
+                                           for t, c in zip(bld.leaf_types, bld.columns)):
+            self._upload_columns()
+        else:
+            self._upload_records()
+        self.d_info = torch.empty(self.B * self.L * 2, dtype=torch.float64, device=_lib.Device.torch_device())
+        if self.sersic_n is None and not self.image_order and self.moffat_beta is None:
+            self.tables = None
+        elif getattr(self, 'tables', None) is None:
+            self.tables = _lib.TablePool.acquire()
+            self._pooled_tables = True
+
+    def _upload_columns(self):
+        import torch
+        B, bld = self.B, self.bld
+        cols = [list(c) for c in bld.columns]
+        sersic = [l for l, t in enumerate(bld.leaf_types) if t == _lib.SERSIC]
+        self.sersic_n = self.sersic_trunc = self.moffat_beta = self.moffat_trunc = None
+        if sersic:
+            # one table per distinct (n, trunc / r0); truncated leaves carry r0 in p[1]
+            nvals, tvals, sizes = [], [], []
+            for l in sersic:
+                n, r0, tr = cols[l][5:8]
+                t = np.where(np.asarray(tr) > 0., np.asarray(tr) / np.asarray(r0), 0.)
+                n, t = np.broadcast_arrays(np.atleast_1d(n), np.atleast_1d(t))
+                nvals.append(n)
+                tvals.append(t)
+                sizes.append(len(n))
+            nvals, tvals = np.concatenate(nvals), np.concatenate(tvals)
+            if np.any(tvals > 0.):
+                un, ut, inv = unique_pairs(nvals, tvals)
+                self.sersic_trunc = np.ascontiguousarray(ut)
+            else:
+                un, inv = np.unique(nvals, return_inverse=True)
+            self.sersic_n = np.ascontiguousarray(un)
+            for l, slot in zip(sersic, np.split(np.asarray(inv).reshape(-1), np.cumsum(sizes)[:-1])):
+                cols[l][8] = float(slot[0]) if len(slot) == 1 else slot.astype(np.float64)
+        for l, slots in self._image_slots():
+            cols[l][8] = float(slots[0]) if len(slots) == 1 else slots.astype(np.float64)
+            addr = self._kinterp_address(l)
+            if addr is not None:
+                cols[l][7] = addr
+        offset = np.full((self.L, 9), -1, dtype=np.int64)
+        value = np.zeros((self.L, 9))
+        arrays = []
+        for l, leaf in enumerate(cols):
+            for f, c in enumerate(leaf):
+                if isinstance(c, np.ndarray):
+                    offset[l, f] = len(arrays) * B
+                    arrays.append(c)
+                else:
+                    value[l, f] = c
+        flags = np.array(bld.leaf_flags, dtype=np.int32)
+        dev = _lib.Device.torch_device()
+        d_cols = None
+        if arrays:
+            # page-locked staging from torch's pool, which reuses a block only after its copy is done
+            host = torch.empty(len(arrays) * B, dtype=torch.float64, pin_memory=True)
+            h = host.numpy()
+            for i, c in enumerate(arrays):
+                h[i * B:(i + 1) * B] = c
+            d_cols = host.to(dev, non_blocking=True)
+        self.d_leaves = torch.empty(B * self.L * _lib.LEAF_DTYPE.itemsize, dtype=torch.uint8, device=dev)
+        _lib.check(_lib.lib().gsb_expand_leaves(
+            _lib.ptr(self.d_leaves), B, self.L, _lib.ptr(d_cols), len(arrays) * B,
+            offset.ctypes.data_as(ctypes.c_void_p), value.ctypes.data_as(ctypes.c_void_p),
+            flags.ctypes.data_as(ctypes.c_void_p), _lib.Device.stream()))
+
+    def _image_slots(self):
+        """(leaf, its slot per source) of every InterpolatedImage leaf; sets image_order."""
+        self.image_order = []
+        slot_of = {}
+        out = []
+        for l in range(self.L):
+            if self.bld.leaf_types[l] != _lib.INTERPOLATED:
+                continue
+            slots = []
+            for src in self.bld.image_sources[l]:
+                if id(src) not in slot_of:
+                    slot_of[id(src)] = len(self.image_order)
+                    self.image_order.append(src)
+                slots.append(slot_of[id(src)])
+            out.append((l, np.array(slots, dtype=np.int32)))
+        return out
+
+    def _kinterp_address(self, l):
+        """The device address of a Lanczos k interpolant's coefficient block, as the bits of p[2]."""
+        ki = self.bld.image_kinterp.get(l)
+        if ki is None:
+            return None
+        return np.array([ki._table.kdevice().data_ptr()], dtype=np.uint64).view(np.float64)[0]
+
+    def _upload_records(self):
         B, L = self.B, self.L
         leaves = stack_records(self.bld.leaves)               # (B, L)
         self.sersic_n = None
@@ -191,30 +308,12 @@ class Program(object):
                     leaves['table'][:, l] = slot[k]
                 self.moffat_beta = np.ascontiguousarray(uniq[:, 0])
                 self.moffat_trunc = np.ascontiguousarray(uniq[:, 1])
-        self.image_order = []
-        image_leaves = [l for l in range(L) if self.bld.leaf_types[l] == _lib.INTERPOLATED]
-        if image_leaves:
-            slot_of = {}
-            for l in image_leaves:
-                slots = []
-                for src in self.bld.image_sources[l]:
-                    if id(src) not in slot_of:
-                        slot_of[id(src)] = len(self.image_order)
-                        self.image_order.append(src)
-                    slots.append(slot_of[id(src)])
-                leaves['table'][:, l] = np.broadcast_to(np.array(slots, dtype=np.int32), (B,))
-                ki = self.bld.image_kinterp.get(l)
-                if ki is not None:
-                    # the coefficient block's device address, as the bits of p[2]
-                    addr = np.array([ki._table.kdevice().data_ptr()], dtype=np.uint64).view(np.float64)[0]
-                    leaves['p'][:, l, 2] = addr
+        for l, slots in self._image_slots():
+            leaves['table'][:, l] = np.broadcast_to(slots, (B,))
+            addr = self._kinterp_address(l)
+            if addr is not None:
+                leaves['p'][:, l, 2] = addr
         self.d_leaves = _lib.to_device(leaves)
-        self.d_info = torch.empty(B * L * 2, dtype=torch.float64, device=_lib.Device.torch_device())
-        if self.sersic_n is None and not self.image_order and self.moffat_beta is None:
-            self.tables = None
-        elif getattr(self, 'tables', None) is None:
-            self.tables = _lib.TablePool.acquire()
-            self._pooled_tables = True
 
     def compute_leaves(self):
         """FP64 on the GPU: build the Sersic and truncated-Moffat FT tables, then every leaf's
@@ -287,6 +386,14 @@ class Program(object):
         self._geom = None
         self._graph_state = None
 
+    def _phase_records(self):
+        if not self.bld.phases:
+            return None
+        return _lib.to_device(self.bld.phases[0] if len(self.bld.phases) == 1 else stack_records(self.bld.phases))
+
+    def _scale_records(self):
+        return _lib.to_device(np.stack(self.bld.scales, axis=1)) if self.bld.scales else None
+
     def _stamp_geometry(self, N, Nk, xmin, ymin, nx, ny):
         """Device stamp records sorted by FFT size, with the bucket boundaries; kept for the
         adjoint of the same draw."""
@@ -294,26 +401,33 @@ class Program(object):
         B, L = self.B, self.L
         dev = _lib.Device.torch_device()
         N = np.asarray(N, np.int64)
-        order = np.argsort(N, kind='stable')
+        # (16-bit keys take numpy's radix sort)
+        order = np.argsort(N.astype(np.uint16) if B > 1 and N.max() < 65536 else N, kind='stable')
         nx = np.broadcast_to(np.asarray(nx, np.int64), (B,))
         ny = np.broadcast_to(np.asarray(ny, np.int64), (B,))
         sizes = nx * ny
         offsets = np.zeros(B, np.int64)
         offsets[1:] = np.cumsum(sizes)[:-1]
-        stamps = np.zeros(B, dtype=_lib.STAMP_DTYPE)
-        stamps['N'] = N
-        stamps['Nk'] = Nk
-        stamps['xmin'] = xmin
-        stamps['ymin'] = ymin
-        stamps['nx'] = nx
-        stamps['ny'] = ny
-        stamps['out_offset'] = offsets
+        stamps = np.empty((B, 8), dtype=np.int32)             # STAMP_DTYPE as words
+        for i, v in enumerate((N, Nk, xmin, ymin, nx, ny)):
+            stamps[:, i] = v
+        stamps[:, 6:8] = offsets.view(np.int32).reshape(B, 2)
         perm = torch.from_numpy(order).to(dev)
-        lv = torch.empty(B * L * _lib.LEAF_DTYPE.itemsize, dtype=torch.uint8, device=dev)
-        _lib.permute_records(lv, self.d_leaves, perm)
-        ph = (_lib.to_device(stack_records(self.bld.phases)[order]) if self.bld.phases else None)
-        sc = (_lib.to_device(np.stack(self.bld.scales, axis=1)[order]) if self.bld.scales else None)
-        st = _lib.to_device(stamps[order])
+
+        def sorted_records(raw, nbytes):
+            out = torch.empty(B * nbytes, dtype=torch.uint8, device=dev)
+            return _lib.permute_records(out, raw, perm)
+
+        if B > 1:
+            lv = sorted_records(self.d_leaves, L * _lib.LEAF_DTYPE.itemsize)
+            ph, sc = self._phase_records(), self._scale_records()
+            ph = sorted_records(ph, len(self.bld.phases) * _lib.PHASE_DTYPE.itemsize) if ph is not None else None
+            sc = sorted_records(sc, len(self.bld.scales) * 8) if sc is not None else None
+            st = sorted_records(_lib.to_device(stamps), _lib.STAMP_DTYPE.itemsize)
+        else:
+            # (a copy: the graph of a repeated geometry refreshes it in place)
+            lv = self.d_leaves.clone()
+            ph, sc, st = self._phase_records(), self._scale_records(), _lib.to_device(stamps)
         Ns = N[order]
         bounds = np.flatnonzero(np.diff(Ns)) + 1
         starts = np.concatenate([[0], bounds]).astype(np.int64)
@@ -339,9 +453,11 @@ class Program(object):
         lib = _lib.lib()
         dev = _lib.Device.torch_device()
         main = torch.cuda.current_stream(dev)
-        streams = _lib.Device.side_streams(len(g['buckets']))
-        for (s0, s1), (wbytes, work), st in zip(g['buckets'], works, streams):
+        # a single bucket runs on the caller's stream
+        streams = _lib.Device.side_streams(len(g['buckets'])) if len(g['buckets']) > 1 else []
+        for st in streams:
             st.wait_stream(main)
+        for (s0, s1), (wbytes, work), st in zip(g['buckets'], works, streams or [main]):
             lvp, php, scp, stp = self._bucket_ptrs(g, s0)
             _lib.check(lib.gsb_draw_bucket(
                 ctypes.byref(self.tpl), int(s1 - s0), ctypes.byref(self.gsp_c), lvp, php, scp, stp,
@@ -433,18 +549,29 @@ class Program(object):
         grad_sorted = torch.empty((B, ng), dtype=torch.float64, device=dev)
         stream = _lib.Device.stream()
         lib = _lib.lib()
-        for s0, s1 in zip(g['starts'], g['ends']):
-            n = int(s1 - s0)
-            NN = int(g['Ns'][s0])
-            wbytes = lib.gsb_adjoint_workspace_size(NN, n, precision)
-            work = torch.empty(max(int(wbytes), 8), dtype=torch.uint8, device=dev) if wbytes else None
-            lvp, php, scp, stp = self._bucket_ptrs(g, s0)
-            _lib.check(lib.gsb_adjoint_images(
-                ctypes.byref(self.tpl), n, ctypes.byref(self.gsp_c), lvp, php, scp, stp,
-                self.tables.handle if self.tables else None, NN,
-                _lib.ptr(cot), cot_dtype, ctypes.c_void_p(grad_sorted.data_ptr() + int(s0) * ng * 8),
-                ctypes.c_uint(int(want) & 0xffffffff), precision, _lib.ptr(work),
-                ctypes.c_size_t(int(wbytes)), stream))
+        # one stream per bucket, largest N first, as the forward (the workspaces are allocated on the
+        # caller's stream before the fork and outlive the join)
+        buckets = sorted(zip(g['starts'], g['ends']), key=lambda se: -int(g['Ns'][se[0]]))
+        works = []
+        for s0, s1 in buckets:
+            wbytes = int(lib.gsb_adjoint_workspace_size(int(g['Ns'][s0]), int(s1 - s0), precision))
+            works.append((wbytes, torch.empty(max(wbytes, 8), dtype=torch.uint8, device=dev) if wbytes else None))
+        main = torch.cuda.current_stream(dev)
+        streams = _lib.Device.side_streams(len(buckets)) if len(buckets) > 1 else []
+        for st in streams:
+            st.wait_stream(main)
+        try:
+            for (s0, s1), (wbytes, work), st in zip(buckets, works, streams or [main]):
+                lvp, php, scp, stp = self._bucket_ptrs(g, s0)
+                _lib.check(lib.gsb_adjoint_images(
+                    ctypes.byref(self.tpl), int(s1 - s0), ctypes.byref(self.gsp_c), lvp, php, scp, stp,
+                    self.tables.handle if self.tables else None, int(g['Ns'][s0]),
+                    _lib.ptr(cot), cot_dtype, ctypes.c_void_p(grad_sorted.data_ptr() + int(s0) * ng * 8),
+                    ctypes.c_uint(int(want) & 0xffffffff), precision, _lib.ptr(work),
+                    ctypes.c_size_t(wbytes), ctypes.c_void_p(st.cuda_stream)))
+        finally:
+            for st in streams:
+                main.wait_stream(st)
         grad = torch.empty_like(grad_sorted)
         _lib.permute_records(grad, grad_sorted, g['perm'], scatter=True, stream=stream)
         return grad

@@ -429,6 +429,16 @@ int gsb_draw_bucket(const gsb_template* tpl, int n_stamps, const gsb_gsparams* g
                     void* d_out, int out_dtype, int add_to_image, double* d_added_flux,
                     int precision, void* d_workspace, size_t workspace_bytes, void* stream);
 
+/* Writes the leaf records of a batch from parameter columns: field f of leaf l (f = 0..3 the Jacobian,
+ * 4 the flux, 5..7 p[0..2], 8 the table slot) of stamp s is d_cols[h_offset[9 l + f] + s], or
+ * h_value[9 l + f] for every stamp where h_offset is negative; h_flags[l] are the leaf's flags, to
+ * which GSB_LEAF_JAC_GENERAL is added where the Jacobian has off-diagonal terms.  So only the
+ * parameters that vary cross the bus, in place of records of which half are working space (the
+ * reference builds one SBProfile per object and leaf, pysrc/SBProfile.cpp:27-73).  d_cols: n_cols
+ * doubles (may be null when every offset is negative).  Asynchronous on `stream`. */
+int gsb_expand_leaves(gsb_leaf* d_leaves, int n_stamps, int n_leaves, const double* d_cols, int64_t n_cols,
+                      const int64_t* h_offset, const double* h_value, const int32_t* h_flags, void* stream);
+
 /* Reorders device records between the caller's stamp order and the FFT-size bucket order that
  * gsb_draw_bucket draws (stamps sorted by N, each bucket contiguous), replacing the per-object
  * order of drawFFT calls (gsobject.py:2014-2045) with one launch: scatter = 0 gathers
