@@ -29,6 +29,11 @@ struct AdjLargeArgs {
     int cache_bytes;     // shared memory for the per-stamp caches of the column kernel
 };
 
+template <typename T> __device__ __forceinline__ const Cx<T>* large_twiddles(const double2* tw, int N);
+template <> __device__ __forceinline__ const double2* large_twiddles<double>(const double2* tw, int) { return tw; }
+template <> __device__ __forceinline__ const float2* large_twiddles<float>(const double2* tw, int N)
+{ return reinterpret_cast<const float2*>(tw + N); }
+
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS) adj_large_row_kernel(const __grid_constant__ AdjLargeArgs la)
 {
@@ -53,7 +58,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_row_kernel(const __grid_con
             buf[pmod(G.xmin + i, N)] = cx<T>(g1, g2);
         }
         __syncthreads();
-        block_fft<T, +1>(buf, N, la.tw);
+        block_fft_any<T, THREADS, false>(buf, N, large_twiddles<T>(la.tw, N));
         const int y1 = pmod(G.ymin + 2 * p, N), y2 = pmod(G.ymin + 2 * p + 1, N);
         for (int c = threadIdx.x; c < H; c += blockDim.x) {
             const Cx<T> z = buf[c];
@@ -75,7 +80,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_col_kernel(const __grid_con
     StampSmem& S = A.S;
     size_t off = (sizeof(AdjSmem) + 15) & ~size_t(15);
     Cx<T>* buf = reinterpret_cast<Cx<T>*>(smem_raw + off);
-    off += sizeof(Cx<T>) * N;
+    off += sizeof(Cx<T>) * fft_buf_len<T>(N);
     unsigned char* cache = smem_raw + ((off + 15) & ~size_t(15));
     const int s = blockIdx.y;
     const int lane = threadIdx.x & 31;
@@ -127,7 +132,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_col_kernel(const __grid_con
         for (int y = threadIdx.x; y < N; y += blockDim.x)
             buf[y] = pmod(y - G.ymin, N) < G.ny ? W[(size_t)c * N + y] : cx<T>(T(0), T(0));
         __syncthreads();
-        block_fft<T, +1>(buf, N, la.tw);
+        block_fft_any<T, THREADS, false>(buf, N, large_twiddles<T>(la.tw, N));
         const T wc = (c == 0 || 2 * c == N) ? inv_n2 : T(2) * inv_n2;
         const int alo = ceil_div(-hk - c, N), ahi = floor_div(hk - c, N);
         for (int r = threadIdx.x; r < N; r += blockDim.x) {
@@ -217,15 +222,15 @@ __global__ void adj_large_finalize_kernel(const __grid_constant__ AdjArgs a)
 template <typename T>
 size_t adj_slab_bytes(int N) { return sizeof(Cx<T>) * (size_t)(N / 2 + 1) * N; }
 
-// ROW_THREADS: one block-wide FFT per row pair; COL_THREADS: 512 where the block FFT allows
-// it (N / R <= 2048), so that the reverse pass keeps 128 registers per thread, else 1024.
+// ROW_THREADS: one block-wide FFT per row pair; COL_THREADS: 512 up to N = 8192, so that the reverse
+// pass keeps 128 registers per thread, else 1024.
 template <typename T, int ROW_THREADS, int COL_THREADS>
 int launch_adj_large_t(const AdjArgs& args, int N, void* work, size_t work_bytes, cudaStream_t stream)
 {
     const size_t slab = adj_slab_bytes<T>(N);
     if (!work || work_bytes < slab) return set_error(GSB_ERR_INVALID, "adjoint workspace too small");
-    const size_t row_sm = sizeof(Cx<T>) * N;
-    const size_t base = ((sizeof(AdjSmem) + 15) & ~size_t(15)) + sizeof(Cx<T>) * N;
+    const size_t row_sm = sizeof(Cx<T>) * fft_buf_len<T>(N);
+    const size_t base = ((sizeof(AdjSmem) + 15) & ~size_t(15)) + sizeof(Cx<T>) * fft_buf_len<T>(N);
     if (base + 1024 > kSmemLimit) return set_error(GSB_ERR_UNSUPPORTED, "FFT size too large for this precision");
     const size_t room = kSmemLimit - base - 1024;
     const int cache_bytes = int(std::min<size_t>(room, 160 * 1024) & ~size_t(15));
@@ -276,10 +281,7 @@ int launch_adj_large_t(const AdjArgs& args, int N, void* work, size_t work_bytes
 template <typename T>
 int launch_adj_large(const AdjArgs& args, int N, void* work, size_t work_bytes, cudaStream_t stream)
 {
-    // the block FFT takes N / R <= 4 blockDim.x butterflies per pass (R = 3 for the first pass of
-    // N = 3 * 2^a, else 4)
-    const int first = (N % 3 == 0) ? N / 3 : N / 4;
-    if (first <= 2048 && N / 4 <= 2048) return launch_adj_large_t<T, 1024, 512>(args, N, work, work_bytes, stream);
+    if (N <= 8192) return launch_adj_large_t<T, 1024, 512>(args, N, work, work_bytes, stream);
     return launch_adj_large_t<T, 1024, 1024>(args, N, work, work_bytes, stream);
 }
 

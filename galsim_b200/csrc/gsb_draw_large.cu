@@ -23,6 +23,7 @@ static __global__ void twiddle_kernel(double2* tw, int N)
     double s, c;
     sincospi(2.0 * m / N, &s, &c);
     tw[m] = make_double2(c, s);
+    reinterpret_cast<float2*>(tw + N)[m] = make_float2(float(c), float(s));
 }
 
 static std::map<int, double2*>& twiddle_cache()
@@ -33,7 +34,8 @@ static std::map<int, double2*>& twiddle_cache()
     return cache[dev & 63];
 }
 
-// exp(+2 pi i m / N), m < N, in FP64: built once per (device, N) and kept for the process.
+// exp(+2 pi i m / N), m < N, in FP64 and after it rounded to FP32: built once per (device, N) and kept
+// for the process.
 int fft_twiddles(int N, cudaStream_t stream, const double2** out)
 {
     static std::mutex mu;
@@ -42,7 +44,7 @@ int fft_twiddles(int N, cudaStream_t stream, const double2** out)
     auto it = c.find(N);
     if (it != c.end()) { *out = it->second; return GSB_OK; }
     double2* tw = nullptr;
-    GSB_CUDA_CHECK(cudaMalloc(&tw, sizeof(double2) * N));
+    GSB_CUDA_CHECK(cudaMalloc(&tw, (sizeof(double2) + sizeof(float2)) * N));
     twiddle_kernel<<<(N + 255) / 256, 256, 0, stream>>>(tw, N);
     GSB_CUDA_CHECK(cudaGetLastError());
     GSB_CUDA_CHECK(cudaStreamSynchronize(stream));
@@ -53,7 +55,10 @@ int fft_twiddles(int N, cudaStream_t stream, const double2** out)
 
 namespace {
 
-constexpr int kLargeThreads = 1024;
+template <typename T> __device__ __forceinline__ const Cx<T>* twiddles(const double2* tw, int N);
+template <> __device__ __forceinline__ const double2* twiddles<double>(const double2* tw, int) { return tw; }
+template <> __device__ __forceinline__ const float2* twiddles<float>(const double2* tw, int N)
+{ return reinterpret_cast<const float2*>(tw + N); }
 
 struct LargeArgs {
     DrawArgs a;          // leaves/phases/scales/stamps already offset to the chunk
@@ -63,15 +68,17 @@ struct LargeArgs {
     int cache_bytes;     // shared memory for the per-stamp caches (factored program)
 };
 
+// 256 threads for N <= 1024 (two CTAs an SM), 512 up to 8192, 1024 above: up to 128 registers but for
+// the last, so that four wave vectors a thread and a radix-8 butterfly stay in them.
 template <typename T, int THREADS, bool II>
-__global__ void __launch_bounds__(THREADS) large_col_kernel(const __grid_constant__ LargeArgs la)
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) large_col_kernel(const __grid_constant__ LargeArgs la)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StampSmem& S = *reinterpret_cast<StampSmem*>(smem_raw);
     Cx<T>* buf = reinterpret_cast<Cx<T>*>(smem_raw + ((sizeof(StampSmem) + 15) & ~size_t(15)));
     const DrawArgs& a = la.a;
     const int N = la.N, H = N / 2 + 1;
-    unsigned char* cache = reinterpret_cast<unsigned char*>(buf + N);
+    unsigned char* cache = reinterpret_cast<unsigned char*>(buf + ((fft_buf_len<T>(N) + 1) & ~size_t(1)));
     const int s = blockIdx.y;
     const double dk = 2. * kPi / N;
     load_stamp(S, a.tpl, s, a.leaves, a.phases, a.scales, a.stamps, a.sersic_header, a.sersic_node,
@@ -139,24 +146,33 @@ __global__ void __launch_bounds__(THREADS) large_col_kernel(const __grid_constan
             }
         }
         __syncthreads();
-        block_fft<T, +1>(buf, N, la.tw);
-        for (int r = threadIdx.x; r < N; r += blockDim.x) W[(size_t)c * N + r] = buf[r];
-        __syncthreads();
+        block_fft_any<T, THREADS, true>(buf, N, twiddles<T>(la.tw, N), W + (size_t)c * N);
     }
 }
 
-template <typename T, int THREADS>
-__global__ void __launch_bounds__(THREADS) large_row_kernel(const __grid_constant__ LargeArgs la)
+// Threads of the row kernel: a radix-8 butterfly each, 512 at most (1024 above N = 8192).
+__host__ __device__ constexpr int row_threads(int N)
 {
+    return N > 8192 ? 1024 : N >= 4096 ? 512 : N >= 2048 ? 256 : N >= 1024 ? 128 : 64;
+}
+
+// The rows' FFT reads its inputs straight from the slab and writes the stamp's pixels from its last
+// pass, two image rows a transform.  Bound by the slab's reads (two of a 32-byte sector's values a
+// row pair, the neighbouring pair's in L2) and the shared-memory passes between.
+template <typename T, int N>
+__global__ void __launch_bounds__(row_threads(N)) large_row_kernel(const __grid_constant__ LargeArgs la)
+{
+    constexpr int THREADS = row_threads(N);
+    constexpr int H = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    StampSmem& S = *reinterpret_cast<StampSmem*>(smem_raw);
-    Cx<T>* buf = reinterpret_cast<Cx<T>*>(smem_raw + ((sizeof(StampSmem) + 15) & ~size_t(15)));
+    Cx<T>* buf = reinterpret_cast<Cx<T>*>(smem_raw);
+    __shared__ gsb_stamp geom;
     const DrawArgs& a = la.a;
-    const int N = la.N, H = N / 2 + 1;
     const int s = blockIdx.y;
-    if (threadIdx.x == 0) S.geom = a.stamps[s];
+    if (threadIdx.x == 0) geom = a.stamps[s];
     __syncthreads();
-    const gsb_stamp G = S.geom;
+    const gsb_stamp G = geom;
+    const Cx<T>* tw = twiddles<T>(la.tw, N);
     const Cx<T>* W = reinterpret_cast<const Cx<T>*>(la.W) + (size_t)s * H * N;
     const T inv_n2 = T(1) / (T(N) * T(N));
     const int npairs = (G.ny + 1) / 2;
@@ -165,47 +181,46 @@ __global__ void __launch_bounds__(THREADS) large_row_kernel(const __grid_constan
         const int py1 = G.ymin + 2 * p;
         const bool two = 2 * p + 1 < G.ny;
         const int y1 = pmod(py1, N), y2 = pmod(py1 + 1, N);
-        for (int kx = threadIdx.x; kx < N; kx += blockDim.x) {
-            Cx<T> a1, a2;
-            if (kx < H) {
-                a1 = W[(size_t)kx * N + y1];
-                a2 = two ? W[(size_t)kx * N + y2] : cx<T>(T(0), T(0));
-            } else {
-                a1 = cconj<T>(W[(size_t)(N - kx) * N + y1]);
-                a2 = two ? cconj<T>(W[(size_t)(N - kx) * N + y2]) : cx<T>(T(0), T(0));
-            }
-            buf[kx] = cx<T>(a1.x - a2.y, a1.y + a2.x);
-        }
-        __syncthreads();
-        block_fft<T, +1>(buf, N, la.tw);
         const long long row1 = G.out_offset + (long long)(2 * p) * G.nx;
-        for (int i = threadIdx.x; i < G.nx; i += blockDim.x) {
-            const Cx<T> v = buf[pmod(G.xmin + i, N)];
-            const T v1 = v.x * inv_n2;
-            store_pixel<T>(a.out, a.out_dtype, a.add, row1 + i, v1);
-            double x = double(v1), t = fsum + x;
+        auto load = [&](int kx) {
+            const bool up = kx < H;
+            const Cx<T>* w = W + (size_t)(up ? kx : N - kx) * N;
+            Cx<T> a1 = w[y1], a2 = two ? w[y2] : cx<T>(T(0), T(0));
+            if (!up) { a1 = cconj<T>(a1); a2 = cconj<T>(a2); }
+            return cx<T>(a1.x - a2.y, a1.y + a2.x);
+        };
+        auto add = [&](double x) {        // Neumaier's compensated sum in FP64
+            const double t = fsum + x;
             fcomp += fabs(fsum) >= fabs(x) ? (fsum - t) + x : (x - t) + fsum;
             fsum = t;
-            if (two) {
-                const T v2 = v.y * inv_n2;
-                store_pixel<T>(a.out, a.out_dtype, a.add, row1 + G.nx + i, v2);
-                x = double(v2);
-                t = fsum + x;
-                fcomp += fabs(fsum) >= fabs(x) ? (fsum - t) + x : (x - t) + fsum;
-                fsum = t;
+        };
+        auto store = [&](int x, Cx<T> v) {
+            int i = x - G.xmin % N;
+            if (i >= N) i -= N;
+            if (i < 0) i += N;
+            for (; i < G.nx; i += N) {
+                const T v1 = v.x * inv_n2;
+                store_pixel<T>(a.out, a.out_dtype, a.add, row1 + i, v1);
+                add(double(v1));
+                if (two) {
+                    const T v2 = v.y * inv_n2;
+                    store_pixel<T>(a.out, a.out_dtype, a.add, row1 + G.nx + i, v2);
+                    add(double(v2));
+                }
             }
-        }
+        };
+        block_fft_pass<T, N, THREADS, 1, +1, false, false>(buf, tw, load, store);
         __syncthreads();
     }
     if (a.added_flux) {
         double v = fsum + fcomp;
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        __shared__ double part[kLargeThreads / 32];
+        __shared__ double part[THREADS / 32];
         if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
         __syncthreads();
         if (threadIdx.x == 0) {
             double tot = 0.;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += part[w];
+            for (int w = 0; w < THREADS / 32; ++w) tot += part[w];
             atomicAdd(&a.added_flux[s], tot);
         }
     }
@@ -217,16 +232,51 @@ size_t slab_bytes(int N) { return sizeof(Cx<T>) * (size_t)(N / 2 + 1) * N; }
 template <typename T>
 size_t large_smem() { return ((sizeof(StampSmem) + 15) & ~size_t(15)); }
 
+template <typename T, int N>
+int launch_rows_n(const LargeArgs& la, dim3 grid, cudaStream_t stream)
+{
+    constexpr size_t sm = sizeof(Cx<T>) * fft_buf_len<T>(N);
+    GSB_CUDA_CHECK(cudaFuncSetAttribute(large_row_kernel<T, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    large_row_kernel<T, N><<<grid, row_threads(N), sm, stream>>>(la);
+    GSB_CUDA_CHECK(cudaGetLastError());
+    return GSB_OK;
+}
+
+template <typename T>
+int launch_rows(const LargeArgs& la, int N, dim3 grid, cudaStream_t stream)
+{
+    switch (N) {
+      case 192: return launch_rows_n<T, 192>(la, grid, stream);
+      case 256: return launch_rows_n<T, 256>(la, grid, stream);
+      case 384: return launch_rows_n<T, 384>(la, grid, stream);
+      case 512: return launch_rows_n<T, 512>(la, grid, stream);
+      case 768: return launch_rows_n<T, 768>(la, grid, stream);
+      case 1024: return launch_rows_n<T, 1024>(la, grid, stream);
+      case 1536: return launch_rows_n<T, 1536>(la, grid, stream);
+      case 2048: return launch_rows_n<T, 2048>(la, grid, stream);
+      case 3072: return launch_rows_n<T, 3072>(la, grid, stream);
+      case 4096: return launch_rows_n<T, 4096>(la, grid, stream);
+      case 6144: return launch_rows_n<T, 6144>(la, grid, stream);
+      case 8192: return launch_rows_n<T, 8192>(la, grid, stream);
+      case 12288: return launch_rows_n<T, 12288>(la, grid, stream);
+      case 16384: if constexpr (sizeof(T) == 4) return launch_rows_n<T, 16384>(la, grid, stream);
+    }
+    return set_error(GSB_ERR_UNSUPPORTED, "FFT size too large for this precision");
+}
+
 template <typename T, int THREADS>
 int launch_large_t(const DrawArgs& args, int N, void* work, size_t work_bytes, cudaStream_t stream)
 {
     const size_t slab = slab_bytes<T>(N);
     if (!work || work_bytes < slab) return set_error(GSB_ERR_INVALID, "draw workspace too small");
-    const size_t base = large_smem<T>() + sizeof(Cx<T>) * N;
+    const size_t base = large_smem<T>() + sizeof(Cx<T>) * ((fft_buf_len<T>(N) + 1) & ~size_t(1));
     if (base > kSmemLimit) return set_error(GSB_ERR_UNSUPPORTED, "FFT size too large for this precision");
-    // the rest of shared memory (up to 192 KB) holds the per-stamp caches of the column kernel
+    // the rest of shared memory (up to 192 KB) holds the per-stamp caches of the column kernel; for
+    // N <= 1024 as much as two CTAs an SM leave (axis tables of up to Nk = 5 N and the Sersic nodes)
     const size_t room = kSmemLimit - base > 1024 ? kSmemLimit - base - 1024 : 0;
-    const int cache_bytes = int(std::min<size_t>(room, 192 * 1024) & ~size_t(15));
+    const size_t want = THREADS == 256 ? std::min<size_t>(28 * 1024 + 64 * sizeof(T) / 4 * N, 112 * 1024 - base)
+                                       : size_t(192) * 1024;
+    const int cache_bytes = int(std::min<size_t>(room, want) & ~size_t(15));
     const size_t sm = base + cache_bytes;
     const double2* tw = nullptr;
     int rc = fft_twiddles(N, stream, &tw);
@@ -239,7 +289,6 @@ int launch_large_t(const DrawArgs& args, int N, void* work, size_t work_bytes, c
     else
         GSB_CUDA_CHECK(cudaFuncSetAttribute(large_col_kernel<T, THREADS, false>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-    GSB_CUDA_CHECK(cudaFuncSetAttribute(large_row_kernel<T, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(base)));
     const int chunk = int(std::max<size_t>(1, std::min<size_t>(work_bytes / slab, 65535)));
     DeviceState* st = device_state();
     if (args.added_flux)
@@ -263,20 +312,21 @@ int launch_large_t(const DrawArgs& args, int N, void* work, size_t work_bytes, c
         if (ii) large_col_kernel<T, THREADS, true><<<dim3(gx, n), THREADS, sm, stream>>>(la);
         else large_col_kernel<T, THREADS, false><<<dim3(gx, n), THREADS, sm, stream>>>(la);
         GSB_CUDA_CHECK(cudaGetLastError());
-        const int gr = std::max(1, std::min(N / 2, (2 * st->sm_count + n - 1) / n));
-        large_row_kernel<T, THREADS><<<dim3(gr, n), THREADS, base, stream>>>(la);
-        GSB_CUDA_CHECK(cudaGetLastError());
+        // (as many row CTAs as are resident at once)
+        const int per_sm = std::max(1, std::min(int(kSmemLimit / (sizeof(Cx<T>) * fft_buf_len<T>(N) + 1024)), 1024 / row_threads(N)));
+        const int gr = std::max(1, std::min(N / 2, (per_sm * st->sm_count + n - 1) / n));
+        const int rr = launch_rows<T>(la, N, dim3(gr, n), stream);
+        if (rr) return rr;
     }
     return GSB_OK;
 }
 
-// Threads per CTA: one per row, 256 to 1024.
 template <typename T>
 int launch_large(const DrawArgs& args, int N, void* work, size_t work_bytes, cudaStream_t stream)
 {
-    if (N <= 256) return launch_large_t<T, 256>(args, N, work, work_bytes, stream);
-    if (N <= 512) return launch_large_t<T, 512>(args, N, work, work_bytes, stream);
-    return launch_large_t<T, kLargeThreads>(args, N, work, work_bytes, stream);
+    if (N <= 1024) return launch_large_t<T, 256>(args, N, work, work_bytes, stream);
+    if (N <= 8192) return launch_large_t<T, 512>(args, N, work, work_bytes, stream);
+    return launch_large_t<T, 1024>(args, N, work, work_bytes, stream);
 }
 
 }  // namespace

@@ -10,6 +10,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <type_traits>
 
 namespace gsb {
 
@@ -52,6 +53,18 @@ __device__ __forceinline__ void dft_small(Cx<T>* v)
         v[1] = cadd<T>(s1, s3);
         v[2] = csub<T>(s0, s2);
         v[3] = csub<T>(s1, s3);
+    } else if constexpr (R == 8) {
+        // two 4-point transforms of the even and odd inputs, joined by the 8th roots of unity
+        Cx<T> e[4] = {v[0], v[2], v[4], v[6]}, o[4] = {v[1], v[3], v[5], v[7]};
+        dft_small<T, 4, SIGN>(e);
+        dft_small<T, 4, SIGN>(o);
+        const T h = T(0.70710678118654752440);
+        const Cx<T> i1 = cmul_si<T, SIGN>(o[1]), i3 = cmul_si<T, SIGN>(o[3]);
+        o[1] = cscale<T>(cadd<T>(o[1], i1), h);
+        o[2] = cmul_si<T, SIGN>(o[2]);
+        o[3] = cscale<T>(csub<T>(i3, o[3]), h);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) { v[r] = cadd<T>(e[r], o[r]); v[r + 4] = csub<T>(e[r], o[r]); }
     }
 }
 
@@ -120,6 +133,142 @@ __device__ inline void fill_twiddles(Cx<T>* tw, int N)
         double s, c;
         sincospi(2.0 * m / N, &s, &c);
         tw[m] = cx<T>(T(c), T(s));
+    }
+}
+
+// Block-wide length-N DFT (N = 2^a or 3 * 2^a) in shared memory, Stockham order, N and the thread
+// count known at compile time so that every index is a shift or a constant: radix 8 (4 and 2 for the
+// rest of the power of two), the factor 3 last.  The first pass takes its inputs from load(i) and
+// the last hands its outputs to store(i, value), so that a caller can read from or write to memory
+// without a trip through the buffer.  tw: exp(+2 pi i m / N), m < N, in T (global).  A radix-8
+// butterfly reads three of its seven twiddles and multiplies the others from them.
+// Between passes the values lie padded by one in 16 (8 in double), which spreads a radix-8 butterfly's
+// adjacent outputs over the banks (16 lanes would share one otherwise): buf holds fft_buf_len values.
+// LOAD_BUF / STORE_BUF: load / store address `buf` itself (their pass then waits for the block
+// between reading and writing).  All threads call; on return the last pass's reads of buf are done
+// by this thread only (sync before reusing it).
+template <typename T>
+__host__ __device__ constexpr bool fft_padded(int N) { return sizeof(Cx<T>) * size_t(N) <= 128 * 1024; }
+template <typename T>
+__host__ __device__ constexpr size_t fft_buf_len(int N)
+{ return size_t(N) + (fft_padded<T>(N) ? size_t(N) >> (sizeof(T) == 4 ? 4 : 3) : 0); }
+
+template <typename T, int N, int THREADS, int NS, int SIGN, bool LOAD_BUF, bool STORE_BUF, class Load, class Store>
+__device__ __forceinline__ void block_fft_pass(Cx<T>* buf, const Cx<T>* __restrict__ tw, const Load& load,
+                                               const Store& store)
+{
+    constexpr int REM = N / NS;
+    constexpr int P2 = REM % 3 == 0 ? REM / 3 : REM;      // what is left of the power of two
+    constexpr int R = P2 == 1 ? 3 : P2 == 2 ? 2 : (P2 == 4 || P2 == 16) ? 4 : 8;
+    constexpr int NB = N / R;
+    constexpr int PER = (NB + THREADS - 1) / THREADS;
+    constexpr int TSTEP = N / (NS * R);
+    constexpr bool FIRST = NS == 1, LAST = NS * R == N;
+    auto at = [](int i) { return fft_padded<T>(N) ? i + (i >> (sizeof(T) == 4 ? 4 : 3)) : i; };
+    Cx<T> v[PER][R];
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = int(threadIdx.x) + t * THREADS;
+        if (NB % THREADS == 0 || b < NB) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[t][r] = FIRST ? load(b + r * NB) : buf[at(b + r * NB)];
+            if (NS > 1) {
+                const int k = b % NS;
+                auto w = [&](int r) {
+                    Cx<T> z = tw[r * k * TSTEP];
+                    if (SIGN < 0) z.y = -z.y;
+                    return z;
+                };
+                if constexpr (R == 8) {
+                    const Cx<T> w1 = w(1), w2 = w(2), w4 = w(4), w3 = cmul<T>(w1, w2);
+                    v[t][1] = cmul<T>(v[t][1], w1);
+                    v[t][2] = cmul<T>(v[t][2], w2);
+                    v[t][3] = cmul<T>(v[t][3], w3);
+                    v[t][4] = cmul<T>(v[t][4], w4);
+                    v[t][5] = cmul<T>(v[t][5], cmul<T>(w1, w4));
+                    v[t][6] = cmul<T>(v[t][6], cmul<T>(w2, w4));
+                    v[t][7] = cmul<T>(v[t][7], cmul<T>(w3, w4));
+                } else {
+#pragma unroll
+                    for (int r = 1; r < R; ++r) v[t][r] = cmul<T>(v[t][r], w(r));
+                }
+            }
+            dft_small<T, R, SIGN>(v[t]);
+        }
+    }
+    if ((!FIRST || LOAD_BUF) && (!LAST || STORE_BUF)) __syncthreads();
+#pragma unroll
+    for (int t = 0; t < PER; ++t) {
+        const int b = int(threadIdx.x) + t * THREADS;
+        if (NB % THREADS == 0 || b < NB) {
+            const int k = b % NS, base = (b / NS) * (NS * R) + k;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (LAST) store(base + r * NS, v[t][r]);
+                else buf[at(base + r * NS)] = v[t][r];
+            }
+        }
+    }
+    if constexpr (!LAST) {
+        __syncthreads();
+        block_fft_pass<T, N, THREADS, NS * R, SIGN, LOAD_BUF, STORE_BUF>(buf, tw, load, store);
+    }
+}
+
+// In place: buf -> buf, synchronised on return.
+template <typename T, int N, int THREADS>
+__device__ __noinline__ void block_fft_n(Cx<T>* buf, const Cx<T>* __restrict__ tw)
+{
+    block_fft_pass<T, N, THREADS, 1, +1, true, true>(buf, tw, [&](int i) { return buf[i]; },
+                                                     [&](int i, Cx<T> z) { buf[i] = z; });
+    __syncthreads();
+}
+
+// buf -> out[0 .. N) (global), synchronised on return.
+template <typename T, int N, int THREADS>
+__device__ __noinline__ void block_fft_out(Cx<T>* buf, const Cx<T>* __restrict__ tw, Cx<T>* __restrict__ out)
+{
+    block_fft_pass<T, N, THREADS, 1, +1, true, false>(buf, tw, [&](int i) { return buf[i]; },
+                                                      [&](int i, Cx<T> z) { out[i] = z; });
+    __syncthreads();
+}
+
+// The sizes of the split path, one instantiation each (N uniform over the block).  OUT: to `out`.
+template <typename T, int THREADS, bool OUT>
+__device__ __forceinline__ void block_fft_any(Cx<T>* buf, int N, const Cx<T>* __restrict__ tw, Cx<T>* out = nullptr)
+{
+    auto run = [&](auto n) {
+        constexpr int M = decltype(n)::value;
+        if constexpr (M <= 32 * THREADS) {
+            if constexpr (OUT) block_fft_out<T, M, THREADS>(buf, tw, out);
+            else block_fft_n<T, M, THREADS>(buf, tw);
+        }
+    };
+    if constexpr (THREADS <= 512) {
+        switch (N) {
+          case 192: run(std::integral_constant<int, 192>{}); return;
+          case 256: run(std::integral_constant<int, 256>{}); return;
+          case 384: run(std::integral_constant<int, 384>{}); return;
+          case 512: run(std::integral_constant<int, 512>{}); return;
+          case 768: run(std::integral_constant<int, 768>{}); return;
+          case 1024: run(std::integral_constant<int, 1024>{}); return;
+        }
+    }
+    if constexpr (THREADS >= 512) {
+        switch (N) {
+          case 1536: run(std::integral_constant<int, 1536>{}); return;
+          case 2048: run(std::integral_constant<int, 2048>{}); return;
+          case 3072: run(std::integral_constant<int, 3072>{}); return;
+          case 4096: run(std::integral_constant<int, 4096>{}); return;
+          case 6144: run(std::integral_constant<int, 6144>{}); return;
+          case 8192: run(std::integral_constant<int, 8192>{}); return;
+        }
+    }
+    if constexpr (THREADS >= 1024) {
+        switch (N) {
+          case 12288: run(std::integral_constant<int, 12288>{}); return;
+          case 16384: run(std::integral_constant<int, 16384>{}); return;
+        }
     }
 }
 

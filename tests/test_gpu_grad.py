@@ -341,3 +341,26 @@ def test_gradients_vs_differenced_reference_drawimage():
         p = torch.as_tensor(params, device=dev, dtype=torch.float64).requires_grad_(True)
         (m(p).double() * wt).sum().backward()
         _assert_grad_close(p.grad.cpu().numpy(), fd, params, 1e-4)
+
+
+@pytest.mark.parametrize('N,prec', [(2048, 'fp64'), (4096, 'fp32'), (6144, 'fp32'), (8192, 'fp32'), (8192, 'fp64'),
+                                    (12288, 'fp32')])
+def test_large_fft_flux_gradient(N, prec):
+    """The drawing is linear in the flux: d<cot, image>/dflux = <cot, image> / flux, at the sizes of the
+    split adjoint (512- and 1024-thread transforms, odd and even powers of two, and three times them)."""
+    from galsim_b200 import autodiff
+    gsp = galsim.GSParams(minimum_fft_size=N, maximum_fft_size=16384)
+    obj = galsim.Convolve(galsim.Exponential(half_light_radius=1., flux=np.array([3.]), gsparams=gsp).shear(g1=0.1, g2=0.05),
+                          galsim.Gaussian(sigma=0.5, gsparams=gsp))
+    dt = np.float32 if prec == 'fp32' else np.float64
+    plan = autodiff.RecordPlan(obj, 33, 28, 0.4, dtype=dt, precision=prec)
+    rec = plan.records()
+    rec['leaf_flux'] = rec['leaf_flux'].clone().requires_grad_(True)
+    img = autodiff.draw_records(plan, **rec)
+    assert int(plan.last.N[0]) == N
+    cot = torch.as_tensor(np.random.default_rng(2).standard_normal((1, 28, 33)), device=img.device).to(img.dtype)
+    img.backward(cot)
+    want = float((cot.double() * img.detach().double()).sum())
+    got = float((rec['leaf_flux'].grad[0, 0] * 3.))
+    # float: ~1e-7 of the terms |cot| |image|, 924 of them with random signs
+    assert abs(got - want) <= (3e-6 if prec == 'fp32' else 1e-11) * float((cot.double() * img.detach().double()).abs().sum())
