@@ -25,30 +25,50 @@ __device__ inline double gamma_p(double a, double x)
     if (x <= 0.) return 0.;
     const double lpre = -x + a * log(x) - lgamma(a);
     if (x < a + 1.) {
+        // (four terms a step: their divisions are independent and overlap; terms past the stop are
+        // below 1e-17 of the sum and leave it as it is.  The Brent solves on this function took
+        // 65-100 us a batch, one dependent division a term.)
         double term = 1. / a, sum = term;
-        for (int k = 1; k < 1000; ++k) {
-            term *= x / (a + k);
+        for (int k = 1; k < 1000; k += 4) {
+            const double r0 = x / (a + k), r1 = x / (a + (k + 1)), r2 = x / (a + (k + 2)), r3 = x / (a + (k + 3));
+            term *= r0;
+            sum += term;
+            term *= r1;
+            sum += term;
+            term *= r2;
+            sum += term;
+            term *= r3;
             sum += term;
             if (fabs(term) < fabs(sum) * 1e-17) break;
         }
         return sum * exp(lpre);
     } else {
-        const double tiny = 1e-300;
+        // Numerators and denominators of the successive convergents (A&S 3.10.1): a step is a chain of
+        // two multiply-adds, where the form that keeps ratios takes two dependent divisions (the
+        // missing-flux radius, ~8 values of ~80 steps: 42 us).  Rescaled every eight steps, where the
+        // last two convergents are compared (a step grows them by b at most: 1e240 from x = 1e30, beyond
+        // which Q is 0).
+        if (x > 1e30) return 1.;
         double b = x + 1. - a;
-        double c = 1. / tiny;
-        double d = 1. / b;
-        double h = d;
-        for (int i = 1; i < 1000; ++i) {
-            const double an = -i * (i - a);
-            b += 2.;
-            d = an * d + b;
-            if (fabs(d) < tiny) d = tiny;
-            c = b + an / c;
-            if (fabs(c) < tiny) c = tiny;
-            d = 1. / d;
-            const double del = d * c;
-            h *= del;
-            if (fabs(del - 1.) < 1e-16) break;
+        double p0 = 0., q0 = 1., p1 = 1., q1 = b, h = 0.;
+        for (int i = 1; i < 1000; i += 8) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const double an = -double(i + j) * (double(i + j) - a);
+                b += 2.;
+                const double p2 = fma(b, p1, an * p0), q2 = fma(b, q1, an * q0);
+                p0 = p1;
+                q0 = q1;
+                p1 = p2;
+                q1 = q2;
+            }
+            const double s = 1. / q1;
+            h = p1 * s;
+            if (fabs(p0 - h * q0) <= 1e-16 * fabs(h * q0)) break;
+            p0 *= s;
+            q0 *= s;
+            p1 = h;
+            q1 = 1.;
         }
         return 1. - exp(lpre) * h;
     }
@@ -249,19 +269,34 @@ __device__ inline double ogata_dpsi(double t)
 // error ~ exp(-pi^2 / (2 tau)).  Used for the Moffat Fourier transform
 // (src/SBMoffat.cpp:296-345: kV = K_{beta-1}(k) k^{beta-1} * 4 / (Gamma(beta-1) 2^beta)).
 // ---------------------------------------------------------------------------------------
-__device__ inline double moffat_kv_fp64(double nu, double x)
+//
+// WARP: the terms dealt to the lanes of a converged warp (the sum then is the same in all).  A
+// maxk solve is a chain of ~10 such sums: 58 us one term at a time in one thread.
+template <bool WARP>
+__device__ inline double moffat_kv_fp64(double nu, double lognorm_nu, double x)
 {
     if (x <= 0.) return 1.;
     const double tau = 0.125;
-    const double lognorm = (1. - nu) * log(2.) - lgamma(nu) + nu * log(x);
+    const double lognorm = lognorm_nu + nu * log(x);
+    const int lane = WARP ? int(threadIdx.x & 31) : 0;
     // 0.5 * tau * f(0) + tau * sum_{j>=1} f(j tau), terms until negligible
-    double sum = 0.5 * exp(lognorm - x);
-    for (int j = 1; j < 2000; ++j) {
-        const double t = j * tau;
-        const double term = exp(lognorm - x * cosh(t) + nu * t) * 0.5 * (1. + exp(-2. * nu * t));
+    double sum = lane == 0 ? 0.5 * exp(lognorm - x) : 0.;
+    for (int j0 = 1; j0 < 2000; j0 += WARP ? 32 : 1) {
+        const double t = (j0 + lane) * tau, xc = x * cosh(t);
+        const double term = exp(lognorm - xc + nu * t) * 0.5 * (1. + exp(-2. * nu * t));
         sum += term;
-        if (term < 1e-18 * sum && x * cosh(t) > nu * t + 50.) break;
+        const bool done = xc > nu * t + 50.;
+        if (WARP) {
+            // (the terms fall from there on: the next 32 are smaller still)
+            double tot = sum;
+            for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+            if (__all_sync(0xffffffffu, (term < 1e-18 * tot && done) || lane < 31)) return tot * tau;
+        } else if (term < 1e-18 * sum && done) {
+            break;
+        }
     }
+    if (WARP)
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     return sum * tau;
 }
 

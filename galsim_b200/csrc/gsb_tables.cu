@@ -228,6 +228,27 @@ __device__ __forceinline__ void correlate(const double* __restrict__ A, int qlo,
                                           const double* gd, int m, int p, int top, double (&acc)[R],
                                           double (&dacc)[R])
 {
+    if constexpr (R == 1 && P1) {
+        // four partial sums, so that the chain of one node's multiply-adds is not the time
+        double s[4] = {0., 0., 0., 0.}, sd[4] = {0., 0., 0., 0.};
+        int q = qlo;
+#pragma unroll 2
+        for (; q + 3 <= qhi; q += 4) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double a = A[q + i];
+                s[i] = fma(a, g[q + i - m], s[i]);
+                if (DN) sd[i] = fma(a, gd[q + i - m], sd[i]);
+            }
+        }
+        for (; q <= qhi; ++q) {
+            s[0] = fma(A[q], g[q - m], s[0]);
+            if (DN) sd[0] = fma(A[q], gd[q - m], sd[0]);
+        }
+        acc[0] += (s[0] + s[1]) + (s[2] + s[3]);
+        if (DN) dacc[0] += (sd[0] + sd[1]) + (sd[2] + sd[3]);
+        return;
+    }
     double w[R], wd[R];
     if (P1) {
 #pragma unroll
@@ -661,17 +682,18 @@ __device__ void natural_spline(const double* x, const double* y, double* z, doub
 // Bound by the latency of the multiply-add chains and the shared-memory reads that feed them (R = 3:
 // one read per three).  4096 tables, n in 0.5 .. 4: 1.05 ms, where integrating each node pair by
 // its scattered sums (three exponentials a pair of terms) in rounds with a scan and a spline
-// kernel after them took 10.3 ms; 113 tables 0.31 ms, 1.4 before.
+// kernel after them took 10.3 ms; 113 tables 0.16 ms (0.31 with one
+// sum a node and the level values read from L2), 1.4 before.
 // R = 1 with 512 threads serves builds of a few tables per SM (kSmallBuild), where a block's
 // latency counts and SMs are idle.
 //
-// Dynamic shared memory: [G samples | (DN) derivative samples | values | (DN) derivative values],
-// gcap + pad doubles a sample array and stride doubles a value array; the spline's right-hand side
-// takes the place of the samples.
+// Dynamic shared memory: [G samples | (DN) derivative samples | values | (DN) derivative values | flags |
+// staged level values], gcap + pad doubles a sample array and stride doubles a value array; the
+// spline's right-hand side takes the place of the samples.
 template <int R, int THREADS, bool DN, bool P1>
 __global__ void __launch_bounds__(THREADS, THREADS > 64 ? 1 : 8) sersic_table_kernel(
     double* header, int count, int stride, gsb_gsparams gsp, const __grid_constant__ OgataLog lg, int p, int gcap,
-    int pad, const SersicScan* scan, const double* tvals, double4* nodes, double4* dnodes, double* dheader,
+    int pad, int stage, const SersicScan* scan, const double* tvals, double4* nodes, double4* dnodes, double* dheader,
     int* status_out)
 {
     extern __shared__ double tsm[];
@@ -728,6 +750,11 @@ __global__ void __launch_bounds__(THREADS, THREADS > 64 ? 1 : 8) sersic_table_ke
     };
 
     unsigned char* ok = reinterpret_cast<unsigned char*>(DN ? DV + stride : V + stride);
+    // the first `stage` level values, for the small builds: a block alone on its SM would wait for each
+    // line of them from L2
+    double* staged = reinterpret_cast<double*>(ok + ((stride + 15) & ~7));
+    for (int i = threadIdx.x; i < stage; i += THREADS) staged[i] = lg.a[i];
+    __syncthreads();
     for (int c0 = 0; c0 < ncand; c0 += THREADS * R) {
         const int c1 = min(ncand, c0 + THREADS * R);
         const int w0 = c0 + int(threadIdx.x >> 5) * 32 * R;      // this warp's nodes w0 .. w0 + 32 R - 1
@@ -757,7 +784,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > 64 ? 1 : 8) sersic_table_ke
                 }
                 const int j = l - kLogLev0;
                 const int qmin = lg.qmin[j];
-                const double* A = lg.a + lg.off[j] - qmin;
+                const double* A = (lg.off[j] + lg.len[j] <= stage ? staged : lg.a) + lg.off[j] - qmin;
                 // the nodes still at work in this warp bound the samples that count
                 int mhi = 0;
 #pragma unroll
@@ -1140,9 +1167,10 @@ __global__ void kolmogorov_finalize_kernel(int ncand, double dlogr, gsb_gsparams
 
 // kV2 for the Moffat maxk solve (MoffatMaxKSolver, SBMoffat.cpp:481-520), normalised to 1
 // at k = 0, as a function of ksq.
+template <bool WARP>
 struct MoffatKV2 {
     int mode;
-    double nu, thresh;
+    double nu, lognorm, thresh;
     __device__ double operator()(double ksq) const
     {
         const double k = sqrt(ksq);
@@ -1150,7 +1178,7 @@ struct MoffatKV2 {
         if (mode == 1) v = exp(-k);
         else if (mode == 2) v = exp(-k) * (1. + k);
         else if (mode == 3) v = exp(-k) * (3. + (3. + k) * k) / 3.;
-        else v = moffat_kv_fp64(nu, k);
+        else v = moffat_kv_fp64<WARP>(nu, lognorm, k);
         return v - thresh;
     }
 };
@@ -1169,11 +1197,14 @@ struct ImageRefs {
     int count;
 };
 
+// WARP: a warp per leaf, all lanes in step (few leaves, where the chain of one thread is the time);
+// else a thread per leaf.
+template <bool WARP>
 __global__ void prepare_leaves_kernel(const __grid_constant__ gsb_template tpl, int n_stamps, gsb_gsparams gsp,
                                       gsb_leaf* leaves, const double* sersic_header, MoffatRefs moffat,
                                       double kolm_stepk, ImageRefs images, double* info, int* status_out)
 {
-    const long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const long long idx = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / (WARP ? 32 : 1);
     if (idx >= (long long)n_stamps * tpl.n_leaves) return;
     const int l = int(idx % tpl.n_leaves);
     gsb_leaf& L = leaves[idx];
@@ -1253,8 +1284,9 @@ __global__ void prepare_leaves_kernel(const __grid_constant__ gsb_template tpl, 
             else if (fabs(beta - 4.) < kacc) { nu = 3.; }
             L.d[2] = mode;
             L.d[3] = nu;
-            L.d[4] = (1. - nu) * log(2.) - lgamma(nu);
-            MoffatKV2 f{mode, nu, gsp.maxk_threshold};
+            const double lognorm = (1. - nu) * log(2.) - lgamma(nu);
+            L.d[4] = lognorm;
+            MoffatKV2<WARP> f{mode, nu, lognorm, gsp.maxk_threshold};
             RootResult r = solve_bracket_upper(f, 0., 100.);
             if (!r.ok) atomicOr(status_out, 4);
             maxk = sqrt(r.x) / rD;
@@ -1499,7 +1531,9 @@ static int ogata_log_levels(DeviceState* st, double h, cudaStream_t stream, Ogat
     return rc;
 }
 
-// Builds of at most this many tables per SM take one 512-thread block of single nodes a table.
+// Builds of at most this many tables per SM take one 512-thread block of single nodes a table: 400
+// tables 295 us against 448 with the three-node blocks, 580 tables 403 against 465; it grows by
+// 0.6 us a table from there, and the others reach 466 us at 1024.
 constexpr int kSmallBuild = 4;
 
 template <int R, int THREADS>
@@ -1515,7 +1549,7 @@ static int launch_sersic_tables(gsb_tables* t, int count, int stride, double nma
     const int pad = p == 1 ? 33 * R : 1;
     const bool dn = dheader != nullptr;
     // per table: the samples (or the spline's right-hand side), the values, one flag byte a node
-    const size_t fixed = (size_t)stride * (dn ? 2 : 1) * sizeof(double) + stride + 16;
+    const size_t fixed = (size_t)stride * (dn ? 2 : 1) * sizeof(double) + ((stride + 15) & ~7);
     const size_t room = 226 * 1024 - sizeof(double) * 4 * THREADS * R;
     const size_t per = sizeof(double) * (dn ? 2 : 1);
     // as many samples as the tables need, at least the right-hand side's room (samples that do not
@@ -1524,11 +1558,15 @@ static int launch_sersic_tables(gsb_tables* t, int count, int stride, double nma
     const size_t least = std::max<size_t>(64, dn ? stride / 2 + 1 : stride);
     if (fixed + per * (least + pad) > room) return set_error(GSB_ERR_UNSUPPORTED, "Sersic table too long");
     gcap = std::max(std::min(gcap, (room - fixed) / per - pad), least);
-    const size_t sm = fixed + per * (gcap + pad);
+    // one-node builds: the levels 5 .. 20 next to them where they fit
+    int stage = 0;
+    for (int j = 0; R == 1 && j < 16; ++j)
+        if (fixed + per * (gcap + pad) + sizeof(double) * (lg.off[j] + lg.len[j]) <= room) stage = lg.off[j] + lg.len[j];
+    const size_t sm = fixed + per * (gcap + pad) + sizeof(double) * stage;
     auto go = [&](auto kernel) -> int {
         if (sm + sizeof(double) * 4 * THREADS * R > 47 * 1024)
             GSB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-        kernel<<<count, THREADS, sm, stream>>>(t->d_header, count, stride, *gsp, lg, p, int(gcap), pad, scan, t->d_val,
+        kernel<<<count, THREADS, sm, stream>>>(t->d_header, count, stride, *gsp, lg, p, int(gcap), pad, stage, scan, t->d_val,
                                                t->d_node, dnode, dheader, d_status);
         GSB_CUDA_CHECK(cudaGetLastError());
         return GSB_OK;
@@ -1877,8 +1915,13 @@ int prepare_leaves(const gsb_template* tpl, int n_stamps, const gsb_gsparams* gs
     GSB_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int), stream));
     const long long n = (long long)n_stamps * tpl->n_leaves;
     if (n > 0) {
-        prepare_leaves_kernel<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(
-            *tpl, n_stamps, *gsp, d_leaves, t ? t->d_header : nullptr, moffat, kolm, images, d_info, d_status);
+        // a warp per leaf while that does not fill the GPU
+        if (n <= 16LL * st->sm_count)
+            prepare_leaves_kernel<true><<<(unsigned)((n * 32 + 127) / 128), 128, 0, stream>>>(
+                *tpl, n_stamps, *gsp, d_leaves, t ? t->d_header : nullptr, moffat, kolm, images, d_info, d_status);
+        else
+            prepare_leaves_kernel<false><<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(
+                *tpl, n_stamps, *gsp, d_leaves, t ? t->d_header : nullptr, moffat, kolm, images, d_info, d_status);
         GSB_CUDA_CHECK(cudaGetLastError());
     }
     int h_status = 0;
