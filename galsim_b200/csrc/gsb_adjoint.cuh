@@ -383,6 +383,14 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
     }
 }
 
+// In-place transform of the warp's buffer (values at fft_slot).
+template <typename T, int N>
+__device__ __forceinline__ void adj_warp_fft(Cx<T>* buf, const Cx<T>* tw)
+{
+    warp_fft_io<T, N, +1, true, true>(buf, tw, [&](int i) { return buf[fft_slot(i)]; },
+                                      [&](int i, Cx<T> z) { buf[fft_slot(i)] = z; });
+}
+
 template <typename T>
 __device__ inline T load_cot(const void* p, int dtype, long long idx)
 {
@@ -471,14 +479,14 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <=
             for (int i = lane; i < G.nx; i += 32) {
                 const T g1 = load_cot<T>(a.cot, a.cot_dtype, row1 + i);
                 const T g2 = two ? load_cot<T>(a.cot, a.cot_dtype, row1 + G.nx + i) : T(0);
-                buf[pmod(G.xmin + i, N)] = cx<T>(g1, g2);
+                buf[fft_slot(pmod(G.xmin + i, N))] = cx<T>(g1, g2);
             }
             __syncwarp();
-            warp_fft<T, N, +1>(buf, tw);
+            adj_warp_fft<T, N>(buf, tw);
             const int y1 = pmod(G.ymin + 2 * p, N), y2 = pmod(G.ymin + 2 * p + 1, N);
             for (int c = lane; c < H; c += 32) {
-                const Cx<T> z = buf[c];
-                const Cx<T> zm = buf[c == 0 ? 0 : N - c];
+                const Cx<T> z = buf[fft_slot(c)];
+                const Cx<T> zm = buf[fft_slot(c == 0 ? 0 : N - c)];
                 W[(size_t)c * WS + y1] = cx<T>(T(0.5) * (z.x + zm.x), T(0.5) * (z.y - zm.y));
                 if (two) W[(size_t)c * WS + y2] = cx<T>(T(0.5) * (z.y + zm.y), T(0.5) * (zm.x - z.x));
             }
@@ -498,15 +506,15 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <=
 #pragma unroll
             for (int e = 0; e < kGradPerPhase; ++e) ga[t][e] = T(0);
         for (int c = warp; c < H; c += NW) {
-            for (int y = lane; y < N; y += 32)
-                buf[y] = pmod(y - G.ymin, N) < G.ny ? W[(size_t)c * WS + y] : cx<T>(T(0), T(0));
-            __syncwarp();
-            warp_fft<T, N, +1>(buf, tw);
+            const Cx<T>* Wc = W + (size_t)c * WS;
+            warp_fft_io<T, N, +1, false, true>(
+                buf, tw, [&](int y) { return pmod(y - G.ymin, N) < G.ny ? Wc[y] : cx<T>(T(0), T(0)); },
+                [&](int i, Cx<T> z) { buf[fft_slot(i)] = z; });
             const T wc = (c == 0 || 2 * c == N) ? inv_n2 : T(2) * inv_n2;
             const int kx0 = c + ceil_div(-hk - c, N) * N;
             // the column's rows ky = -hk .. hk in order, every alias once, as the forward takes them
             for (int ky = -hk + lane; ky <= hk; ky += 32) {
-                const Cx<T> gh = cscale<T>(buf[pmod(ky, N)], wc);
+                const Cx<T> gh = cscale<T>(buf[fft_slot(pmod(ky, N))], wc);
                 for (int kx = kx0; kx <= hk; kx += N) {
                     const bool pos = kx >= 0;
                     // an alias taken as conj(F(-k)) contributes Re(Ghat conj(dF)) = Re(conj(Ghat) dF)

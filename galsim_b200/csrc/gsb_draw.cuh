@@ -31,7 +31,7 @@ constexpr int kWarps = 16;          // most warps per CTA
 
 // How a leaf's value is formed at a wave vector.  The named kinds read constants of type T formed
 // once per stamp (LeafT); kLeafGeneric goes through leaf_kvalue.
-enum LeafKind { kLeafGeneric = 0, kLeafSep, kLeafExp, kLeafSersic, kLeafMoffat1, kLeafMoffat2, kLeafMoffat3,
+enum LeafKind { kLeafGeneric = 0, kLeafSep, kLeafExp, kLeafExpFast, kLeafSersic, kLeafMoffat1, kLeafMoffat2, kLeafMoffat3,
                 kLeafMoffatSum, kLeafKolm, kLeafAiry };
 
 // A leaf's constants in the working precision: (u, v) = (a i + c j, b i + d j) is the wave vector of
@@ -424,6 +424,10 @@ __device__ __noinline__ void set_leaf_const(StampSmem& S, int l, double dk, bool
     if (S.leaf_cache[l] >= 0) {
         t.kind = kLeafSep;
         t.cache = S.leaf_cache[l];
+    } else if (L.type == GSB_EXPONENTIAL && S.aux_cache[l] >= 0 && sizeof(T) == 4 && !mixed) {
+        t.kind = kLeafExpFast;
+        t.cache = S.aux_cache[l];
+        size = L.d[0];
     } else if (L.type == GSB_EXPONENTIAL && S.aux_cache[l] >= 0) {
         // (the general path's own order of operations: k = (i dk, j dk), then r0 squared)
         t.kind = kLeafExp;
@@ -808,6 +812,15 @@ __device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned c
         }
         if (kind == kLeafSersic) {
             sersic_points<V>(L, cache, ksq, out);
+        } else if (kind == kLeafExpFast) {
+            // (1 + k^2)^(-3/2) where the clip keeps it
+            const ushort2* R = reinterpret_cast<const ushort2*>(cache + L.cache) + hk + j0;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const ushort2 r = R[v * js];
+                const float s = fast_rsqrt(1.f + ksq[v]);
+                out[v] = i >= int(r.x) && i < int(r.y) ? s * s * s : 0.f;
+            }
         } else if (kind == kLeafKolm) {
             // exp(-(k^2)^(5/6)); log2 of 0 is -inf, and its power 0
 #pragma unroll
@@ -1053,12 +1066,15 @@ __host__ __device__ constexpr int fused_min_blocks()
     return kSmemPerSM / (smem_bytes<T, N>(w_fits_smem<T, N>()) + 1024) >= 2 ? 2 : 1;
 }
 
-// Bound by instruction issue and its latencies: of ~94 K warp instructions of a 64 x 64 stamp at
-// N = 128 the k-space evaluation takes half, the FFTs a sixth; issue slots 35 % active with the 16
-// warps that 128 registers leave.  Against one wave vector a lane with constants converted from the
-// FP64 records at each (179 K warp instructions): catalog stamps (Sersic x Kolmogorov) N = 128 1.36 ->
-// 1.11 ms, N = 192 1.00 -> 0.85; bulge + disk x Moffat (general beta) N = 128 5.4 -> 2.9, N = 192
-// 14.6 -> 6.0 ms, 16384 stamps.
+// Bound by instruction issue and its latencies, with the 16 warps an SM that 128 registers leave: the
+// k-space evaluation is half the instructions, the FFTs a sixth.  686 catalog stamps (Sersic x
+// Kolmogorov) at N = 128: 222 us with the evaluator as a call and each FFT in its buffer, 182 with the
+// evaluator of the float kernels compiled in place (its callers' registers need not be saved), the
+// column FFT's last pass writing W and the rows' first reading it; N = 192 100 -> 89.  (Compiled in
+// place for the double and image kernels, or a row FFT that writes pixels from its last pass, it
+// spills: 239 us.)  Before both, one wave vector a lane with constants converted from the FP64
+// records at each: bulge + disk x Moffat (general beta), 16384 stamps, N = 128 5.4 ms and N = 192 14.6
+// against 2.9 and 6.0 with the calls.
 template <typename T, int N, bool WSMEM, bool II = true>
 __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, N>()) draw_fused_kernel(const __grid_constant__ DrawArgs a)
 {
@@ -1141,8 +1157,8 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
                         for (int e0 = -hk + 32 * s0; e0 <= top; e0 += N) {
                             if (e0 + 32 * V - 1 <= top) {
                                 const int ky = e0 + lane;
-                                const Values<T, V> z = eval_any<T, II, V>(a.tpl, S, cache, ii, pos ? ky : -ky,
-                                                                          pos ? 32 : -32, hk, dk);
+                                const Values<T, V> z = eval_any<T, II, V, !II && sizeof(T) == 4>(a.tpl, S, cache, ii, pos ? ky : -ky,
+                                                                                        pos ? 32 : -32, hk, dk);
 #pragma unroll
                                 for (int v = 0; v < V; ++v) {
                                     const Cx<T> w = pos ? z.v[v] : cconj<T>(z.v[v]);
@@ -1166,12 +1182,12 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
                         }
                     }
 #pragma unroll
-                    for (int v = 0; v < V; ++v) buf[pmod(-hk + 32 * (s0 + v) + lane, N)] = acc[v];
+                    for (int v = 0; v < V; ++v) buf[fft_slot(pmod(-hk + 32 * (s0 + v) + lane, N))] = acc[v];
                 }
                 __syncwarp();
-                warp_fft<T, N, +1>(buf, tw);
-                for (int r = lane; r < N; r += 32) W[(size_t)c * WS + r] = buf[r];
-                __syncwarp();
+                Cx<T>* Wc = W + (size_t)c * WS;
+                warp_fft_io<T, N, +1, true, false>(buf, tw, [&](int i) { return buf[fft_slot(i)]; },
+                                                   [&](int i, Cx<T> z) { Wc[i] = z; });
             }
         } else {
             for (int c = warp; c < H; c += NW) {
@@ -1187,12 +1203,12 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
                             kahan_add<T>(acc, comp, pos ? v : cconj<T>(v));
                         }
                     }
-                    buf[r] = acc;
+                    buf[fft_slot(r)] = acc;
                 }
                 __syncwarp();
-                warp_fft<T, N, +1>(buf, tw);
-                for (int r = lane; r < N; r += 32) W[(size_t)c * WS + r] = buf[r];
-                __syncwarp();
+                Cx<T>* Wc = W + (size_t)c * WS;
+                warp_fft_io<T, N, +1, true, false>(buf, tw, [&](int i) { return buf[fft_slot(i)]; },
+                                                   [&](int i, Cx<T> z) { Wc[i] = z; });
             }
         }
         __syncthreads();
@@ -1200,41 +1216,40 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
         // ---- row phase: two image rows per complex transform ----
         const gsb_stamp& G = S.geom;
         const int npairs = (G.ny + 1) / 2;
+        const int xstart = pmod(G.xmin, N);
         double fsum = 0., fcomp = 0.;
         for (int p = warp; p < npairs; p += NW) {
             const int py1 = G.ymin + 2 * p;
             const bool two = 2 * p + 1 < G.ny;
             const int y1 = pmod(py1, N), y2 = pmod(py1 + 1, N);
-            for (int kx = lane; kx < N; kx += 32) {
-                Cx<T> a1, a2;
-                if (kx < H) {
-                    a1 = W[(size_t)kx * WS + y1];
-                    a2 = two ? W[(size_t)kx * WS + y2] : cx<T>(T(0), T(0));
-                } else {
-                    a1 = cconj<T>(W[(size_t)(N - kx) * WS + y1]);
-                    a2 = two ? cconj<T>(W[(size_t)(N - kx) * WS + y2]) : cx<T>(T(0), T(0));
-                }
-                buf[kx] = cx<T>(a1.x - a2.y, a1.y + a2.x);
-            }
-            __syncwarp();
-            warp_fft<T, N, +1>(buf, tw);
             const long long row1 = G.out_offset + (long long)(2 * p) * G.nx;
+            // the transform reads the two rows from W
+            auto load = [&](int kx) {
+                const bool up = kx < H;
+                const Cx<T>* w = W + (size_t)(up ? kx : N - kx) * WS;
+                Cx<T> a1 = w[y1], a2 = two ? w[y2] : cx<T>(T(0), T(0));
+                if (!up) { a1 = cconj<T>(a1); a2 = cconj<T>(a2); }
+                return cx<T>(a1.x - a2.y, a1.y + a2.x);
+            };
+            warp_fft_io<T, N, +1, false, true>(buf, tw, load, [&](int i, Cx<T> z) { buf[fft_slot(i)] = z; });
+#pragma unroll 1
             for (int i = lane; i < G.nx; i += 32) {
-                const Cx<T> v = buf[pmod(G.xmin + i, N)];
-                const T v1 = v.x * inv_n2;
-                store_pixel<T>(a.out, a.out_dtype, a.add, row1 + i, v1);
-                // Neumaier compensated sum in FP64
-                const double x1 = double(v1);
-                double tsum = fsum + x1;
-                fcomp += fabs(fsum) >= fabs(x1) ? (fsum - tsum) + x1 : (x1 - tsum) + fsum;
-                fsum = tsum;
-                if (two) {
-                    const T v2 = v.y * inv_n2;
-                    store_pixel<T>(a.out, a.out_dtype, a.add, row1 + G.nx + i, v2);
-                    const double x2 = double(v2);
-                    tsum = fsum + x2;
-                    fcomp += fabs(fsum) >= fabs(x2) ? (fsum - tsum) + x2 : (x2 - tsum) + fsum;
-                    fsum = tsum;
+                int x = xstart + i;
+                while (x >= N) x -= N;
+                const Cx<T> v = buf[fft_slot(x)];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    if (r == 1 && !two) break;
+                    const T px = (r ? v.y : v.x) * inv_n2;
+                    store_pixel<T>(a.out, a.out_dtype, a.add, row1 + (r ? G.nx : 0) + i, px);
+                    const double d = double(px);
+                    if (sizeof(T) == 4) {          // (float pixels: exact to ~1e-13 in a plain FP64 sum)
+                        fsum += d;
+                    } else {                       // Neumaier compensated sum in FP64
+                        const double tsum = fsum + d;
+                        fcomp += fabs(fsum) >= fabs(d) ? (fsum - tsum) + d : (d - tsum) + fsum;
+                        fsum = tsum;
+                    }
                 }
             }
             __syncwarp();

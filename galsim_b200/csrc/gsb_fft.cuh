@@ -68,12 +68,22 @@ __device__ __forceinline__ void dft_small(Cx<T>* v)
     }
 }
 
-template <typename T, int N, int R, int NS, int SIGN>
-__device__ __forceinline__ void stockham_pass(Cx<T>* buf, const Cx<T>* tw, int lane)
+// Where value i of a warp's buffer lies: bits 4-5 of the index are folded into bits 0-1 and 2-3, so
+// that 16 lanes storing with stride 1, 4 or 16 values (the radix-4 passes' outputs), or loading
+// consecutive ones, touch 16 different bank pairs (without it the first two passes' stores take
+// four times as long).
+__device__ __forceinline__ int fft_slot(int i) { return i ^ (((i >> 4) & 3) * 5); }
+
+// One pass of the warp transform.  The first takes its inputs from load(i), the last hands its
+// outputs to store(i, value); between passes the values are in buf (fft_slot).  LOAD_BUF / STORE_BUF:
+// load / store address buf, so the warp waits between reading and writing.
+template <typename T, int N, int R, int NS, int SIGN, bool LOAD_BUF, bool STORE_BUF, class Load, class Store>
+__device__ __forceinline__ void stockham_pass(Cx<T>* buf, const Cx<T>* tw, int lane, const Load& load, const Store& store)
 {
     constexpr int NB = N / R;
     constexpr int PER = (NB + 31) / 32;
     constexpr int TSTEP = N / (NS * R);
+    constexpr bool FIRST = NS == 1, LAST = NS * R == N;
     Cx<T> v[PER][R];
 #pragma unroll
     for (int t = 0; t < PER; ++t) {
@@ -81,7 +91,7 @@ __device__ __forceinline__ void stockham_pass(Cx<T>* buf, const Cx<T>* tw, int l
         if (NB % 32 == 0 || b < NB) {
             const int k = b % NS;
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[t][r] = buf[b + r * NB];
+            for (int r = 0; r < R; ++r) v[t][r] = FIRST ? load(b + r * NB) : buf[fft_slot(b + r * NB)];
 #pragma unroll
             for (int r = 1; r < R && NS > 1; ++r) {      // (the first pass's twiddles are 1)
                 // r k TSTEP <= (R - 1)(NS - 1) N / (NS R) < N: no reduction mod N needed
@@ -93,7 +103,7 @@ __device__ __forceinline__ void stockham_pass(Cx<T>* buf, const Cx<T>* tw, int l
             dft_small<T, R, SIGN>(v[t]);
         }
     }
-    __syncwarp();
+    if ((!FIRST || LOAD_BUF) && (!LAST || STORE_BUF)) __syncwarp();
 #pragma unroll
     for (int t = 0; t < PER; ++t) {
         const int b = lane + 32 * t;
@@ -101,28 +111,32 @@ __device__ __forceinline__ void stockham_pass(Cx<T>* buf, const Cx<T>* tw, int l
             const int k = b % NS;
             const int base = (b / NS) * NS * R + k;
 #pragma unroll
-            for (int r = 0; r < R; ++r) buf[base + r * NS] = v[t][r];
+            for (int r = 0; r < R; ++r) {
+                if (LAST) store(base + r * NS, v[t][r]);
+                else buf[fft_slot(base + r * NS)] = v[t][r];
+            }
         }
     }
     __syncwarp();
 }
 
-template <typename T, int N, int NS, int SIGN>
-__device__ __forceinline__ void fft_passes(Cx<T>* buf, const Cx<T>* tw, int lane)
+template <typename T, int N, int NS, int SIGN, bool LOAD_BUF, bool STORE_BUF, class Load, class Store>
+__device__ __forceinline__ void fft_passes(Cx<T>* buf, const Cx<T>* tw, int lane, const Load& load, const Store& store)
 {
     if constexpr (NS < N) {
         constexpr int rem = N / NS;
         constexpr int R = (NS == 1 && (N % 3) == 0) ? 3 : ((rem % 4) == 0 ? 4 : 2);
-        stockham_pass<T, N, R, NS, SIGN>(buf, tw, lane);
-        fft_passes<T, N, NS * R, SIGN>(buf, tw, lane);
+        stockham_pass<T, N, R, NS, SIGN, LOAD_BUF, STORE_BUF>(buf, tw, lane, load, store);
+        fft_passes<T, N, NS * R, SIGN, LOAD_BUF, STORE_BUF>(buf, tw, lane, load, store);
     }
 }
 
-// In-place length-N DFT of buf (shared memory) by the calling warp.  All 32 lanes must call.
-template <typename T, int N, int SIGN>
-__device__ __forceinline__ void warp_fft(Cx<T>* buf, const Cx<T>* tw)
+// Length-N DFT by the calling warp (all 32 lanes call) from load(i) to store(i, value); buf holds N
+// values of working space.  LOAD_BUF / STORE_BUF: load / store address buf[fft_slot(i)].
+template <typename T, int N, int SIGN, bool LOAD_BUF, bool STORE_BUF, class Load, class Store>
+__device__ __forceinline__ void warp_fft_io(Cx<T>* buf, const Cx<T>* tw, const Load& load, const Store& store)
 {
-    fft_passes<T, N, 1, SIGN>(buf, tw, threadIdx.x & 31);
+    fft_passes<T, N, 1, SIGN, LOAD_BUF, STORE_BUF>(buf, tw, threadIdx.x & 31, load, store);
 }
 
 // tw[m] = exp(+2 pi i m / N), filled by the whole block.
@@ -272,12 +286,10 @@ __device__ __forceinline__ void block_fft_any(Cx<T>* buf, int N, const Cx<T>* __
     }
 }
 
-constexpr int kBlockFftMaxPerThread = 4;   // N / R <= 4096 butterflies per pass at 1024 threads
-
-// Block-wide in-place Stockham FFT of length N (2^a or 3 * 2^a, N / R <= blockDim.x *
-// kBlockFftMaxPerThread) in shared memory, the same radix plan as warp_fft; all threads of the
-// block must call.  tw: exp(+2 pi i m / N) for m < N (global, FP64).
-template <typename T, int SIGN>
+// Block-wide in-place Stockham FFT of length N (2^a or 3 * 2^a, N / R <= PER blockDim.x) in shared
+// memory with warp_fft_io's radix plan; all threads of the block must call.  tw: exp(+2 pi i m / N) for
+// m < N (global, FP64).
+template <typename T, int SIGN, int PER = 4>
 __device__ void block_fft(Cx<T>* buf, int N, const double2* __restrict__ tw)
 {
     int NS = 1;
@@ -286,9 +298,9 @@ __device__ void block_fft(Cx<T>* buf, int N, const double2* __restrict__ tw)
         const int R = (NS == 1 && N % 3 == 0) ? 3 : ((rem % 4) == 0 ? 4 : 2);
         const int NB = N / R;
         const int tstep = N / (NS * R);
-        Cx<T> v[kBlockFftMaxPerThread][4];
+        Cx<T> v[PER][4];
 #pragma unroll
-        for (int t = 0; t < kBlockFftMaxPerThread; ++t) {
+        for (int t = 0; t < PER; ++t) {
             const int b = threadIdx.x + t * blockDim.x;
             if (b < NB) {
                 const int k = b % NS;
@@ -305,7 +317,7 @@ __device__ void block_fft(Cx<T>* buf, int N, const double2* __restrict__ tw)
         }
         __syncthreads();
 #pragma unroll
-        for (int t = 0; t < kBlockFftMaxPerThread; ++t) {
+        for (int t = 0; t < PER; ++t) {
             const int b = threadIdx.x + t * blockDim.x;
             if (b < NB) {
                 const int k = b % NS;
