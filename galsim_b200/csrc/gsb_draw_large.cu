@@ -68,6 +68,18 @@ struct LargeArgs {
     int cache_bytes;     // shared memory for the per-stamp caches (factored program)
 };
 
+// Float arithmetic drawn into a double image (drawImage's default precision with an ImageD) shows the
+// last bit of every operation, and its users compare such images across versions: it keeps the fused
+// kernels' radix plan.  One object at a time is what is drawn so, and its FFTs are a small part of the
+// call (0.8 ms with either plan at N = 256); in a batch of large stamps block_fft_pass is the faster by far
+// (six stamps of N = 4096 .. 8192: 6.3 ms against 11.7).  PER: radix 2 at N = 8192 has 8 butterflies a
+// thread.
+template <int THREADS>
+__device__ __noinline__ void block_fft_mixed(float2* buf, int N, const double2* tw)
+{ block_fft<float, +1, (THREADS >= 1024 ? 4 : 8)>(buf, N, tw); }
+template <int THREADS>
+__device__ __forceinline__ void block_fft_mixed(double2*, int, const double2*) {}
+
 // 256 threads for N <= 1024 (two CTAs an SM), 512 up to 8192, 1024 above: up to 128 registers but for
 // the last, so that four wave vectors a thread and a radix-8 butterfly stay in them.
 template <typename T, int THREADS, bool II>
@@ -146,7 +158,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) large_col_ker
             }
         }
         __syncthreads();
-        block_fft_any<T, THREADS, true>(buf, N, twiddles<T>(la.tw, N), W + (size_t)c * N);
+        if (sizeof(T) == 4 && a.out_dtype == GSB_F64) {
+            block_fft_mixed<THREADS>(buf, N, la.tw);
+            for (int r = threadIdx.x; r < N; r += blockDim.x) W[(size_t)c * N + r] = buf[r];
+            __syncthreads();
+        } else {
+            block_fft_any<T, THREADS, true>(buf, N, twiddles<T>(la.tw, N), W + (size_t)c * N);
+        }
     }
 }
 
@@ -209,7 +227,14 @@ __global__ void __launch_bounds__(row_threads(N)) large_row_kernel(const __grid_
                 }
             }
         };
-        block_fft_pass<T, N, THREADS, 1, +1, false, false>(buf, tw, load, store);
+        if (sizeof(T) == 4 && a.out_dtype == GSB_F64) {
+            for (int kx = threadIdx.x; kx < N; kx += THREADS) buf[kx] = load(kx);
+            __syncthreads();
+            block_fft_mixed<THREADS>(buf, N, la.tw);
+            for (int x = threadIdx.x; x < N; x += THREADS) store(x, buf[x]);
+        } else {
+            block_fft_pass<T, N, THREADS, 1, +1, false, false>(buf, tw, load, store);
+        }
         __syncthreads();
     }
     if (a.added_flux) {

@@ -54,3 +54,15 @@ def test_double_image_keeps_the_general_path():
     sb = galsim.draw_batch(many, nx=48, ny=40, scale=0.2, dtype=np.float64, precision='fp32')
     for a in sb.flat.cpu().numpy().reshape(3, 40, 48):
         assert np.array_equal(a, im.array)
+
+
+@pytest.mark.parametrize('n', [192, 256, 384, 768, 1024, 1536, 2048, 4096, 6144, 8192, 12288])
+def test_one_object_into_a_double_image_by_the_split_path(n):
+    gsp = galsim.GSParams(minimum_fft_size=n, maximum_fft_size=16384, folding_threshold=0.05, stepk_minimum_hlr=1.)
+    obj = galsim.Convolve(galsim.Exponential(flux=np.full(1, 3.), half_light_radius=0.8, gsparams=gsp).shear(g1=0.1, g2=-0.05),
+                          galsim.Moffat(beta=3., fwhm=0.7, gsparams=gsp), galsim.Pixel(0.2, gsparams=gsp))
+    lo, hi = [galsim.draw_batch(obj, nx=41, ny=30, scale=0.2, dtype=np.float64, precision=q) for q in ('fp32', 'fp64')]
+    assert lo.N[0] == n == hi.N[0]
+    a, b = lo.flat.cpu().numpy(), hi.flat.cpu().numpy()
+    # single precision: a few 1e-7 of the value a wave vector, summed over the image with random signs
+    assert np.abs(a - b).max() <= 3e-6 * np.abs(b).max()
