@@ -295,6 +295,42 @@ __device__ __noinline__ void sum_atom_grads(const gsb_template& tpl, const AdjSm
     }
 }
 
+// Values and derivatives of the two leaves of a Sum atom [o0, o0 + 3) (values only where not wanted).
+template <typename T> struct LeafPair { LeafD<T> d[2]; };
+
+template <typename T>
+__device__ __noinline__ LeafPair<T> sum_pair_grads(const gsb_template& tpl, const AdjSmem& A, const unsigned char* cache,
+                                                   unsigned want, T kx, T ky, int i, int j, const GridRef& g, int o0)
+{
+    LeafPair<T> r;
+    r.d[0] = r.d[1] = LeafD<T>{T(0), T(0), T(0), T(0), T(0)};
+#pragma unroll 1
+    for (int q = 0; q < 2; ++q) {
+        const int l = tpl.op_arg[o0 + q];
+        LeafD<T> d{T(0), T(0), T(0), T(0), T(0)};
+        if (want_leaf(want, l)) d = leaf_grad_fast<T>(A, cache, l, i, j, g.n / 2, g, kx, ky);
+        else d.v = leaf_fast<T>(A.S, cache, l, i, j, g.n / 2, g.dk);
+        r.d[1] = d;
+        if (q == 0) r.d[0] = d;
+    }
+    return r;
+}
+
+// The first atom that is a Sum of two leaves with derivatives of their own (bulge + disk), or -1: its
+// leaves are evaluated once, value and derivatives together, and their gradients stay in registers
+// (any other Sum takes its value from eval_range and its derivatives from sum_atom_grads).
+template <bool II>
+__device__ __forceinline__ int sum_pair_atom(const gsb_template& tpl, const StampSmem& S)
+{
+    for (int t = 0; t < S.n_atoms; ++t) {
+        const int o0 = S.atom_o0[t];
+        if (S.atom_kind[t] != kAtomSum || S.atom_o1[t] - o0 != 3) continue;
+        if (II && (S.leaf[tpl.op_arg[o0]].type == GSB_INTERPOLATED || S.leaf[tpl.op_arg[o0 + 1]].type == GSB_INTERPOLATED)) continue;
+        return t;
+    }
+    return -1;
+}
+
 // Factored reverse pass at (i, j): F = prod_a atom_a * XS[i] YS[j]; the cotangent of atom a
 // is u XS YS prod_{b != a} atom_b (prefix and suffix products, no division).  Leaf, phase and
 // scale atoms accumulate into ga[a][*] (registers); subtree atoms run adjoint_range into acc.
@@ -302,7 +338,8 @@ template <typename T, bool II = true>
 __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, const AdjSmem& A,
                                                        const unsigned char* cache, unsigned want, double dk,
                                                        int i, int j, const GridRef& g, Cx<T> u,
-                                                       T (&ga)[kAdjAtoms][kGradPerPhase], T* acc)
+                                                       T (&ga)[kAdjAtoms][kGradPerPhase], T* acc, int pair,
+                                                       T (&gs)[2][kGradPerLeaf])
 {
     const StampSmem& S = A.S;
     const int hk = g.n / 2;
@@ -311,6 +348,7 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
     // ld[a] holds a leaf atom's derivatives, or a phase atom's unit phasor in (gx, gy)
     Cx<T> val[kAdjAtoms], pre[kAdjAtoms];
     LeafD<T> ld[kAdjAtoms];
+    LeafPair<T> ps;
     Cx<T> run = cx<T>(T(1), T(0));
 #pragma unroll
     for (int a = 0; a < kAdjAtoms; ++a) {
@@ -333,8 +371,11 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
                     ld[a] = leaf_grad_fast<T>(A, cache, l, i, j, hk, g, kx, ky);
                     val[a] = cx<T>(ld[a].v, T(0));
                 } else {
-                    val[a] = leaf_cfast<T, II>(S, cache, l, i, j, g);
+                    val[a] = leaf_cfast<T, II, !II && sizeof(T) == 4>(S, cache, l, i, j, g);
                 }
+            } else if (a == pair) {
+                ps = sum_pair_grads<T>(tpl, A, cache, want, kx, ky, i, j, g, o0);
+                val[a] = cx<T>(ps.d[0].v + ps.d[1].v, T(0));
             } else {
                 val[a] = eval_range<T, II>(tpl, S, cache, dk, i, j, g, o0, o1);
             }
@@ -373,6 +414,18 @@ __device__ __forceinline__ void adjoint_point_factored(const gsb_template& tpl, 
                 ga[a][3] += ar * ld[a].gx * ky;
                 ga[a][4] += ar * ld[a].gy * ky;
                 ga[a][5] += ar * ld[a].gn;
+            } else if (a == pair) {
+                const T ar = w.x;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const T gx = ar * ps.d[q].gx, gy = ar * ps.d[q].gy;
+                    gs[q][0] += ar * ps.d[q].unit;
+                    gs[q][1] += gx * kx;
+                    gs[q][2] += gy * kx;
+                    gs[q][3] += gx * ky;
+                    gs[q][4] += gy * ky;
+                    gs[q][5] += ar * ps.d[q].gn;
+                }
             } else if (kind == kAtomSum) {
                 sum_atom_grads<T>(tpl, A, cache, want, kx, ky, i, j, g, w, acc, o0, o1);
             } else {
@@ -408,7 +461,10 @@ __host__ __device__ constexpr int adj_warps()
             kSmemLimit) ? kWarps : kWarps / 2;
 }
 
-template <typename T, int N, bool WSMEM, bool II>
+// PAIR: compiled for programs with a Sum of two leaves (sum_pair_atom), whose 22 registers the others
+// should not pay for: bulge + disk gradients of 2048 stamps at N = 192 4.2 -> 2.3 ms (the leaf of an
+// atom inlined included, 4.2 -> 3.1 by itself), a Sersic fit at N = 128 0.51 ms without against 0.69.
+template <typename T, int N, bool WSMEM, bool II, bool PAIR>
 __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <= 128 ? 2 : 1) adjoint_fused_kernel(const __grid_constant__ AdjArgs a)
 {
     constexpr int NW = adj_warps<T, N>();
@@ -463,10 +519,11 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <=
         fill_dn_cache(A, a.tpl, cache, a.sersic_dheader != nullptr);
         __syncthreads();
         const bool factored = S.xy_cache >= 0 && S.n_atoms <= kAdjAtoms;
+        const int pair = PAIR && factored ? sum_pair_atom<II>(a.tpl, S) : -1;
         bool subtree = !factored;
         if (factored)
             for (int t = 0; t < S.n_atoms; ++t)
-                subtree |= (S.atom_kind[t] == kAtomRange || S.atom_kind[t] == kAtomSum) &&
+                subtree |= t != pair && (S.atom_kind[t] == kAtomRange || S.atom_kind[t] == kAtomSum) &&
                            S.atom_o1[t] - S.atom_o0[t] > 1;
 
         // ---- row phase: forward-sign DFT of pairs of cotangent rows ----
@@ -498,13 +555,15 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <=
         // Each lane accumulates its gradient terms over all of its warp's columns; the warp
         // reduces them once per stamp.
         T acc[kMaxGrad];
-        T ga[kAdjAtoms][kGradPerPhase];
+        T ga[kAdjAtoms][kGradPerPhase], gs[2][kGradPerLeaf];
         if (subtree)
             for (int k = 0; k < ng; ++k) acc[k] = T(0);
 #pragma unroll
         for (int t = 0; t < kAdjAtoms; ++t)
 #pragma unroll
             for (int e = 0; e < kGradPerPhase; ++e) ga[t][e] = T(0);
+#pragma unroll
+        for (int e = 0; e < kGradPerLeaf; ++e) gs[0][e] = gs[1][e] = T(0);
         for (int c = warp; c < H; c += NW) {
             const Cx<T>* Wc = W + (size_t)c * WS;
             warp_fft_io<T, N, +1, false, true>(
@@ -520,7 +579,7 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <=
                     // an alias taken as conj(F(-k)) contributes Re(Ghat conj(dF)) = Re(conj(Ghat) dF)
                     if (factored)
                         adjoint_point_factored<T, II>(a.tpl, A, cache, a.want, dk, pos ? kx : -kx,
-                                                  pos ? ky : -ky, g, pos ? gh : cconj<T>(gh), ga, acc);
+                                                  pos ? ky : -ky, g, pos ? gh : cconj<T>(gh), ga, acc, pair, gs);
                     else
                         adjoint_range<T, II>(a.tpl, A, dk, pos ? kx : -kx, pos ? ky : -ky, g,
                                          pos ? gh : cconj<T>(gh), acc, 0, a.tpl.n_ops);
@@ -556,6 +615,14 @@ __global__ void __launch_bounds__(adj_warps<T, N>() * 32, sizeof(T) == 4 && N <=
                     if (lane == 0) atomicAdd(&A.gacc[base + e], v);
                 }
             }
+            if (pair >= 0)
+#pragma unroll
+                for (int e = 0; e < 2 * kGradPerLeaf; ++e) {
+                    double v = double(gs[e / kGradPerLeaf][e % kGradPerLeaf]);
+                    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                    if (lane == 0)
+                        atomicAdd(&A.gacc[kGradPerLeaf * a.tpl.op_arg[S.atom_o0[pair] + e / kGradPerLeaf] + e % kGradPerLeaf], v);
+                }
         }
         __syncthreads();
         // Sersic leaves given by half-light radius: r0 = hlr / r_e(n), so at fixed hlr
@@ -621,16 +688,21 @@ int launch_adjoint(const AdjArgs& args, size_t work_bytes, cudaStream_t stream)
     const int grid = adj_grid<T, N>(args.n_stamps);
     if (!wsmem && (args.work == nullptr || work_bytes < adj_workspace_bytes_for<T, N>(args.n_stamps)))
         return set_error(GSB_ERR_INVALID, "adjoint workspace too small");
-    // programs without image leaves run the instance compiled without their code
-    if (has_image_leaves(args.tpl)) {
-        GSB_CUDA_CHECK(cudaFuncSetAttribute(adjoint_fused_kernel<T, N, wsmem, true>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-        adjoint_fused_kernel<T, N, wsmem, true><<<grid, adj_warps<T, N>() * 32, sm, stream>>>(args);
-    } else {
-        GSB_CUDA_CHECK(cudaFuncSetAttribute(adjoint_fused_kernel<T, N, wsmem, false>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-        adjoint_fused_kernel<T, N, wsmem, false><<<grid, adj_warps<T, N>() * 32, sm, stream>>>(args);
-    }
+    auto run = [&](auto kernel) -> int {
+        GSB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+        kernel<<<grid, adj_warps<T, N>() * 32, sm, stream>>>(args);
+        return GSB_OK;
+    };
+    // programs without image leaves run the instance compiled without their code, and those with a Sum of
+    // two leaves the one that keeps both in registers (float; in double the registers are not there)
+    bool pair = false;
+    for (int f = 0; f < args.fac.n; ++f)
+        pair = pair || (args.fac.kind[f] == kFactorSum && args.fac.o1[f] - args.fac.o0[f] == 3);
+    int rc;
+    if (has_image_leaves(args.tpl)) rc = run(adjoint_fused_kernel<T, N, wsmem, true, false>);
+    else if (pair && sizeof(T) == 4) rc = run(adjoint_fused_kernel<T, N, wsmem, false, sizeof(T) == 4>);
+    else rc = run(adjoint_fused_kernel<T, N, wsmem, false, false>);
+    if (rc) return rc;
     GSB_CUDA_CHECK(cudaGetLastError());
     return GSB_OK;
 }

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_col_kernel(const __grid_con
                        S.atom_o1[t] - S.atom_o0[t] > 1;
     const Cx<T>* W = reinterpret_cast<const Cx<T>*>(la.W) + (size_t)s * H * N;
     T acc[kMaxGrad];
-    T ga[kAdjAtoms][kGradPerPhase];
+    T ga[kAdjAtoms][kGradPerPhase], gs[2][kGradPerLeaf];      // (gs: no leaf pair in registers here)
     if (subtree)
         for (int k = 0; k < ng; ++k) acc[k] = T(0);
 #pragma unroll
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(THREADS) adj_large_col_kernel(const __grid_con
                     // an alias taken as conj(F(-k)) contributes Re(Ghat conj(dF)) = Re(conj(Ghat) dF)
                     if (factored)
                         adjoint_point_factored<T, II>(a.tpl, A, cache, a.want, dk, pos ? kx : -kx,
-                                                      pos ? ky : -ky, g, pos ? gh : cconj<T>(gh), ga, acc);
+                                                      pos ? ky : -ky, g, pos ? gh : cconj<T>(gh), ga, acc, -1, gs);
                     else
                         adjoint_range<T, II>(a.tpl, A, dk, pos ? kx : -kx, pos ? ky : -ky, g,
                                              pos ? gh : cconj<T>(gh), acc, 0, a.tpl.n_ops);

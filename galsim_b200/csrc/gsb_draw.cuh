@@ -862,8 +862,9 @@ __device__ __noinline__ T leaf_fast(const StampSmem& S, const unsigned char* cac
     return out[0];
 }
 
-// One leaf as a complex value: InterpolatedImage leaves are complex, the others real.
-template <typename T, bool II = true>
+// One leaf as a complex value: InterpolatedImage leaves are complex, the others real.  INL: compiled
+// into the caller.
+template <typename T, bool II = true, bool INL = false>
 __device__ __forceinline__ Cx<T> leaf_cfast(const StampSmem& S, const unsigned char* cache, int arg, int i, int j,
                                             const GridRef& g)
 {
@@ -874,6 +875,11 @@ __device__ __forceinline__ Cx<T> leaf_cfast(const StampSmem& S, const unsigned c
             return ii_sum<T>(S.leaf[arg], E[i], E[hk + 1 + j + hk]);
         }
         return ii_kvalue<T>(S.leaf[arg], g.dk, i, j);
+    }
+    if constexpr (INL) {
+        T out[1];
+        leaf_points<T, 1>(S, cache, arg, i, j, 0, g.n / 2, g.dk, out);
+        return cx<T>(out[0], T(0));
     }
     return cx<T>(leaf_fast<T>(S, cache, arg, i, j, g.n / 2, g.dk), T(0));
 }

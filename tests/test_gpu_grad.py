@@ -364,3 +364,31 @@ def test_large_fft_flux_gradient(N, prec):
     got = float((rec['leaf_flux'].grad[0, 0] * 3.))
     # float: ~1e-7 of the terms |cot| |image|, 924 of them with random signs
     assert abs(got - want) <= (3e-6 if prec == 'fp32' else 1e-11) * float((cot.double() * img.detach().double()).abs().sum())
+
+
+@pytest.mark.parametrize('min_n', [64, 96, 192, 256])
+@pytest.mark.parametrize('leaves,want', [(2, 0b01), (2, 0b10), (2, 0b11), (3, 0b101)])
+def test_sum_of_leaves_fp32_adjoint_vs_fp64(leaves, want, min_n):
+    """A Sum of two leaves (both kept in registers, in float) and of three (the general way), with one or
+    more of them wanted, against the double adjoint, to the float adjoint's 1e-4 of the largest entry."""
+    rng = np.random.default_rng(17)
+    B = 3
+    gsp = galsim.GSParams(minimum_fft_size=min_n)
+    u = lambda a, b: rng.uniform(a, b, B)
+    parts = [galsim.Sersic(n=u(1.5, 4.), half_light_radius=u(0.3, 0.5), flux=u(100., 300.), gsparams=gsp),
+             galsim.Exponential(half_light_radius=u(0.6, 1.), flux=u(300., 700.), gsparams=gsp),
+             galsim.Gaussian(sigma=u(0.3, 0.5), flux=u(100., 300.), gsparams=gsp)][:leaves]
+    obj = galsim.Convolve(galsim.Add(*[p.shear(g1=u(-0.2, 0.2), g2=u(-0.2, 0.2)) for p in parts]),
+                          galsim.Moffat(beta=3.7, fwhm=0.7, gsparams=gsp), galsim.Pixel(0.2, gsparams=gsp))
+    grads = []
+    for prec, dt in (('fp64', np.float64), ('fp32', np.float32)):
+        plan = autodiff.RecordPlan(obj, 41, 38, 0.2, dtype=dt, precision=prec)
+        img = plan.draw()
+        plan.want = want
+        w = torch.as_tensor(np.random.default_rng(1).standard_normal(tuple(img.shape)), device=img.device, dtype=img.dtype)
+        grads.append(plan.adjoint(w))
+    for k in ('leaf_flux', 'leaf_jac', 'leaf_size', 'leaf_n'):
+        a, b = grads[0][k].cpu().numpy(), grads[1][k].cpu().numpy()
+        assert np.abs(a - b).max() <= 1e-4 * np.abs(a).max(), k
+        for l in range(leaves):
+            assert (want >> l) & 1 or np.all(b[:, l] == 0.)
