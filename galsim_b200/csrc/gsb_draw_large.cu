@@ -70,9 +70,9 @@ struct LargeArgs {
 
 // Float arithmetic drawn into a double image (drawImage's default precision with an ImageD) shows the
 // last bit of every operation, and its users compare such images across versions: it keeps the fused
-// kernels' radix plan.  One object at a time is what is drawn so, and its FFTs are a small part of the
-// call (0.8 ms with either plan at N = 256); in a batch of large stamps block_fft_pass is the faster by far
-// (six stamps of N = 4096 .. 8192: 6.3 ms against 11.7).  PER: radix 2 at N = 8192 has 8 butterflies a
+// kernels' radix plan.  One object at a time is what is drawn so, where the FFTs are little of the call
+// (a 150 x 150 image 0.86 ms); in a batch of large stamps block_fft_pass is the faster by far (six
+// stamps of N = 4096 .. 8192: 6.8 ms against 11.7).  PER: radix 2 at N = 8192 has 8 butterflies a
 // thread.
 template <int THREADS>
 __device__ __noinline__ void block_fft_mixed(float2* buf, int N, const double2* tw)
