@@ -185,12 +185,26 @@ class Program(object):
             self._upload_columns()
         else:
             self._upload_records()
-        self.d_info = torch.empty(self.B * self.L * 2, dtype=torch.float64, device=_lib.Device.torch_device())
+        dev = _lib.Device.torch_device()
+        self.d_info = torch.empty(self.B * self.L * 2, dtype=torch.float64, device=dev)
+        self._uploaded = torch.cuda.current_stream(dev).record_event()
+        self._upload_stream = torch.cuda.current_stream(dev)
         if self.sersic_n is None and not self.image_order and self.moffat_beta is None:
             self.tables = None
         elif getattr(self, 'tables', None) is None:
             self.tables = _lib.TablePool.acquire()
             self._pooled_tables = True
+
+    def _use_uploaded(self):
+        """Order the current stream after the upload, and keep its memory until that stream is done
+        with it: a batch may be planned by one thread and run by another (draw_batches), each on
+        its own current stream, and the expansion of the columns is asynchronous."""
+        import torch
+        cur = torch.cuda.current_stream(_lib.Device.torch_device())
+        if cur != self._upload_stream:
+            cur.wait_event(self._uploaded)
+            self.d_leaves.record_stream(cur)
+            self.d_info.record_stream(cur)
 
     def _upload_columns(self):
         import torch
@@ -319,6 +333,7 @@ class Program(object):
         """FP64 on the GPU: build the Sersic and truncated-Moffat FT tables, then every leaf's
         derived constants, stepk and maxk; copy stepk / maxk back for the host-side composition."""
         self.upload()
+        self._use_uploaded()
         B, L = self.B, self.L
         if self.tables is not None and self.sersic_n is not None:
             self.tables.build_sersic(self.sersic_n, self.gsparams, with_dn=self.need_dn,
@@ -490,6 +505,7 @@ class Program(object):
         into its input buffers first.  The returned buffers are copies."""
         import torch
         self.prepare()
+        self._use_uploaded()
         B = self.B
         dev = _lib.Device.torch_device()
         tdt = torch.float32 if dtype == _lib.F32 else torch.float64
@@ -580,6 +596,7 @@ class Program(object):
         """Evaluate the program on a k grid; returns a host complex array (B, nky, nkx)."""
         import torch
         self.prepare()
+        self._use_uploaded()
         dev = _lib.Device.torch_device()
         tdt = torch.float32 if dtype == _lib.F32 else torch.float64
         out = torch.empty(self.B * nkx * nky * 2, dtype=tdt, device=dev)
