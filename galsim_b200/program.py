@@ -565,25 +565,32 @@ class Program(object):
         grad_sorted = torch.empty((B, ng), dtype=torch.float64, device=dev)
         stream = _lib.Device.stream()
         lib = _lib.lib()
-        # one stream per bucket, largest N first, as the forward (the workspaces are allocated on the
-        # caller's stream before the fork and outlive the join)
-        buckets = sorted(zip(g['starts'], g['ends']), key=lambda se: -int(g['Ns'][se[0]]))
-        works = []
-        for s0, s1 in buckets:
-            wbytes = int(lib.gsb_adjoint_workspace_size(int(g['Ns'][s0]), int(s1 - s0), precision))
-            works.append((wbytes, torch.empty(max(wbytes, 8), dtype=torch.uint8, device=dev) if wbytes else None))
+        # Buckets run side by side, largest N first, as the forward, while their workspaces together stay
+        # within kept bounds; the others (N > 1024 above all, which fill the GPU by themselves) take turns
+        # on the caller's stream with one workspace of the largest's size.  The workspaces are allocated
+        # on the caller's stream before the fork and outlive the join.
+        buckets = [(int(lib.gsb_adjoint_workspace_size(int(g['Ns'][s0]), int(s1 - s0), precision)), s0, s1)
+                   for s0, s1 in zip(g['starts'], g['ends'])]
+        side, turns = adjoint_schedule([w for w, _, _ in buckets], [int(g['Ns'][s0]) for _, s0, _ in buckets])
+        shared = max([buckets[i][0] for i in turns], default=0)
+        shared = torch.empty(shared, dtype=torch.uint8, device=dev) if shared else None
         main = torch.cuda.current_stream(dev)
-        streams = _lib.Device.side_streams(len(buckets)) if len(buckets) > 1 else []
+        streams = _lib.Device.side_streams(len(side))
+        runs = [(i, main, shared) for i in turns]
+        for i, st in zip(side, streams):
+            work = torch.empty(buckets[i][0], dtype=torch.uint8, device=dev) if buckets[i][0] else None
+            runs.append((i, st, work))
         for st in streams:
             st.wait_stream(main)
         try:
-            for (s0, s1), (wbytes, work), st in zip(buckets, works, streams or [main]):
+            for i, st, work in runs:
+                wbytes, s0, s1 = buckets[i]
                 lvp, php, scp, stp = self._bucket_ptrs(g, s0)
                 _lib.check(lib.gsb_adjoint_images(
                     ctypes.byref(self.tpl), int(s1 - s0), ctypes.byref(self.gsp_c), lvp, php, scp, stp,
                     self.tables.handle if self.tables else None, int(g['Ns'][s0]),
                     _lib.ptr(cot), cot_dtype, ctypes.c_void_p(grad_sorted.data_ptr() + int(s0) * ng * 8),
-                    ctypes.c_uint(int(want) & 0xffffffff), precision, _lib.ptr(work),
+                    ctypes.c_uint(int(want) & 0xffffffff), precision, _lib.ptr(work if wbytes else None),
                     ctypes.c_size_t(wbytes), ctypes.c_void_p(st.cuda_stream)))
         finally:
             for st in streams:
@@ -610,6 +617,23 @@ class Program(object):
         a = out.cpu().numpy().reshape(self.B, nky, nkx, 2)
         cdt = np.complex64 if dtype == _lib.F32 else np.complex128
         return (a[..., 0] + 1j * a[..., 1]).astype(cdt)
+
+
+# Bytes of workspaces that adjoint buckets running side by side may hold together.  The fused sizes of a
+# batch of bulge + disk galaxies (N <= 512) need 0.6 GB at most; a bucket of N > 1024 by itself up to 8 GB.
+ADJOINT_SIDE_BYTES = 1 << 30
+
+
+def adjoint_schedule(work_bytes, sizes):
+    """(side, turns): the buckets (by index, largest FFT size first) that run side by side, each with
+    its own workspace, and those that take turns with one workspace.  A single bucket is a turn."""
+    order = sorted(range(len(sizes)), key=lambda i: -sizes[i])
+    side, total = [], 0
+    for i in reversed(order):
+        if sizes[i] <= 1024 and total + work_bytes[i] <= ADJOINT_SIDE_BYTES and len(sizes) > 1:
+            side.append(i)
+            total += work_bytes[i]
+    return side[::-1], [i for i in order if i not in side]
 
 
 # ---- GalSim-exact sizing helpers (gsobject.py:1900-1963) -------------------------------------

@@ -392,3 +392,37 @@ def test_sum_of_leaves_fp32_adjoint_vs_fp64(leaves, want, min_n):
         assert np.abs(a - b).max() <= 1e-4 * np.abs(a).max(), k
         for l in range(leaves):
             assert (want >> l) & 1 or np.all(b[:, l] == 0.)
+
+
+def test_workspace_of_buckets_of_several_sizes():
+    """The adjoint of a batch over several FFT sizes above 1024 holds one bucket's workspace at a time."""
+    from galsim_b200 import _lib
+    sizes = np.repeat([96, 192, 1536, 2048, 3072], 4)
+    B = len(sizes)
+    obj = galsim.Convolve(galsim.Exponential(half_light_radius=np.linspace(0.5, 1., B)), galsim.Moffat(beta=3., fwhm=0.7))
+    prog = galsim.plan_batch(obj, nx=24, ny=20, scale=0.2).prog
+    cot = torch.randn(B, 20, 24, dtype=torch.float32, device='cuda')
+
+    def gradients():
+        prog.draw_stamps(sizes, sizes, -12, -10, 24, 20, _lib.F32)
+        torch.cuda.synchronize()
+        base = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        g = prog.adjoint_stamps(cot.reshape(-1), _lib.F32)
+        torch.cuda.synchronize()
+        return g, torch.cuda.max_memory_allocated() - base
+
+    g, peak = gradients()
+    works = {int(n): _lib.lib().gsb_adjoint_workspace_size(int(n), 4, _lib.F32) for n in np.unique(sizes)}
+    fused = sum(w for n, w in works.items() if n <= 1024)
+    assert peak <= max(works.values()) + fused + (1 << 20)
+    assert sum(works.values()) > 1.5 * peak
+    # the same gradients, one bucket a call
+    for n in np.unique(sizes):
+        i = np.flatnonzero(sizes == n)
+        part = galsim.plan_batch(galsim.Convolve(galsim.Exponential(half_light_radius=np.linspace(0.5, 1., B)[i]),
+                                                 galsim.Moffat(beta=3., fwhm=0.7)), nx=24, ny=20, scale=0.2).prog
+        part.draw_stamps(sizes[i], sizes[i], -12, -10, 24, 20, _lib.F32)
+        ref = part.adjoint_stamps(cot[torch.as_tensor(i, device='cuda')].contiguous().reshape(-1), _lib.F32)
+        # (sums over a stamp's blocks: atomics in another order each time)
+        assert torch.allclose(g[torch.as_tensor(i, device='cuda')], ref, rtol=1e-9, atol=1e-12 * float(ref.abs().max()))

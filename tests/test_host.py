@@ -129,3 +129,17 @@ def test_bench_table_launch_count_follows_the_round_size():
         dlogk = math.sqrt(math.sqrt(1e-6))
         stride = int((math.log(500.) - (math.log(kmin) - 0.001)) / dlogk) + 4
         assert bench.table_build_launches(np.array([n])) == 3 + 2 * ((stride + rnd - 1) // rnd)
+
+
+def test_adjoint_schedule():
+    """Adjoint buckets: side by side within the budget, the others in turn, largest first."""
+    from galsim_b200.program import ADJOINT_SIDE_BYTES as budget, adjoint_schedule
+    assert adjoint_schedule([0], [128]) == ([], [0])
+    assert adjoint_schedule([5], [4096]) == ([], [0])
+    assert adjoint_schedule([0, 10, 20], [96, 128, 512]) == ([2, 1, 0], [])
+    big = 8 << 30
+    side, turns = adjoint_schedule([big, 0, big, 30, big], [2048, 128, 4096, 256, 8192])
+    assert side == [3, 1] and turns == [4, 2, 0]
+    # fused sizes beyond the budget take turns too, the small ones stay side by side
+    side, turns = adjoint_schedule([0, budget // 2, budget // 2 + 1, budget + 1], [96, 256, 512, 1024])
+    assert side == [1, 0] and turns == [3, 2]
