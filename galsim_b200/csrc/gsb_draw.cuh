@@ -84,8 +84,11 @@ struct StampSmem {
     unsigned char scale_sep[GSB_MAX_SCALES];   // scale folded into XS / YS
 };
 
-// Bytes of shared memory reserved for the per-stamp caches.
+// Bytes of shared memory reserved for the per-stamp caches (kCacheBytes; the fused kernels in double at N = 768
+// and 1024, one CTA an SM as it is, hold twice that, so that Nk = N stays factored).
 constexpr int kCacheBytes = 24 * 1024;
+template <typename T>
+__host__ __device__ constexpr int form_budget(int N) { return sizeof(T) == 8 && N >= 768 ? 2 * kCacheBytes : kCacheBytes; }
 
 constexpr size_t kSmemLimit = 227 * 1024;
 
@@ -223,8 +226,6 @@ template <typename T> struct NodeT;
 template <> struct NodeT<float> { using type = float4; };
 template <> struct NodeT<double> { using type = double4; };
 
-// Decide which factors of this stamp are cached in shared memory (thread 0), in order:
-// Sersic spline nodes, phase factors, separable leaf factors, until the budget is used.
 // kAtomSum: a subtree of LEAF and ADD ops only (e.g. bulge + disk), whose cotangent passes
 // unchanged to each of its leaves.
 enum { kAtomRange = 0, kAtomPhase = 1, kAtomScale = 2, kAtomSum = 3 };
@@ -335,10 +336,15 @@ __device__ inline void plan_factored(StampSmem& S, const gsb_template& tpl, cons
 constexpr int kMoffatNodes = 64;
 constexpr double kMoffatTau = 0.25;
 
+// Decide which factors of this stamp are cached in shared memory (thread 0), in order: the folded
+// separable factors, Sersic spline nodes, phase factors, separable leaf factors, per-leaf tables, until
+// the budget is used; image taps in what is left of the room.  What is not cached is evaluated in
+// another form, so kernels that are to give the same bits plan with the same budget (form_budget).
 template <typename T, bool II = true>
 __device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, const FactorPlan& fac, int Nk,
-                                   unsigned want = 0u, int budget = kCacheBytes)
+                                   unsigned want = 0u, int budget = kCacheBytes, int room = 0)
 {
+    room = max(room, budget);
     const int hk = Nk / 2;
     int used = 0;
     S.regstack = fac.depth <= 4;
@@ -361,16 +367,6 @@ __device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, const 
             const int bytes = (S.sersic[l].n * (int)sizeof(typename NodeT<T>::type) + 15) & ~15;
             if (used + bytes <= budget) { S.sersic_cache[l] = used; used += bytes; }
         }
-    }
-    // InterpolatedImage leaves with a diagonal Jacobian: the taps, weights and transform
-    // factor of every column and row (the reference's separable fill caches the same per
-    // column, SBInterpolatedImage.cpp:820-866)
-    for (int l = 0; l < tpl.n_leaves; ++l) {
-        S.ii_cache[l] = -1;
-        const LeafParams& L = S.leaf[l];
-        if (!II || L.type != GSB_INTERPOLATED || (L.flags & GSB_LEAF_JAC_GENERAL)) continue;
-        const int bytes = ((hk + 1 + Nk + 1) * (int)sizeof(IITaps<T>) + 15) & ~15;
-        if (used + bytes <= budget) { S.ii_cache[l] = used; used += bytes; }
     }
     for (int p = 0; p < tpl.n_phases; ++p) {
         S.phase_cache[p] = -1;
@@ -395,6 +391,17 @@ __device__ inline void plan_caches(StampSmem& S, const gsb_template& tpl, const 
             bytes = (S.sersic[l].n * (int)sizeof(float2) + 15) & ~15;
         else continue;
         if (hk < 65535 && used + bytes <= budget) { S.aux_cache[l] = used; used += bytes; }
+    }
+    // InterpolatedImage leaves with a diagonal Jacobian: the taps, weights and transform
+    // factor of every column and row (the reference's separable fill caches the same per
+    // column, SBInterpolatedImage.cpp:820-866).  Kept or not they are the same numbers, so they may
+    // take what room there is.
+    for (int l = 0; l < tpl.n_leaves; ++l) {
+        S.ii_cache[l] = -1;
+        const LeafParams& L = S.leaf[l];
+        if (!II || L.type != GSB_INTERPOLATED || (L.flags & GSB_LEAF_JAC_GENERAL)) continue;
+        const int bytes = ((hk + 1 + Nk + 1) * (int)sizeof(IITaps<T>) + 15) & ~15;
+        if (used + bytes <= room) { S.ii_cache[l] = used; used += bytes; }
     }
 }
 
@@ -659,7 +666,8 @@ __device__ inline T sersic_kvalue_smem(const SersicTableView& tb, const typename
     const T h = T(tb.da);
     const T aa = T(0.5) * log(n1.w / ksq);
     const T bb = h - aa;
-    const T num = aa * n0.y + bb * n1.y - (T(1) / T(6)) * aa * bb * ((aa + h) * n0.z + (bb + h) * n1.z);
+    const T num = mul_add(-((T(1) / T(6)) * aa * bb), mul_add(aa + h, n0.z, mul_rn(bb + h, n1.z)),
+                          mul_add(aa, n0.y, mul_rn(bb, n1.y)));
     return num / h / ksq;
 }
 
@@ -704,7 +712,7 @@ __device__ __forceinline__ void sersic_points(const LeafT<float>& L, const unsig
             p = fmaf(e, p, 0.5f);
             aa = e * p;
         } else {
-            aa = 0.5f * logf(n1.w * inv);
+            aa = mul_rn(0.5f, logf(n1.w * inv));
         }
         const float bb = h - aa;
         const float cub = aa * bb * fmaf(aa + h, n0.z, (bb + h) * n1.z);
@@ -742,9 +750,9 @@ __device__ __forceinline__ void moffat_sum_points(const LeafT<float>& L, const u
     for (int v = 0; v < V; ++v) out[v] = x[v] > 0.f ? sum[v] * exp2f(L.q[0] * log2f(x[v])) : 1.f;
 }
 
-// Real leaf l at the V points (i, j0 + v js) with the shared-memory caches, the leaf's flux included.
+// Real leaf l at the V points (i, j0 + v js) with the shared-memory caches: out[] times the returned factor.
 template <typename T, int V>
-__device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned char* cache, int l, int i, int j0,
+__device__ __forceinline__ T leaf_points(const StampSmem& S, const unsigned char* cache, int l, int i, int j0,
                                             int js, int hk, double dk, T (&out)[V])
 {
     const LeafT<T>& L = leaf_const<T>(S, l);
@@ -759,7 +767,7 @@ __device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned c
 #pragma unroll
             for (int w = 0; w < V; ++w) if (w == v) out[w] = val;
         }
-        return;
+        return T(1);
     }
     const T flux = L.flux;
     if (kind == kLeafSep) {
@@ -767,7 +775,7 @@ __device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned c
         const T x = flux * X[i];
 #pragma unroll
         for (int v = 0; v < V; ++v) out[v] = x * X[hk + 1 + hk + j0 + v * js];
-        return;
+        return T(1);
     }
     const T jf = T(j0), jd = T(js);
     if constexpr (sizeof(T) == 8) {
@@ -775,11 +783,12 @@ __device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned c
         if (kind == kLeafSersic) {
 #pragma unroll
             for (int v = 0; v < V; ++v) {
-                const T j = jf + T(v) * jd, u = L.a * T(i) + L.c * j, w = L.b * T(i) + L.d * j;
+                const T j = jf + T(v) * jd, u = mul_add(L.c, j, mul_rn(L.a, T(i))), w = mul_add(L.d, j, mul_rn(L.b, T(i)));
                 out[v] = flux * sersic_kvalue_smem<T>(
-                                    S.sersic[l], reinterpret_cast<const typename NodeT<T>::type*>(cache + L.cache), u * u + w * w);
+                                    S.sersic[l], reinterpret_cast<const typename NodeT<T>::type*>(cache + L.cache),
+                                    mul_add(u, u, mul_rn(w, w)));
             }
-            return;
+            return T(1);
         }
     }
     if (kind == kLeafExp) {
@@ -791,23 +800,22 @@ __device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned c
         for (int v = 0; v < V; ++v) {
             const ushort2 r = R[v * js];
             const T ky = (jf + T(v) * jd) * tdk;
-            const T u = A * kx + C * ky;
-            const T w = B * kx + D * ky;
-            const T q = T(1) + (u * u + w * w) * r0 * r0;
+            const T u = mul_add(A, kx, mul_rn(C, ky)), w = mul_add(B, kx, mul_rn(D, ky));
+            const T q = mul_add(mul_add(u, u, mul_rn(w, w)) * r0, r0, T(1));
             const T val = flux / (q * sqrt(q));
             out[v] = i >= int(r.x) && i < int(r.y) ? val : T(0);
         }
-        return;
+        return T(1);
     }
     if constexpr (sizeof(T) == 4) {
         float ksq[V];
         {
-            const float ui = L.a * float(i), wi = L.b * float(i), c = L.c, d = L.d;
+            const float ui = mul_rn(L.a, float(i)), wi = mul_rn(L.b, float(i)), c = L.c, d = L.d;
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 const float j = jf + float(v) * jd;
-                const float u = ui + c * j, w = wi + d * j;
-                ksq[v] = u * u + w * w;
+                const float u = mul_add(c, j, ui), w = mul_add(d, j, wi);
+                ksq[v] = mul_add(u, u, mul_rn(w, w));
             }
         }
         if (kind == kLeafSersic) {
@@ -847,9 +855,8 @@ __device__ __forceinline__ void leaf_points(const StampSmem& S, const unsigned c
                 out[v] = expf(-k) * (1.f + k * (c1 + k * c2));
             }
         }
-#pragma unroll
-        for (int v = 0; v < V; ++v) out[v] *= flux;
     }
+    return flux;
 }
 
 // One leaf at k index (i, j) with the shared-memory caches.
@@ -858,8 +865,8 @@ __device__ __noinline__ T leaf_fast(const StampSmem& S, const unsigned char* cac
                                     double dk)
 {
     T out[1];
-    leaf_points<T, 1>(S, cache, arg, i, j, 0, hk, dk, out);
-    return out[0];
+    const T f = leaf_points<T, 1>(S, cache, arg, i, j, 0, hk, dk, out);
+    return mul_rn(out[0], f);
 }
 
 // One leaf as a complex value: InterpolatedImage leaves are complex, the others real.  INL: compiled
@@ -878,8 +885,8 @@ __device__ __forceinline__ Cx<T> leaf_cfast(const StampSmem& S, const unsigned c
     }
     if constexpr (INL) {
         T out[1];
-        leaf_points<T, 1>(S, cache, arg, i, j, 0, g.n / 2, g.dk, out);
-        return cx<T>(out[0], T(0));
+        const T f = leaf_points<T, 1>(S, cache, arg, i, j, 0, g.n / 2, g.dk, out);
+        return cx<T>(mul_rn(out[0], f), T(0));
     }
     return cx<T>(leaf_fast<T>(S, cache, arg, i, j, g.n / 2, g.dk), T(0));
 }
@@ -903,16 +910,16 @@ __device__ __noinline__ Cx<T> eval_range(const gsb_template& tpl, const StampSme
         } else if (code == GSB_OP_MUL || code == GSB_OP_ADD) {
             --sp;
             const bool mul = code == GSB_OP_MUL;
-            if (sp == 1) s0 = mul ? cmul<T>(s0, s1) : cadd<T>(s0, s1);
-            else if (sp == 2) s1 = mul ? cmul<T>(s1, s2) : cadd<T>(s1, s2);
-            else s2 = mul ? cmul<T>(s2, s3) : cadd<T>(s2, s3);
+            if (sp == 1) s0 = mul ? cmul_yx<T>(s0, s1) : cadd<T>(s0, s1);
+            else if (sp == 2) s1 = mul ? cmul_yx<T>(s1, s2) : cadd<T>(s1, s2);
+            else s2 = mul ? cmul_yx<T>(s2, s3) : cadd<T>(s2, s3);
         } else {
             Cx<T> f;
             if (code == GSB_OP_PHASE) {
                 const T fs = T(S.phase[arg].flux_scaling);
                 if (S.phase_cache[arg] >= 0) {
                     const Cx<T>* PX = reinterpret_cast<const Cx<T>*>(cache + S.phase_cache[arg]);
-                    f = cscale<T>(cmul<T>(PX[i], PX[hk + 1 + j + hk]), fs);
+                    f = cscale<T>(cmul_yx<T>(PX[i], PX[hk + 1 + j + hk]), fs);
                 } else {
                     double tt = i * S.phase_ax[arg] + j * S.phase_ay[arg];
                     tt -= rint(tt);
@@ -923,10 +930,10 @@ __device__ __noinline__ Cx<T> eval_range(const gsb_template& tpl, const StampSme
             } else {
                 f = cx<T>(T(S.scale[arg]), T(0));
             }
-            if (sp == 1) s0 = cmul<T>(s0, f);
-            else if (sp == 2) s1 = cmul<T>(s1, f);
-            else if (sp == 3) s2 = cmul<T>(s2, f);
-            else s3 = cmul<T>(s3, f);
+            if (sp == 1) s0 = cmul_yx<T>(s0, f);
+            else if (sp == 2) s1 = cmul_yx<T>(s1, f);
+            else if (sp == 3) s2 = cmul_yx<T>(s2, f);
+            else s3 = cmul_yx<T>(s3, f);
         }
     }
     return s0;
@@ -934,16 +941,14 @@ __device__ __noinline__ Cx<T> eval_range(const gsb_template& tpl, const StampSme
 
 // The factored program at the V points (i, j0 + v js): the folded separable factors XS[i] YS[j + hk]
 // times the atoms.  Taking V points through each atom at a time shares the program's control flow
-// and the atoms' constants, and gives the latencies V independent chains to overlap.  (A function
-// call per V points, so that the kernels of all sizes share one compiled body.)
-template <typename T, int V> struct Values { Cx<T> v[V]; };
+// and the atoms' constants, and gives the latencies V independent chains to overlap.  The value of point v is
+// handed to fold(v, z, r) as a complex z and a real factor r, which the fold multiplies in (kahan_add).
+template <typename T, int V> struct Values { Cx<T> v[V]; T r[V]; };
 
-template <typename T, bool II, int V>
-__device__ __forceinline__ Values<T, V> eval_points_inline(const gsb_template& tpl, const StampSmem& S,
-                                                           const unsigned char* cache, int i, int j0, int js, int hk,
-                                                           double dk)
+template <typename T, bool II, int V, class Fold>
+__device__ __forceinline__ void eval_points_fold(const gsb_template& tpl, const StampSmem& S, const unsigned char* cache,
+                                                 int i, int j0, int js, int hk, double dk, const Fold& fold)
 {
-    Values<T, V> res;
     T r[V], sum[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) { r[v] = T(1); sum[v] = T(0); }
@@ -951,11 +956,11 @@ __device__ __forceinline__ Values<T, V> eval_points_inline(const gsb_template& t
 #pragma unroll 1
     for (int q = 0; q < nr; ++q) {
         T t[V];
-        leaf_points<T, V>(S, cache, S.real_leaf[q], i, j0, js, hk, dk, t);
+        const T f = leaf_points<T, V>(S, cache, S.real_leaf[q], i, j0, js, hk, dk, t);
         const bool last = S.real_last[q];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            sum[v] += t[v];
+            sum[v] = mul_add(t[v], f, sum[v]);
             if (last) { r[v] *= sum[v]; sum[v] = T(0); }
         }
     }
@@ -965,8 +970,8 @@ __device__ __forceinline__ Values<T, V> eval_points_inline(const gsb_template& t
     const int no = S.n_other;
     if (no == 0) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) res.v[v] = cscale<T>(cmul<T>(x, YS[v * js]), r[v]);
-        return res;
+        for (int v = 0; v < V; ++v) fold(v, cmul_yx<T>(x, YS[v * js]), r[v]);
+        return;
     }
     const GridRef g{dk, 0, -hk, hk + 1, 2 * hk + 1};
 #pragma unroll 1
@@ -978,55 +983,63 @@ __device__ __forceinline__ Values<T, V> eval_points_inline(const gsb_template& t
             c = cmul<T>(c, o1 - o0 == 1 ? leaf_cfast<T, II>(S, cache, S.atom_arg[a], i, j, g)
                                         : eval_range<T, II>(tpl, S, cache, dk, i, j, g, o0, o1));
         }
-        T rv = r[0];
+        const Cx<T> z = cmul<T>(c, cmul_yx<T>(x, YS[v * js]));
 #pragma unroll
-        for (int w = 1; w < V; ++w) if (w == v) rv = r[w];
-        const Cx<T> z = cscale<T>(cmul<T>(c, cmul<T>(x, YS[v * js])), rv);
-#pragma unroll
-        for (int w = 0; w < V; ++w) if (w == v) res.v[w] = z;
+        for (int w = 0; w < V; ++w) if (w == v) fold(w, z, r[w]);
     }
-    return res;
 }
 
 template <typename T, bool II, int V>
 __device__ __noinline__ Values<T, V> eval_points(const gsb_template& tpl, const StampSmem& S,
                                                  const unsigned char* cache, int i, int j0, int js, int hk, double dk)
 {
-    return eval_points_inline<T, II, V>(tpl, S, cache, i, j0, js, hk, dk);
+    Values<T, V> res;
+    eval_points_fold<T, II, V>(tpl, S, cache, i, j0, js, hk, dk, [&](int v, Cx<T> z, T r) { res.v[v] = z; res.r[v] = r; });
+    return res;
 }
 
-// V points of the program, by the best of its three forms.  INL: compiled into the caller.
-template <typename T, bool II, int V, bool INL = false>
-__device__ __forceinline__ Values<T, V> eval_any(const gsb_template& tpl, const StampSmem& S,
-                                                 const unsigned char* cache, int i, int j0, int js, int hk, double dk)
+// V points of the program to fold(v, z, r), by the best of its three forms.  INL: compiled into the caller
+// (else a function call per V points, so that the kernels of all sizes share one compiled body).
+template <typename T, bool II, int V, bool INL, class Fold>
+__device__ __forceinline__ void eval_any(const gsb_template& tpl, const StampSmem& S, const unsigned char* cache, int i,
+                                         int j0, int js, int hk, double dk, const Fold& fold)
 {
-    if (S.xy_cache >= 0)
-        return INL ? eval_points_inline<T, II, V>(tpl, S, cache, i, j0, js, hk, dk)
-                   : eval_points<T, II, V>(tpl, S, cache, i, j0, js, hk, dk);
+    if (S.xy_cache >= 0) {
+        if constexpr (INL) {
+            eval_points_fold<T, II, V>(tpl, S, cache, i, j0, js, hk, dk, fold);
+        } else {
+            const Values<T, V> z = eval_points<T, II, V>(tpl, S, cache, i, j0, js, hk, dk);
+#pragma unroll
+            for (int v = 0; v < V; ++v) fold(v, z.v[v], z.r[v]);
+        }
+        return;
+    }
     const GridRef g{dk, 0, -hk, hk + 1, 2 * hk + 1};
-    Values<T, V> res;
 #pragma unroll 1
     for (int v = 0; v < V; ++v) {
         const Cx<T> z = S.regstack ? eval_range<T, II>(tpl, S, cache, dk, i, j0 + v * js, g, 0, tpl.n_ops)
                                    : eval_program<T, II>(tpl, S, dk, i, j0 + v * js, g);
 #pragma unroll
-        for (int w = 0; w < V; ++w) if (w == v) res.v[w] = z;
+        for (int w = 0; w < V; ++w) if (w == v) fold(w, z, T(1));
     }
-    return res;
 }
 
 template <typename T, bool II, bool INL = false>
-__device__ __forceinline__ Cx<T> eval_point(const gsb_template& tpl, const StampSmem& S, const unsigned char* cache,
+__device__ __forceinline__ Values<T, 1> eval_point(const gsb_template& tpl, const StampSmem& S, const unsigned char* cache,
                                             int i, int j, int hk, double dk)
 {
-    return eval_any<T, II, 1, INL>(tpl, S, cache, i, j, 0, hk, dk).v[0];
+    Values<T, 1> res;
+    eval_any<T, II, 1, INL>(tpl, S, cache, i, j, 0, hk, dk, [&](int, Cx<T> z, T r) { res.v[0] = z; res.r[0] = r; });
+    return res;
 }
 
-// acc += v with Kahan's compensation term comp (componentwise).
+// acc += v r (conjugated where not pos) with Kahan's compensation term comp, componentwise.  The real
+// part's product is not rounded before the compensation is taken off; the imaginary part's is.
 template <typename T>
-__device__ __forceinline__ void kahan_add(Cx<T>& acc, Cx<T>& comp, Cx<T> v)
+__device__ __forceinline__ void kahan_add(Cx<T>& acc, Cx<T>& comp, Cx<T> v, T r, bool pos)
 {
-    const T yx = v.x - comp.x, yy = v.y - comp.y;
+    const T vy = mul_rn(v.y, r);
+    const T yx = mul_add(v.x, r, -comp.x), yy = add_rn(pos ? vy : -vy, -comp.y);
     const T tx = acc.x + yx, ty = acc.y + yy;
     comp.x = (tx - acc.x) - yx;
     comp.y = (ty - acc.y) - yy;
@@ -1052,7 +1065,7 @@ constexpr size_t smem_bytes(bool wsmem)
     size_t off = (sizeof(StampSmem) + 15) & ~size_t(15);
     off += sizeof(Cx<T>) * N * (1 + fused_warps<T, N>());
     if (wsmem) off += sizeof(Cx<T>) * (N / 2 + 1) * (N + 1);
-    return ((off + 15) & ~size_t(15)) + kCacheBytes;
+    return ((off + 15) & ~size_t(15)) + form_budget<T>(N);
 }
 
 template <typename T, int N>
@@ -1112,7 +1125,7 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
         __syncthreads();
         const int Nk = S.geom.Nk;
         const int hk = Nk / 2;
-        if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk);
+        if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, 0u, form_budget<T>(N));
         __syncthreads();
         fill_caches<T, II>(S, a.tpl, cache, dk, Nk, sizeof(T) == 4 && a.out_dtype == GSB_F64);
         __syncthreads();
@@ -1123,68 +1136,67 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
             // of 32, so slots s, s + N/32, ... of a lane are the aliases of one wrapped row: the lane
             // folds them (with Kahan compensation) in registers, and a column costs
             // ceil((Nk + 1) / 32) slots.  When Nk is a multiple of 32 (Nk = N above all) the last slot
-            // would hold the single point ky = hk: those points of all the warp's columns are taken
-            // together, one column a lane, before its columns.
+            // would hold the single point ky = hk: up to Nk = N, where a column has one alias in kx (but for
+            // c = N / 2, which has a slot for them), those points of all the warp's columns are taken
+            // together, one column a lane, before its columns, and folded in their turn.
             constexpr int NS = N / 32;
             constexpr int V = sizeof(T) == 8 ? (NS % 2 == 0 ? 2 : 1) : NS % 4 == 0 ? 4 : NS % 3 == 0 ? 3 : NS;
             constexpr int COLS = (H + NW - 1) / NW;
-            const bool edge = COLS <= 32 && Nk % 32 == 0;
-            const int top = edge ? hk - 1 : hk;
-            const int edge_slot = edge ? (Nk % N) / 32 : -1;
+            const bool edge = COLS <= 32 && Nk % 32 == 0 && Nk <= N;
             Cx<T> edge_val = cx<T>(T(0), T(0));
             if (edge) {
                 const int c = warp + lane * NW;
-                if (c < H) {
-                    for (int kx = c + ceil_div(-hk - c, N) * N; kx <= hk; kx += N) {
-                        const Cx<T> v = eval_point<T, II>(a.tpl, S, cache, kx >= 0 ? kx : -kx, kx >= 0 ? hk : -hk, hk, dk);
-                        edge_val = cadd<T>(edge_val, kx >= 0 ? v : cconj<T>(v));
-                    }
+                if (c <= hk && c + c < N) {
+                    const Values<T, 1> z = eval_point<T, II>(a.tpl, S, cache, c, hk, hk, dk);
+                    edge_val = cscale<T>(z.v[0], z.r[0]);
                 }
                 __syncwarp();
             }
             int q = 0;
             for (int c = warp; c < H; c += NW, ++q) {
                 const int kx0 = c + ceil_div(-hk - c, N) * N;
+                const bool has_edge = edge && c <= hk && c + c < N;
+                const int top = has_edge ? hk - 1 : hk;
+                const int edge_slot = has_edge ? (Nk % N) / 32 : -1;
                 for (int s0 = 0; s0 < NS; s0 += V) {
                     Cx<T> acc[V], comp[V];
 #pragma unroll
                     for (int v = 0; v < V; ++v) acc[v] = comp[v] = cx<T>(T(0), T(0));
-                    if (edge && edge_slot >= s0 && edge_slot < s0 + V) {
-                        const Cx<T> e = cx<T>(__shfl_sync(0xffffffffu, edge_val.x, q), __shfl_sync(0xffffffffu, edge_val.y, q));
-#pragma unroll
-                        for (int v = 0; v < V; ++v)
-                            if (lane == 0 && s0 + v == edge_slot) acc[v] = e;
-                    }
-                    // a lane's first value needs no compensation
-                    bool first = !(edge && edge_slot >= s0 && edge_slot < s0 + V);
+                    bool first = true;       // a lane's first value needs no compensation
                     for (int kx = kx0; kx <= hk; kx += N) {
                         const bool pos = kx >= 0;
                         const int ii = pos ? kx : -kx;
                         for (int e0 = -hk + 32 * s0; e0 <= top; e0 += N) {
                             if (e0 + 32 * V - 1 <= top) {
                                 const int ky = e0 + lane;
-                                const Values<T, V> z = eval_any<T, II, V, !II && sizeof(T) == 4>(a.tpl, S, cache, ii, pos ? ky : -ky,
-                                                                                        pos ? 32 : -32, hk, dk);
-#pragma unroll
-                                for (int v = 0; v < V; ++v) {
-                                    const Cx<T> w = pos ? z.v[v] : cconj<T>(z.v[v]);
-                                    if (first) acc[v] = w;
-                                    else kahan_add<T>(acc[v], comp[v], w);
-                                }
+                                eval_any<T, II, V, !II && sizeof(T) == 4>(
+                                    a.tpl, S, cache, ii, pos ? ky : -ky, pos ? 32 : -32, hk, dk, [&](int v, Cx<T> z, T r) {
+                                        if (first) {
+                                            acc[v] = cscale<T>(z, r);
+                                            if (!pos) acc[v].y = -acc[v].y;
+                                        } else {
+                                            kahan_add<T>(acc[v], comp[v], z, r, pos);
+                                        }
+                                    });
                                 first = false;
                             } else {
                                 // the last, partial slots of the column (lanes beyond it repeat its end)
 #pragma unroll 1
                                 for (int u = 0; u < V && e0 + 32 * u <= top; ++u) {
                                     const int ky = e0 + 32 * u + lane, kc = min(ky, top);
-                                    Cx<T> z = eval_point<T, II>(a.tpl, S, cache, ii, pos ? kc : -kc, hk, dk);
-                                    if (!pos) z = cconj<T>(z);
-                                    if (ky > top) z = cx<T>(T(0), T(0));
+                                    const Values<T, 1> z = eval_point<T, II>(a.tpl, S, cache, ii, pos ? kc : -kc, hk, dk);
 #pragma unroll
                                     for (int v = 0; v < V; ++v)
-                                        if (v == u) kahan_add<T>(acc[v], comp[v], z);
+                                        if (v == u && ky <= top) kahan_add<T>(acc[v], comp[v], z.v[0], z.r[0], pos);
                                 }
+                                first = false;
                             }
+                        }
+                        if (edge_slot >= s0 && edge_slot < s0 + V) {
+                            const Cx<T> e = cx<T>(__shfl_sync(0xffffffffu, edge_val.x, q), __shfl_sync(0xffffffffu, edge_val.y, q));
+#pragma unroll
+                            for (int v = 0; v < V; ++v)
+                                if (lane == 0 && s0 + v == edge_slot) kahan_add<T>(acc[v], comp[v], e, T(1), true);
                         }
                     }
 #pragma unroll
@@ -1205,8 +1217,8 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
                     for (int kx = kx0; kx <= hk; kx += N) {
                         const bool pos = kx >= 0;
                         for (int ky = kyc + ceil_div(-hk - kyc, N) * N; ky <= hk; ky += N) {
-                            const Cx<T> v = eval_point<T, II>(a.tpl, S, cache, pos ? kx : -kx, pos ? ky : -ky, hk, dk);
-                            kahan_add<T>(acc, comp, pos ? v : cconj<T>(v));
+                            const Values<T, 1> z = eval_point<T, II>(a.tpl, S, cache, pos ? kx : -kx, pos ? ky : -ky, hk, dk);
+                            kahan_add<T>(acc, comp, z.v[0], z.r[0], pos);
                         }
                     }
                     buf[fft_slot(r)] = acc;

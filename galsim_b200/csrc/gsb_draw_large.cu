@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) large_col_ker
                a.sersic_stride, 1. / N);
     __syncthreads();
     const int Nk = S.geom.Nk, hk = Nk / 2;
-    if (threadIdx.x == 0) plan_caches<T, II>(S, a.tpl, a.fac, Nk, 0u, la.cache_bytes);
+    if (threadIdx.x == 0)
+        plan_caches<T, II>(S, a.tpl, a.fac, Nk, 0u, N <= 1024 ? form_budget<T>(N) : la.cache_bytes, la.cache_bytes);
     __syncthreads();
     fill_caches<T, II>(S, a.tpl, cache, dk, Nk, sizeof(T) == 4 && a.out_dtype == GSB_F64);
     __syncthreads();
@@ -120,19 +121,18 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) large_col_ker
                     for (int e0 = -hk + THREADS * s0; e0 <= hk; e0 += N) {
                         const int ky = e0 + int(threadIdx.x);
                         if (nv == V && e0 + THREADS * V - 1 <= hk) {
-                            const Values<T, V> z = eval_any<T, II, V>(a.tpl, S, cache, ii, pos ? ky : -ky,
-                                                                      pos ? THREADS : -THREADS, hk, dk);
-#pragma unroll
-                            for (int v = 0; v < V; ++v) kahan_add<T>(acc[v], comp[v], pos ? z.v[v] : cconj<T>(z.v[v]));
+                            eval_any<T, II, V, false>(
+                                a.tpl, S, cache, ii, pos ? ky : -ky, pos ? THREADS : -THREADS, hk, dk,
+                                [&](int v, Cx<T> z, T r) { kahan_add<T>(acc[v], comp[v], z, r, pos); });
                         } else {
 #pragma unroll 1
                             for (int u = 0; u < nv; ++u) {
                                 const int ku = ky + THREADS * u;
                                 if (ku > hk) break;
-                                const Cx<T> z = eval_point<T, II>(a.tpl, S, cache, ii, pos ? ku : -ku, hk, dk);
+                                const Values<T, 1> z = eval_point<T, II>(a.tpl, S, cache, ii, pos ? ku : -ku, hk, dk);
 #pragma unroll
                                 for (int v = 0; v < V; ++v)
-                                    if (v == u) kahan_add<T>(acc[v], comp[v], pos ? z : cconj<T>(z));
+                                    if (v == u) kahan_add<T>(acc[v], comp[v], z.v[0], z.r[0], pos);
                             }
                         }
                     }
@@ -150,15 +150,15 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) large_col_ker
                 for (int kx = kx0; kx <= hk; kx += N) {
                     const bool pos = kx >= 0;
                     for (int ky = kyc + ceil_div(-hk - kyc, N) * N; ky <= hk; ky += N) {
-                        const Cx<T> v = eval_point<T, II, sizeof(T) == 8>(a.tpl, S, cache, pos ? kx : -kx, pos ? ky : -ky, hk, dk);
-                        kahan_add<T>(acc, comp, pos ? v : cconj<T>(v));
+                        const Values<T, 1> z = eval_point<T, II, sizeof(T) == 8>(a.tpl, S, cache, pos ? kx : -kx, pos ? ky : -ky, hk, dk);
+                        kahan_add<T>(acc, comp, z.v[0], z.r[0], pos);
                     }
                 }
                 buf[r] = acc;
             }
         }
         __syncthreads();
-        if (sizeof(T) == 4 && a.out_dtype == GSB_F64) {
+        if (sizeof(T) == 4 && a.out_dtype == GSB_F64 && N > 1024) {
             block_fft_mixed<THREADS>(buf, N, la.tw);
             for (int r = threadIdx.x; r < N; r += blockDim.x) W[(size_t)c * N + r] = buf[r];
             __syncthreads();
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(row_threads(N)) large_row_kernel(const __grid_
                 }
             }
         };
-        if (sizeof(T) == 4 && a.out_dtype == GSB_F64) {
+        if (sizeof(T) == 4 && N > 1024 && a.out_dtype == GSB_F64) {
             for (int kx = threadIdx.x; kx < N; kx += THREADS) buf[kx] = load(kx);
             __syncthreads();
             block_fft_mixed<THREADS>(buf, N, la.tw);
@@ -297,10 +297,12 @@ int launch_large_t(const DrawArgs& args, int N, void* work, size_t work_bytes, c
     const size_t base = large_smem<T>() + sizeof(Cx<T>) * ((fft_buf_len<T>(N) + 1) & ~size_t(1));
     if (base > kSmemLimit) return set_error(GSB_ERR_UNSUPPORTED, "FFT size too large for this precision");
     // the rest of shared memory (up to 192 KB) holds the per-stamp caches of the column kernel; for
-    // N <= 1024 as much as two CTAs an SM leave (axis tables of up to Nk = 5 N and the Sersic nodes)
+    // N <= 1024 as much as two CTAs an SM leave (the fused kernels' budget, and image taps)
     const size_t room = kSmemLimit - base > 1024 ? kSmemLimit - base - 1024 : 0;
     const size_t want = THREADS == 256 ? std::min<size_t>(28 * 1024 + 64 * sizeof(T) / 4 * N, 112 * 1024 - base)
                                        : size_t(192) * 1024;
+    if (THREADS == 256 && std::min(room, want) < size_t(form_budget<T>(N)))
+        return set_error(GSB_ERR_UNSUPPORTED, "FFT size too large for this precision");
     const int cache_bytes = int(std::min<size_t>(room, want) & ~size_t(15));
     const size_t sm = base + cache_bytes;
     const double2* tw = nullptr;

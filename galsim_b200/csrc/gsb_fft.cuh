@@ -22,8 +22,20 @@ template <typename T> using Cx = typename CxT<T>::type;
 template <typename T> __device__ __forceinline__ Cx<T> cx(T x, T y) { Cx<T> r; r.x = x; r.y = y; return r; }
 template <typename T> __device__ __forceinline__ Cx<T> cadd(Cx<T> a, Cx<T> b) { return cx<T>(a.x + b.x, a.y + b.y); }
 template <typename T> __device__ __forceinline__ Cx<T> csub(Cx<T> a, Cx<T> b) { return cx<T>(a.x - b.x, a.y - b.y); }
+// Multiply-adds and additions whose rounding is stated rather than left to the compiler, which contracts
+// a sum of products by its surroundings: what the fused and the split draw kernels share gives the same
+// bits in both.
+__device__ __forceinline__ float mul_add(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double mul_add(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 template <typename T> __device__ __forceinline__ Cx<T> cmul(Cx<T> a, Cx<T> b)
-{ return cx<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+{ return cx<T>(mul_add(a.x, b.x, -mul_rn(a.y, b.y)), mul_add(a.x, b.y, mul_rn(a.y, b.x))); }
+// The same with the imaginary part's other product rounded (the k-space products of the program).
+template <typename T> __device__ __forceinline__ Cx<T> cmul_yx(Cx<T> a, Cx<T> b)
+{ return cx<T>(mul_add(a.x, b.x, -mul_rn(a.y, b.y)), mul_add(a.y, b.x, mul_rn(a.x, b.y))); }
 template <typename T> __device__ __forceinline__ Cx<T> cconj(Cx<T> a) { return cx<T>(a.x, -a.y); }
 template <typename T> __device__ __forceinline__ Cx<T> cscale(Cx<T> a, T s) { return cx<T>(a.x * s, a.y * s); }
 // multiply by SIGN * i
@@ -152,7 +164,8 @@ __device__ inline void fill_twiddles(Cx<T>* tw, int N)
 
 // Block-wide length-N DFT (N = 2^a or 3 * 2^a) in shared memory, Stockham order, N and the thread
 // count known at compile time so that every index is a shift or a constant: radix 8 (4 and 2 for the
-// rest of the power of two), the factor 3 last.  The first pass takes its inputs from load(i) and
+// rest of the power of two), the factor 3 last.  Up to N = 1024, where a bucket may also run the fused
+// kernel, warp_fft_io's radix plan and twiddles, so that both give the same bits.  The first pass takes its inputs from load(i) and
 // the last hands its outputs to store(i, value), so that a caller can read from or write to memory
 // without a trip through the buffer.  tw: exp(+2 pi i m / N), m < N, in T (global).  A radix-8
 // butterfly reads all seven twiddles: three read and the others multiplied from them are 8 % faster
@@ -175,7 +188,8 @@ __device__ __forceinline__ void block_fft_pass(Cx<T>* buf, const Cx<T>* __restri
 {
     constexpr int REM = N / NS;
     constexpr int P2 = REM % 3 == 0 ? REM / 3 : REM;      // what is left of the power of two
-    constexpr int R = P2 == 1 ? 3 : P2 == 2 ? 2 : (P2 == 4 || P2 == 16) ? 4 : 8;
+    constexpr int R = N <= 1024 ? (NS == 1 && N % 3 == 0 ? 3 : REM % 4 == 0 ? 4 : 2)
+                                : P2 == 1 ? 3 : P2 == 2 ? 2 : (P2 == 4 || P2 == 16) ? 4 : 8;
     constexpr int NB = N / R;
     constexpr int PER = (NB + THREADS - 1) / THREADS;
     constexpr int TSTEP = N / (NS * R);
@@ -249,7 +263,7 @@ __device__ __forceinline__ void block_fft_any(Cx<T>* buf, int N, const Cx<T>* __
             else block_fft_n<T, M, THREADS>(buf, tw);
         }
     };
-    if constexpr (THREADS <= 512) {
+    if constexpr (THREADS == 256) {
         switch (N) {
           case 192: run(std::integral_constant<int, 192>{}); return;
           case 256: run(std::integral_constant<int, 256>{}); return;

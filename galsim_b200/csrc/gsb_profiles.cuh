@@ -118,8 +118,8 @@ __device__ inline T sersic_kvalue(const SersicTableView& tb, T ksq)
         const T h = T(tb.da);
         const T aa = T(0.5) * log(T(n1.w) / ksq);
         const T bb = h - aa;
-        const T f = (aa * T(n0.y) + bb * T(n1.y) -
-                     (T(1) / T(6)) * aa * bb * ((aa + h) * T(n0.z) + (bb + h) * T(n1.z))) / h;
+        const T f = mul_add(-((T(1) / T(6)) * aa * bb), mul_add(aa + h, T(n0.z), mul_rn(bb + h, T(n1.z))),
+                            mul_add(aa, T(n0.y), mul_rn(bb, T(n1.y)))) / h;
         return f / ksq;
     }
 }
@@ -198,8 +198,9 @@ __device__ inline T leaf_kvalue(const LeafParams& L, const SersicTableView* tabl
                                 const GridRef& g, int gi, int gj)
 {
     const T A = T(L.jac[0]), B = T(L.jac[1]), C = T(L.jac[2]), D = T(L.jac[3]);
-    const T kxp = A * kx + C * ky;
-    const T kyp = B * kx + D * ky;
+    const T kxp = mul_add(A, kx, mul_rn(C, ky));
+    const T kyp = mul_add(B, kx, mul_rn(D, ky));
+    const T kk = mul_add(kxp, kxp, mul_rn(kyp, kyp));
     const T flux = T(L.flux);
     switch (L.type) {
       case GSB_GAUSSIAN: {
@@ -209,7 +210,7 @@ __device__ inline T leaf_kvalue(const LeafParams& L, const SersicTableView* tabl
             const T ax = kxp * s, ay = kyp * s;
             return flux * exp(T(-0.5) * ax * ax) * exp(T(-0.5) * ay * ay);
         }
-        const T ksq = (kxp * kxp + kyp * kyp) * s * s;
+        const T ksq = kk * s * s;
         if (ksq > T(L.d[1])) return T(0);
         if (ksq < T(L.d[2])) return flux * (T(1) - T(0.5) * ksq * (T(1) - T(0.25) * ksq));
         return flux * exp(T(-0.5) * ksq);
@@ -217,12 +218,12 @@ __device__ inline T leaf_kvalue(const LeafParams& L, const SersicTableView* tabl
       case GSB_EXPONENTIAL: {
         if (!exponential_keep(L, g.dk, g.x0, g.y0, g.m, g.n, gi, gj)) return T(0);
         const T r0 = T(L.d[0]);
-        const T ksqp1 = T(1) + (kxp * kxp + kyp * kyp) * r0 * r0;
+        const T ksqp1 = mul_add(kk * r0, r0, T(1));
         return flux / (ksqp1 * sqrt(ksqp1));
       }
       case GSB_SERSIC: {
         const T r0 = T(L.d[0]);
-        const T ksq = (kxp * kxp + kyp * kyp) * r0 * r0;
+        const T ksq = kk * r0 * r0;
         return flux * sersic_kvalue<T>(tables[L.table], ksq);
       }
       case GSB_MOFFAT: {
@@ -232,9 +233,9 @@ __device__ inline T leaf_kvalue(const LeafParams& L, const SersicTableView* tabl
         if (mode == 4) {
             const double4* nd = reinterpret_cast<const double4*>(__double_as_longlong(L.d[6]));
             return knorm * moffat_trunc_kvalue<T>(nd, int(L.d[5]), T(L.d[3]), T(L.d[4]),
-                                                  (kxp * kxp + kyp * kyp) * rD * rD);
+                                                  kk * rD * rD);
         }
-        const T k = sqrt(kxp * kxp + kyp * kyp) * rD;
+        const T k = sqrt(kk) * rD;
         if (mode == 1) return knorm * exp(-k);
         if (mode == 2) return knorm * exp(-k) * (T(1) + k);
         if (mode == 3) return knorm * exp(-k) * (T(3) + (T(3) + k) * k) * T(1. / 3.);
@@ -242,14 +243,14 @@ __device__ inline T leaf_kvalue(const LeafParams& L, const SersicTableView* tabl
       }
       case GSB_KOLMOGOROV: {
         const T ik0 = T(L.d[0]);
-        const T ksq = (kxp * kxp + kyp * kyp) * ik0 * ik0;
+        const T ksq = kk * ik0 * ik0;
         return flux * exp(-kolm_pow56<T>(ksq));
       }
       case GSB_AIRY: {
         const T s = T(L.d[0]);       // 1 / (D pi)
         const T knorm = T(L.d[1]);
         const T obs = T(L.d[2]), obssq = T(L.d[3]);
-        const T t = (kxp * kxp + kyp * kyp) * s * s;   // ksq / (pi D)^2
+        const T t = kk * s * s;   // ksq / (pi D)^2
         return knorm * airy_kvalue<T>(t, obs, obssq);
       }
       case GSB_BOX: {

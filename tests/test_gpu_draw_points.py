@@ -66,3 +66,47 @@ def test_one_object_into_a_double_image_by_the_split_path(n):
     a, b = lo.flat.cpu().numpy(), hi.flat.cpu().numpy()
     # single precision: a few 1e-7 of the value a wave vector, summed over the image with random signs
     assert np.abs(a - b).max() <= 3e-6 * np.abs(b).max()
+
+
+MODES = {'float': ('fp32', np.float32), 'float into double': ('fp32', np.float64), 'double': ('fp64', np.float64)}
+
+
+# (FFT size, pixel scale): Nk = N at 0.2, several times N at the larger scales
+@pytest.mark.parametrize('min_n,scale', [(192, 0.2), (192, 1.), (256, 2.2), (384, 1.), (512, 0.2), (768, 1.5), (1024, 0.2),
+                                         (1024, 1.)])
+@pytest.mark.parametrize('mode', sorted(MODES))
+def test_fused_and_split_kernels_give_the_same_bits(mode, min_n, scale):
+    """Which of the two a bucket runs on is chosen by a timing, so it must not show in the pixels."""
+    from galsim_b200 import _lib
+    B = 3
+    gsp = galsim.GSParams(minimum_fft_size=min_n, folding_threshold=0.05, stepk_minimum_hlr=1., maximum_fft_size=1 << 15)
+    p = _profiles(gsp, B)
+    y, x = np.mgrid[:24, :24] - 11.5
+    psf = galsim.InterpolatedImage(galsim.Image((1. + (x * x + 1.1 * y * y) / 4.) ** -3., scale=0.35), gsparams=gsp)
+    p['sum'] = galsim.Convolve(galsim.Add(p['sersic'] * 0.4, p['exponential'] * 0.6), p['moffat'])
+    p['image'] = galsim.Convolve(p['sersic'], psf)
+    p['tree'] = galsim.Add(galsim.Convolve(p['exponential'], p['kolmogorov']), p['moffat'].shift(0.2, 0.1))
+    precision, dtype = MODES[mode]
+    for kind, obj in p.items():
+        obj = galsim.Convolve(obj, galsim.Gaussian(sigma=0.4, gsparams=gsp)).shift(0.3, -0.2)
+        got = []
+        try:
+            for variant in (1, 2):
+                _lib.set_draw_variant(variant)
+                got.append(galsim.draw_batch(obj, nx=25, ny=18, scale=scale, dtype=dtype, precision=precision))
+        finally:
+            _lib.set_draw_variant(0)
+        assert got[0].N.min() >= min_n
+        assert np.array_equal(got[0].host(copy=True), got[1].host(copy=True)), kind
+
+
+@pytest.mark.parametrize('mode', sorted(MODES))
+def test_a_first_draw_equals_the_next_ones(mode):
+    """The call that times the two kernels returns what later calls return."""
+    precision, dtype = MODES[mode]
+    hlr = np.linspace(1., 2.5, 37)
+    obj = galsim.Convolve(galsim.Exponential(half_light_radius=hlr).shear(g1=0.1, g2=0.2), galsim.Kolmogorov(fwhm=0.7))
+    a = [galsim.draw_batch(obj, nx=150, ny=130, scale=0.2, dtype=dtype, precision=precision) for _ in range(3)]
+    assert a[0].N.min() >= 192        # (two kernels to choose from)
+    for b in a[1:]:
+        assert np.array_equal(a[0].host(copy=True), b.host(copy=True))
