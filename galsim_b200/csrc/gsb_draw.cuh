@@ -414,9 +414,10 @@ __device__ __forceinline__ const LeafT<T>& leaf_const(const StampSmem& S, int l)
 
 // The constants of leaf l in the working precision (one thread per leaf, after plan_caches).
 //
-// Float arithmetic drawn into a double image (drawImage's default precision with an ImageD) keeps
-// the general path for the profiles whose fast form rounds differently: the double image shows the
-// last bit of every operation, and its users compare such images across versions.
+// mixed: float arithmetic drawn into a double image (drawImage's default precision with an ImageD).  No
+// rounding to a float pixel hides the arithmetic there, so every profile takes its general form, whose
+// operations are correctly rounded and follow the reference's, and none the shared-constant forms with
+// hardware approximations.
 template <typename T>
 __device__ __noinline__ void set_leaf_const(StampSmem& S, int l, double dk, bool mixed)
 {
@@ -446,7 +447,7 @@ __device__ __noinline__ void set_leaf_const(StampSmem& S, int l, double dk, bool
         t.c = T(L.jac[2]);
         t.d = T(L.jac[3]);
         return;
-    } else if (L.type == GSB_SERSIC && S.sersic_cache[l] >= 0) {
+    } else if (L.type == GSB_SERSIC && S.sersic_cache[l] >= 0 && !(sizeof(T) == 4 && mixed)) {
         const SersicTableView& v = S.sersic[l];
         t.kind = kLeafSersic;
         t.cache = S.sersic_cache[l];
@@ -763,7 +764,17 @@ __device__ __forceinline__ T leaf_points(const StampSmem& S, const unsigned char
 #pragma unroll 1
         for (int v = 0; v < V; ++v) {
             const int j = j0 + v * js;
-            const T val = leaf_kvalue<T>(S.leaf[l], S.sersic, kx, T(j) * T(dk), g, i, j + hk);
+            T val;
+            if (sizeof(T) == 4 && S.leaf[l].type == GSB_SERSIC && S.sersic_cache[l] >= 0) {
+                const LeafParams& P = S.leaf[l];
+                const T A = T(P.jac[0]), B = T(P.jac[1]), C = T(P.jac[2]), D = T(P.jac[3]), r0 = T(P.d[0]), ky = T(j) * T(dk);
+                const T u = mul_add(A, kx, mul_rn(C, ky)), w = mul_add(B, kx, mul_rn(D, ky));
+                val = T(P.flux) * sersic_kvalue_smem<T>(
+                          S.sersic[l], reinterpret_cast<const typename NodeT<T>::type*>(cache + S.sersic_cache[l]),
+                          mul_add(u, u, mul_rn(w, w)) * r0 * r0);
+            } else {
+                val = leaf_kvalue<T>(S.leaf[l], S.sersic, kx, T(j) * T(dk), g, i, j + hk);
+            }
 #pragma unroll
             for (int w = 0; w < V; ++w) if (w == v) out[w] = val;
         }

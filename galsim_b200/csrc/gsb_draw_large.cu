@@ -68,12 +68,11 @@ struct LargeArgs {
     int cache_bytes;     // shared memory for the per-stamp caches (factored program)
 };
 
-// Float arithmetic drawn into a double image (drawImage's default precision with an ImageD) shows the
-// last bit of every operation, and its users compare such images across versions: it keeps the fused
-// kernels' radix plan.  One object at a time is what is drawn so, where the FFTs are little of the call
-// (a 150 x 150 image 0.86 ms); in a batch of large stamps block_fft_pass is the faster by far (six
-// stamps of N = 4096 .. 8192: 6.8 ms against 11.7).  PER: radix 2 at N = 8192 has 8 butterflies a
-// thread.
+// Float arithmetic drawn into a double image takes the fused kernels' radix plan above N = 1024 too, with
+// the general forms of the profiles (set_leaf_const): what such an image holds does not depend on its FFT
+// size.  One object at a time is what is mostly drawn so, where the FFTs are little of the call (a 150 x 150
+// image 0.86 ms); a batch of large stamps is slower by it (six of N = 4096 .. 8192: 11.7 ms against 6.8).
+// PER: radix 2 at N = 8192 has 8 butterflies a thread.
 template <int THREADS>
 __device__ __noinline__ void block_fft_mixed(float2* buf, int N, const double2* tw)
 { block_fft<float, +1, (THREADS >= 1024 ? 4 : 8)>(buf, N, tw); }
