@@ -764,17 +764,7 @@ __device__ __forceinline__ T leaf_points(const StampSmem& S, const unsigned char
 #pragma unroll 1
         for (int v = 0; v < V; ++v) {
             const int j = j0 + v * js;
-            T val;
-            if (sizeof(T) == 4 && S.leaf[l].type == GSB_SERSIC && S.sersic_cache[l] >= 0) {
-                const LeafParams& P = S.leaf[l];
-                const T A = T(P.jac[0]), B = T(P.jac[1]), C = T(P.jac[2]), D = T(P.jac[3]), r0 = T(P.d[0]), ky = T(j) * T(dk);
-                const T u = mul_add(A, kx, mul_rn(C, ky)), w = mul_add(B, kx, mul_rn(D, ky));
-                val = T(P.flux) * sersic_kvalue_smem<T>(
-                          S.sersic[l], reinterpret_cast<const typename NodeT<T>::type*>(cache + S.sersic_cache[l]),
-                          mul_add(u, u, mul_rn(w, w)) * r0 * r0);
-            } else {
-                val = leaf_kvalue<T>(S.leaf[l], S.sersic, kx, T(j) * T(dk), g, i, j + hk);
-            }
+            const T val = leaf_kvalue<T>(S.leaf[l], S.sersic, kx, T(j) * T(dk), g, i, j + hk);
 #pragma unroll
             for (int w = 0; w < V; ++w) if (w == v) out[w] = val;
         }
