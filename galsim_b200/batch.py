@@ -328,7 +328,7 @@ def plan_batch(obj, nx=None, ny=None, scale=None, dtype=np.float32, method='fft'
         prof = compound.Convolve(prof, box.Pixel(scale=1.0, gsparams=obj.gsparams),
                                  real_space=False, gsparams=obj.gsparams)
     prog = Program(prof, tables=tables)
-    prog.upload()
+    prog.upload_ahead()
     plan = BatchPlan(prog, nx, ny, nx is not None, flux_scale, dtype, scale, precision)
     # 'no_pixel' / 'sb' on a profile analytic in real space is drawn in real space, as
     # drawImage does (gsobject.py:1810-1811)

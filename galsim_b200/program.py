@@ -185,24 +185,34 @@ class Program(object):
             self._upload_columns()
         else:
             self._upload_records()
-        dev = _lib.Device.torch_device()
-        self.d_info = torch.empty(self.B * self.L * 2, dtype=torch.float64, device=dev)
-        self._uploaded = torch.cuda.current_stream(dev).record_event()
-        self._upload_stream = torch.cuda.current_stream(dev)
+        self.d_info = torch.empty(self.B * self.L * 2, dtype=torch.float64, device=_lib.Device.torch_device())
         if self.sersic_n is None and not self.image_order and self.moffat_beta is None:
             self.tables = None
         elif getattr(self, 'tables', None) is None:
             self.tables = _lib.TablePool.acquire()
             self._pooled_tables = True
 
+    def upload_ahead(self):
+        """upload() for a later use under any stream: a batch may be planned by one thread and run by
+        another (draw_batches), each on its own current stream, and the expansion of the columns is
+        asynchronous."""
+        import torch
+        self.upload()
+        stream = torch.cuda.current_stream(_lib.Device.torch_device())
+        self._uploaded = (stream, stream.record_event())
+
+    _uploaded = None
+
     def _use_uploaded(self):
-        """Order the current stream after the upload, and keep its memory until that stream is done
-        with it: a batch may be planned by one thread and run by another (draw_batches), each on
-        its own current stream, and the expansion of the columns is asynchronous."""
+        """Order the current stream after upload_ahead's, and keep the records' memory until it is done
+        with them.  (Records uploaded by the call that uses them are on its stream.)"""
+        if self._uploaded is None:
+            return
         import torch
         cur = torch.cuda.current_stream(_lib.Device.torch_device())
-        if cur != self._upload_stream:
-            cur.wait_event(self._uploaded)
+        stream, event = self._uploaded
+        if cur != stream:
+            cur.wait_event(event)
             self.d_leaves.record_stream(cur)
             self.d_info.record_stream(cur)
 
@@ -397,6 +407,7 @@ class Program(object):
         """Forget the device copy and sizing after the host records (bld.leaves / phases /
         scales) were changed in place."""
         self.d_leaves = None
+        self._uploaded = None
         self._prepared = False
         self._geom = None
         self._graph_state = None
