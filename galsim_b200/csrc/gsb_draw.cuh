@@ -680,11 +680,29 @@ __device__ __forceinline__ float fast_rcp(float x) { float y; asm("rcp.approx.ft
 __device__ __forceinline__ float fast_rsqrt(float x) { float y; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float fast_sqrt(float x) { float y; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 
+// f / x, inv the hardware's reciprocal of x: its quotient corrected once by the exact residual (rounded
+// once, as a division; inv alone is wrong by up to one ulp, f inv by two).
+__device__ __forceinline__ float quotient(float f, float x, float inv)
+{
+    const float q = mul_rn(f, inv);
+    return fmaf(fmaf(-q, x, f), inv, q);
+}
+
+// 1 / sqrt(x): the hardware's, after one Newton step.
+__device__ __forceinline__ float refined_rsqrt(float x)
+{
+    const float s = fast_rsqrt(x);
+    return fmaf(0.5f * s, fmaf(-mul_rn(x, s), s, 1.f), s);
+}
+
 // Sersic FT at V points from the shared-memory nodes (FP32).  One reciprocal of k^2 serves the node
-// offset and both divisions; the offset's logarithm is a series in the ratio's excess over 1 (an
+// offset and the final quotient; the offset's logarithm is a series in the ratio's excess over 1 (an
 // exact difference) where the table is fine enough for its degree; the interval comes from the
 // hardware logarithm (a point within rounding of a node may take the neighbouring cubic, which
-// agrees there to third order).
+// agrees there to third order).  The offset enters as a share s of the spacing, so that the two nodes'
+// weights add up to 1 whatever the spacing's rounding.  Against the general form (divisions, logf) the rms
+// error of a float image is 0.85 times as large; with f inv in place of the quotient and weights aa / h and
+// bb / h by a rounded 1 / h it was 1.3 to 1.5 times.
 template <int V>
 __device__ __forceinline__ void sersic_points(const LeafT<float>& L, const unsigned char* cache,
                                               const float (&ksq)[V], float (&out)[V])
@@ -716,10 +734,11 @@ __device__ __forceinline__ void sersic_points(const LeafT<float>& L, const unsig
             aa = mul_rn(0.5f, logf(n1.w * inv));
         }
         const float bb = h - aa;
-        const float cub = aa * bb * fmaf(aa + h, n0.z, (bb + h) * n1.z);
-        float r = fmaf(cub, -1.f / 6.f, fmaf(aa, n0.y, bb * n1.y)) * inv_h * inv;
+        const float s = mul_rn(aa, inv_h);
+        const float lin = fmaf(s, n0.y - n1.y, n1.y);
+        float r = quotient(fmaf(s * bb * (-1.f / 6.f), fmaf(aa + h, n0.z, mul_rn(bb + h, n1.z)), lin), k2, inv);
         if (!(k2 >= kmin && k2 < kmax)) {
-            if (k2 >= kmax) r = fmaf(L.q[5], fast_rsqrt(k2), L.q[4]) * inv;
+            if (k2 >= kmax) r = quotient(fmaf(L.q[5], refined_rsqrt(k2), L.q[4]), k2, inv);
             else r = fmaf(k2, fmaf(k2, L.q[3], L.q[2]), 1.f);
         }
         out[v] = r;
@@ -831,10 +850,16 @@ __device__ __forceinline__ T leaf_points(const StampSmem& S, const unsigned char
                 out[v] = i >= int(r.x) && i < int(r.y) ? s * s * s : 0.f;
             }
         } else if (kind == kLeafKolm) {
-            // exp(-(k^2)^(5/6)); log2 of 0 is -inf, and its power 0
+            // exp(-(k^2)^(5/6)), the power as k^2 times its -1/6th power r, whose error is a sixth of the
+            // logarithm's and is then taken out by a Newton step on r^6 k^2 = 1 (the general form's power
+            // has 5/6 of the logarithm's: 1e-7 at k^2 = 4).  Below 1e-30 the value is 1.
 #pragma unroll
-            for (int v = 0; v < V; ++v)
-                out[v] = fast_exp2(-1.44269504f * fast_exp2(fast_log2(ksq[v]) * (5.f / 6.f)));
+            for (int v = 0; v < V; ++v) {
+                const float x = fmaxf(ksq[v], 1e-30f);
+                const float r = fast_exp2(fast_log2(x) * (-1.f / 6.f)), r3 = mul_rn(mul_rn(r, r), r);
+                const float y = mul_rn(x, fmaf(mul_rn(r, 1.f / 6.f), fmaf(-mul_rn(x, r3), r3, 1.f), r));
+                out[v] = expf(-y);
+            }
         } else if (kind == kLeafMoffatSum) {
             moffat_sum_points<V>(L, cache, ksq, out);
         } else if (kind == kLeafAiry) {

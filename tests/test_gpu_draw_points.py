@@ -123,3 +123,21 @@ def test_double_images_are_those_of_the_general_forms():
     for name, obj, nx, ny in cases(galsim):
         a = obj.drawImage(galsim.ImageD(nx, ny), scale=0.2, method='fft').array
         assert np.abs(a - gold[name]).max() <= 1e-8 * gold[name].max(), name
+
+
+@pytest.mark.parametrize('kind', ['exponential', 'sersic', 'moffat', 'moffat_half', 'kolmogorov', 'sersic_kolmogorov'])
+def test_float_forms_are_as_exact_as_the_general_ones(kind):
+    """rms error of float images against double: the fast forms' against that of the general forms (which a
+    double image takes; rounded to float here), over FFT sizes and pixel scales.  Not larger, with a tenth for
+    the scatter of the ratio (13 sizes of three images, whose roundings the two share in part)."""
+    ratio = []
+    for min_n, scale in [(64, 1.), (64, 0.2), (96, 0.7), (128, 1.3), (128, 0.2), (192, 1.), (192, 0.2), (256, 0.6), (384, 1.),
+                         (512, 0.2), (768, 0.4), (1024, 0.2), (2048, 0.2)]:
+        gsp = galsim.GSParams(minimum_fft_size=min_n, folding_threshold=0.05, stepk_minimum_hlr=1., maximum_fft_size=1 << 15)
+        p = _profiles(gsp, 3)
+        p['sersic_kolmogorov'] = galsim.Convolve(p['sersic'], galsim.Kolmogorov(fwhm=0.7, gsparams=gsp))
+        obj = galsim.Convolve(p[kind], galsim.Gaussian(sigma=0.4, gsparams=gsp)).shift(0.3, -0.2)
+        fast, general, exact = [galsim.draw_batch(obj, nx=41, ny=30, scale=scale, dtype=d, precision=q).host(copy=True)
+                                for q, d in (('fp32', np.float32), ('fp32', np.float64), ('fp64', np.float64))]
+        ratio.append(np.sqrt(np.mean((fast - exact) ** 2) / np.mean((general.astype(np.float32) - exact) ** 2)))
+    assert np.exp(np.mean(np.log(ratio))) <= 1.1, ratio
