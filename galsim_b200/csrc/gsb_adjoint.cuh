@@ -194,7 +194,7 @@ __device__ __forceinline__ LeafD<T> leaf_grad_fast(const AdjSmem& A, const unsig
         if (L.kind == kLeafSersic && S.aux_cache[l] >= 0) {
             const float u = L.a * float(i) + L.c * float(j), w = L.b * float(i) + L.d * float(j);
             const float k2 = u * u + w * w, flux = L.flux;
-            const float inv = fast_rcp(k2);
+            const float inv0 = fast_rcp(k2), inv = fmaf(fmaf(-k2, inv0, 1.f), inv0, inv0);
             const float h = L.q[6], inv_h = L.q[7];
             float phi, dphi, dphin;
             if (k2 >= L.q[0] && k2 < L.q[1]) {
@@ -203,7 +203,7 @@ __device__ __forceinline__ LeafD<T> leaf_grad_fast(const AdjSmem& A, const unsig
                 const int q = max(1, min(__float_as_int(fmaf(fast_log2(k2), L.q[8], L.q[9]) + 12582912.f) - 0x4b400000, L.n - 1));
                 const float4 n0 = node[q - 1], n1 = node[q];
                 const float2 d0 = dnode[q - 1], d1 = dnode[q];
-                const float e = (n1.w - k2) * inv;
+                const float e = (n1.w - k2) * inv0;
                 float aa;
                 if (h < 0.04f) {
                     float p = fmaf(e, -1.f / 16.f, 1.f / 14.f);      // ln(1 + e) / 2, as sersic_points
@@ -215,15 +215,15 @@ __device__ __forceinline__ LeafD<T> leaf_grad_fast(const AdjSmem& A, const unsig
                     p = fmaf(e, p, 0.5f);
                     aa = e * p;
                 } else {
-                    aa = 0.5f * logf(n1.w * inv);
+                    aa = 0.5f * logf(n1.w * inv0);
                 }
-                const float bb = h - aa, P = aa * bb;
+                const float bb = h - aa, P = aa * bb, s = aa * inv_h, c = s * bb * (-1.f / 6.f);
                 const float Q = fmaf(aa + h, n0.z, (bb + h) * n1.z);
-                const float f = fmaf(P * Q, -1.f / 6.f, fmaf(aa, n0.y, bb * n1.y)) * inv_h;
+                const float f = fmaf(c, Q, fmaf(s, n0.y - n1.y, n1.y));
                 const float fl = fmaf(fmaf(aa - bb, Q, P * (n1.z - n0.z)), -1.f / 6.f, n1.y - n0.y) * inv_h;
                 const float Qn = fmaf(aa + h, d0.y, (bb + h) * d1.y);
-                const float fn = fmaf(P * Qn, -1.f / 6.f, fmaf(aa, d0.x, bb * d1.x)) * inv_h;
-                phi = f * inv;
+                const float fn = fmaf(c, Qn, fmaf(s, d0.x - d1.x, d1.x));
+                phi = quotient(f, k2, inv0);
                 dphi = (0.5f * fl - f) * inv * inv;
                 dphin = (fn - float(A.dn[l].dfront) * fl) * inv;     // the argument moves with the grid origin
             } else {
@@ -238,8 +238,21 @@ __device__ __forceinline__ LeafD<T> leaf_grad_fast(const AdjSmem& A, const unsig
             r.gy = d2 * w;
             return r;
         }
+        if (L.kind == kLeafExpFast) {
+            const ushort2 c = reinterpret_cast<const ushort2*>(cache + L.cache)[hk + j];
+            LeafD<T> r{T(0), T(0), T(0), T(0), T(0)};
+            if (i < int(c.x) || i >= int(c.y)) return r;
+            const float u = L.a * float(i) + L.c * float(j), w = L.b * float(i) + L.d * float(j);
+            const float s = refined_rsqrt(1.f + (u * u + w * w)), ss = s * s;
+            r.unit = ss * s;
+            r.v = L.flux * r.unit;
+            const float d2 = -3.f * r.v * ss * L.size;
+            r.gx = d2 * u;
+            r.gy = d2 * w;
+            return r;
+        }
     }
-    if (leaf_const<T>(S, l).kind == kLeafExp) {
+    if (sizeof(T) == 8 && leaf_const<T>(S, l).kind == kLeafExp) {
         const LeafT<T>& L = leaf_const<T>(S, l);
         const ushort2 c = reinterpret_cast<const ushort2*>(cache + L.cache)[hk + j];
         LeafD<T> r{T(0), T(0), T(0), T(0), T(0)};

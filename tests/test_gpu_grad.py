@@ -426,3 +426,33 @@ def test_workspace_of_buckets_of_several_sizes():
         ref = part.adjoint_stamps(cot[torch.as_tensor(i, device='cuda')].contiguous().reshape(-1), _lib.F32)
         # (sums over a stamp's blocks: atomics in another order each time)
         assert torch.allclose(g[torch.as_tensor(i, device='cuda')], ref, rtol=1e-9, atol=1e-12 * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize('min_n,scale', [(32, 1.), (64, 0.2), (96, 0.7), (192, 0.2), (192, 1.), (512, 0.2), (1024, 0.2), (2048, 0.2)])
+@pytest.mark.parametrize('kind', ['exponential', 'sum'])
+def test_float_gradients_of_exponential_leaves(kind, min_n, scale):
+    """The float adjoint's form of Exponential leaves (column ranges, one square root), alone and in a bulge + disk
+    pair, against the double adjoint: a few 1e-7 of a term, over up to N^2 terms of either sign: 1e-5 of the
+    largest entry."""
+    rng = np.random.default_rng(8)
+    B = 3
+    gsp = galsim.GSParams(minimum_fft_size=min_n, folding_threshold=0.05, stepk_minimum_hlr=1., maximum_fft_size=1 << 15)
+
+    def sheared(obj):
+        g = rng.uniform(-0.2, 0.2, (2, B))
+        return obj.shear(g1=g[0], g2=g[1])
+
+    disk = sheared(galsim.Exponential(half_light_radius=rng.uniform(0.8, 1.5, B), flux=rng.uniform(1., 3., B), gsparams=gsp))
+    bulge = sheared(galsim.Sersic(n=rng.uniform(1., 3.5, B), half_light_radius=rng.uniform(0.8, 1.5, B), gsparams=gsp))
+    gal = {'exponential': disk, 'sum': galsim.Add(bulge, disk)}[kind]
+    obj = galsim.Convolve(gal.shift(0.1, -0.2), galsim.Moffat(beta=3., fwhm=0.8, gsparams=gsp))
+    cot = torch.as_tensor(rng.standard_normal((B, 22, 24)), device='cuda')
+    got = {}
+    for precision, dtype in (('fp32', np.float32), ('fp64', np.float64)):
+        plan = autodiff.RecordPlan(obj, 24, 22, scale, dtype, precision)
+        plan.draw()
+        got[precision] = plan.adjoint(cot)
+    for key in ('leaf_flux', 'leaf_jac', 'leaf_size'):
+        a, b = got['fp32'][key], got['fp64'][key]
+        for l in range(b.shape[1]):
+            assert float((a[:, l] - b[:, l]).abs().max()) <= 1e-5 * max(float(b[:, l].abs().max()), 1e-3), (key, l)
