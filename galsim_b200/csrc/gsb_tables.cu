@@ -172,13 +172,16 @@ constexpr int kLogLevels = 57;            // levels 5 .. 61: all the halving can
 struct OgataLog {
     double h;
     const double* a;
+    int have;                             // levels that are spread (kLogLev0 on)
     int qmin[kLogLevels], len[kLogLevels], off[kLogLevels];
 };
 
-// A_l[q], one block per grid point q: the nodes within W / 2 grid points of it (the node list is
-// ascending in ln x).
+// A_l[q]: the nodes within W / 2 grid points of q (the node list is ascending in ln x), a block per grid point
+// and slice of its nodes, the slices added up by ogata_log_sum_kernel.  (Half of a level's nodes lie within
+// the last 20 grid points: a block per grid point alone took 1.6 ms a level of a million nodes.)
+constexpr int kLogSlices = 16;
 __global__ void __launch_bounds__(256) ogata_log_kernel(const double2* __restrict__ xw, int n, double h, int qmin,
-                                                        double* __restrict__ a)
+                                                        double* __restrict__ slices)
 {
     const int q = qmin + int(blockIdx.x);
     auto lower = [&](double u) {
@@ -189,9 +192,12 @@ __global__ void __launch_bounds__(256) ogata_log_kernel(const double2* __restric
         }
         return lo;
     };
-    const int i0 = lower(q - 0.5 * kLogW), i1 = lower(q + 0.5 * kLogW);
+    __shared__ int range[2];
+    if (threadIdx.x < 2) range[threadIdx.x] = lower(q + (threadIdx.x == 0 ? -0.5 : 0.5) * kLogW);
+    __syncthreads();
+    const int i0 = range[0], i1 = range[1];
     double sum = 0.;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+    for (int i = i0 + int(blockIdx.y) * 256 + threadIdx.x; i < i1; i += 256 * kLogSlices) {
         const double t = xw[i].x / h - q;
         const double v = 2. * t / kLogW;
         const double s = fabs(t) < 1e-9 ? 1. : sinpi(t) / (kPi * t);
@@ -203,8 +209,17 @@ __global__ void __launch_bounds__(256) ogata_log_kernel(const double2* __restric
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int w = 1; w < 8; ++w) sum += part[w];
-        a[blockIdx.x] = sum;
+        slices[blockIdx.x * kLogSlices + blockIdx.y] = sum;
     }
+}
+
+__global__ void ogata_log_sum_kernel(const double* __restrict__ slices, int len, double* __restrict__ a)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= len) return;
+    double sum = 0.;
+    for (int c = 0; c < kLogSlices; ++c) sum += slices[q * kLogSlices + c];
+    a[q] = sum;
 }
 
 // The Sersic profile and its n-derivative along the table's moving grid (GSB_TABLES_DN) at
@@ -778,8 +793,8 @@ __global__ void __launch_bounds__(THREADS, THREADS > 64 ? 1 : 8) sersic_table_ke
             const int mlast = min(c1 - 1, w0 + 32 * R - 1);
             while (__any_sync(0xffffffffu, run != 0u)) {
                 // the reference halves until its level counter passes 60: the last sum is at 61
-                if (l > kLogLev0 + kLogLevels - 1) {
-                    if (lane == 0) atomicOr(status_out, 1);
+                if (l >= kLogLev0 + lg.have) {
+                    if (lane == 0) atomicOr(status_out, lg.have == kLogLevels ? 1 : 2);   // (2: spread more)
                     break;
                 }
                 const int j = l - kLogLev0;
@@ -1458,7 +1473,9 @@ static int sersic_stride(const double* h_n, int count, const gsb_gsparams* gsp)
 }
 
 // The resampled quadrature levels of each device and spacing, kept while they are among the last
-// few spacings used (a spacing is a GSParams setting: a program has one or two; 0.4 MB each).
+// few spacings used (a spacing is a GSParams setting: a program has one or two; 0.4 MB each).  Levels are
+// spread as far as a build needs them: those up to level 15 (n <= 2) take 0.4 ms, up to 20 (n <= 4) 2.5, all 57,
+// most of a million nodes each, 60.
 namespace {
 struct LogEntry {
     double* a = nullptr;
@@ -1471,24 +1488,27 @@ unsigned long long g_log_clock = 0;
 std::mutex g_log_mutex;
 }  // namespace
 
-// The levels for grid spacing h (g_log_mutex held).
-static int ogata_log_levels(DeviceState* st, double h, cudaStream_t stream, OgataLog* out)
+// The first `need` levels for grid spacing h (g_log_mutex held).
+static int ogata_log_levels(DeviceState* st, double h, int need, cudaStream_t stream, OgataLog* out)
 {
     int dev = 0;
     cudaGetDevice(&dev);
     LogEntry* slots = g_log[dev & 63];
     LogEntry* e = slots;
-    for (int i = 0; i < kLogEntries; ++i) {
-        if (slots[i].a && slots[i].lg.h == h) {
-            slots[i].used = ++g_log_clock;
-            *out = slots[i].lg;
-            return GSB_OK;
-        }
-        if (slots[i].used < e->used) e = &slots[i];
+    bool found = false;
+    for (int i = 0; i < kLogEntries && !found; ++i) {
+        found = slots[i].a && slots[i].lg.h == h;
+        if (found || slots[i].used < e->used) e = &slots[i];
+    }
+    need = std::min(std::max(need, 1), kLogLevels);
+    if (found && e->lg.have >= need) {
+        e->used = ++g_log_clock;
+        *out = e->lg;
+        return GSB_OK;
     }
     OgataLog lg{};
     lg.h = h;
-    int total = 0, cnt[kLogLevels];
+    int total = 0, cnt[kLogLevels], longest = 0;
     auto psi = [](double t) { return t * std::tanh(0.5 * M_PI * std::sinh(t)); };
     for (int j = 0; j < kLogLevels; ++j) {
         const double hl = std::ldexp(1.0, -(kLogLev0 + j));
@@ -1500,35 +1520,46 @@ static int ogata_log_levels(DeviceState* st, double h, cudaStream_t stream, Ogat
         lg.len[j] = int(std::ceil(std::log(x1) / h)) + kLogW / 2 + 1 - lg.qmin[j] + 1;
         lg.off[j] = total;
         total += lg.len[j];
+        longest = std::max(longest, lg.len[j]);
     }
-    cudaFree(e->a);
-    e->a = nullptr;
-    e->lg.h = 0.;
-    GSB_CUDA_CHECK(cudaMalloc(&e->a, sizeof(double) * total));
+    // a new spacing takes the place of the one used longest ago; more levels of a known one are added to
+    // its array (builds in flight read the levels they were given)
+    if (!found) {
+        cudaFree(e->a);
+        e->a = nullptr;
+        e->lg = OgataLog{};
+        GSB_CUDA_CHECK(cudaMalloc(&e->a, sizeof(double) * (total + (size_t)kLogSlices * longest)));
+    }
+    const int have = e->lg.have;
     double2* d_tmp = nullptr;
-    int rc = GSB_OK;
-    cudaError_t ce = cudaMallocAsync(&d_tmp, sizeof(double2) * kNroot, stream);
-    for (int j = 0; j < kLogLevels && ce == cudaSuccess; ++j) {
+    double* d_slices = e->a + total;                      // (this function's alone: the mutex is held to its end)
+    cudaError_t ce = cudaSuccess;
+    if (kLogLev0 + need - 1 > kLevMax) ce = cudaMalloc(&d_tmp, sizeof(double2) * kNroot);
+    for (int j = have; j < need && ce == cudaSuccess; ++j) {
         const int lev = kLogLev0 + j;
         const double2* xw = d_tmp;
         if (lev <= kLevMax) xw = st->d_xw + st->og.off[lev - kLevMin];
         else ogata_level_kernel<<<(cnt[j] + 255) / 256, 256, 0, stream>>>(d_tmp, st->d_root, std::ldexp(1.0, -lev), cnt[j]);
-        ogata_log_kernel<<<lg.len[j], 256, 0, stream>>>(xw, cnt[j], h, lg.qmin[j], e->a + lg.off[j]);
+        ogata_log_kernel<<<dim3(lg.len[j], kLogSlices), 256, 0, stream>>>(xw, cnt[j], h, lg.qmin[j], d_slices);
+        ogata_log_sum_kernel<<<(lg.len[j] + 127) / 128, 128, 0, stream>>>(d_slices, lg.len[j], e->a + lg.off[j]);
         ce = cudaGetLastError();
     }
-    if (d_tmp) cudaFreeAsync(d_tmp, stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);
+    if (d_tmp) cudaFree(d_tmp);
     if (ce != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(e->a);
-        e->a = nullptr;
+        if (!found) {
+            cudaFree(e->a);
+            e->a = nullptr;
+        }
         return set_error(GSB_ERR_CUDA, std::string("resampled quadrature levels: ") + cudaGetErrorString(ce));
     }
     lg.a = e->a;
+    lg.have = need;
     e->lg = lg;
     e->used = ++g_log_clock;
     *out = lg;
-    return rc;
+    return GSB_OK;
 }
 
 // Builds of at most this many tables per SM take one 512-thread block of single nodes a table: 400
@@ -1639,46 +1670,60 @@ int sersic_tables_build(gsb_tables* t, const double* h_n, const double* h_trunc,
     const int p = std::max(1, int(std::ceil(dlogk / kLogMaxStep)));
     // held until the launch that reads the resampled levels is queued: an eviction frees only
     // after the device has finished it
-    std::unique_lock<std::mutex> lock(g_log_mutex);
+    std::unique_lock<std::mutex> lock(g_log_mutex, std::defer_lock);
+    double nmax = 0.;
+    for (int i = 0; i < count; ++i) nmax = std::max(nmax, h_n[i]);
+    // levels: at the default accuracies the last one that a table's nodes ask for is 13, 15, 18, 20, 22 and 26 at
+    // n = 1.5, 2, 3, 4, 5 and 6.2; and two from the one that its lowest node starts at.  A node that asks for
+    // more has the build run again with three more.
+    int need = 2;
     {
-        const int rc = ogata_log_levels(st, dlogk / p, stream, &lg);
-        if (rc) return rc;
+        const double kderiv6 = std::exp(std::lgamma(8. * nmax) - std::lgamma(2. * nmax)) / 2304.;
+        const double k = std::exp(std::log(gsp->kvalue_accuracy / kderiv6) / 6. - 0.001);
+        for (double h0 = 1. / 32.; h0 > 100. * k && need < kLogLevels; h0 *= 0.5) ++need;
+        need = std::max(need, int(10.5 + 2.55 * nmax) - kLogLev0 + 1);
     }
     // truncated tables: rounds of kTableRound ln k nodes, each followed by the stopping scan
     const int rounds = has_trunc ? (stride + kTableRound - 1) / kTableRound : 0;
     if (rounds > kMaxRounds) return set_error(GSB_ERR_UNSUPPORTED, "Sersic table too long");
-    // d_status[0]: convergence status; d_status[1 + r]: some table still needs nodes after round r
-    GSB_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int) * (1 + rounds), stream));
-    sersic_setup_kernel<<<(count + 31) / 32, 96, 0, stream>>>(d_n, d_trunc, count, *gsp, t->d_header, stride, dheader);
-    GSB_CUDA_CHECK(cudaGetLastError());
-    SersicScan* scan = static_cast<SersicScan*>(t->d_scan);
-    if (has_trunc) {
-        sersic_scan_init_kernel<<<(count + 127) / 128, 128, 0, stream>>>(t->d_header, count, scan);
-        GSB_CUDA_CHECK(cudaGetLastError());
-        for (int r = 0; r < rounds; ++r) {
-            const int* prev_live = r > 0 ? d_status + r : nullptr;
-            const long long tw = (long long)count * kTableRound;
-            sersic_trunc_nodes_kernel<<<(unsigned)((tw * 32 + 255) / 256), 256, 0, stream>>>(
-                t->d_header, count, r * kTableRound, kTableRound, st->og, scan, t->d_val, stride, prev_live, d_status);
-            GSB_CUDA_CHECK(cudaGetLastError());
-            sersic_scan_kernel<<<(count + 63) / 64, 64, 0, stream>>>(t->d_header, count, stride, r * kTableRound,
-                                                                     kTableRound, *gsp, t->d_val, scan, prev_live,
-                                                                     d_status + 1 + r);
-            GSB_CUDA_CHECK(cudaGetLastError());
-        }
-    }
-    double nmax = 0.;
-    for (int i = 0; i < count; ++i) nmax = std::max(nmax, h_n[i]);
-    {
-        const int rc = count <= kSmallBuild * st->sm_count
-                           ? launch_sersic_tables<1, 512>(t, count, stride, nmax, gsp, lg, p, scan, dnode, dheader, d_status, stream)
-                           : launch_sersic_tables<3, 64>(t, count, stride, nmax, gsp, lg, p, scan, dnode, dheader, d_status, stream);
-        if (rc) return rc;
-    }
-    lock.unlock();
     int h_status = 0;
-    GSB_CUDA_CHECK(cudaMemcpyAsync(&h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    GSB_CUDA_CHECK(cudaStreamSynchronize(stream));
+    for (;; need = std::max(need, lg.have) + 3) {
+        lock.lock();
+        {
+            const int rc = ogata_log_levels(st, dlogk / p, need, stream, &lg);
+            if (rc) return rc;
+        }
+        // d_status[0]: convergence status; d_status[1 + r]: some table still needs nodes after round r
+        GSB_CUDA_CHECK(cudaMemsetAsync(d_status, 0, sizeof(int) * (1 + rounds), stream));
+        sersic_setup_kernel<<<(count + 31) / 32, 96, 0, stream>>>(d_n, d_trunc, count, *gsp, t->d_header, stride, dheader);
+        GSB_CUDA_CHECK(cudaGetLastError());
+        SersicScan* scan = static_cast<SersicScan*>(t->d_scan);
+        if (has_trunc) {
+            sersic_scan_init_kernel<<<(count + 127) / 128, 128, 0, stream>>>(t->d_header, count, scan);
+            GSB_CUDA_CHECK(cudaGetLastError());
+            for (int r = 0; r < rounds; ++r) {
+                const int* prev_live = r > 0 ? d_status + r : nullptr;
+                const long long tw = (long long)count * kTableRound;
+                sersic_trunc_nodes_kernel<<<(unsigned)((tw * 32 + 255) / 256), 256, 0, stream>>>(
+                    t->d_header, count, r * kTableRound, kTableRound, st->og, scan, t->d_val, stride, prev_live, d_status);
+                GSB_CUDA_CHECK(cudaGetLastError());
+                sersic_scan_kernel<<<(count + 63) / 64, 64, 0, stream>>>(t->d_header, count, stride, r * kTableRound,
+                                                                         kTableRound, *gsp, t->d_val, scan, prev_live,
+                                                                         d_status + 1 + r);
+                GSB_CUDA_CHECK(cudaGetLastError());
+            }
+        }
+        {
+            const int rc = count <= kSmallBuild * st->sm_count
+                               ? launch_sersic_tables<1, 512>(t, count, stride, nmax, gsp, lg, p, scan, dnode, dheader, d_status, stream)
+                               : launch_sersic_tables<3, 64>(t, count, stride, nmax, gsp, lg, p, scan, dnode, dheader, d_status, stream);
+            if (rc) return rc;
+        }
+        lock.unlock();
+        GSB_CUDA_CHECK(cudaMemcpyAsync(&h_status, d_status, sizeof(int), cudaMemcpyDeviceToHost, stream));
+        GSB_CUDA_CHECK(cudaStreamSynchronize(stream));
+        if (!(h_status & 2)) break;
+    }
     if (h_status) return set_error(GSB_ERR_NUMERIC, "Sersic Hankel transform did not converge");
     return GSB_OK;
 }

@@ -60,3 +60,31 @@ def test_large_build_draws_and_differentiates_as_small_builds(spacing):
     # levels' own cancellation
     np.testing.assert_allclose(img[some], simg, rtol=0, atol=1e-10 * np.abs(simg).max())
     np.testing.assert_allclose(grad[some], sgrad, rtol=0, atol=1e-8 * np.abs(sgrad).max())
+
+
+def test_levels_are_resampled_as_builds_need_them():
+    """A first build of a spacing spreads the quadrature levels its nodes ask for, not all 57; a later build that
+    needs more adds them, and one that needs no more launches none."""
+    from galsim_b200 import _lib
+    from torch.profiler import ProfilerActivity, profile
+
+    def levels(n, gsp):
+        tb = _lib.Tables()
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            tb.build_sersic(np.array([n]), gsp)
+            torch.cuda.synchronize()
+        info = tb.sersic_info()[0]
+        return sum(e.count for e in p.key_averages() if 'ogata_log_kernel' in e.key), info
+
+    gsp = galsim.GSParams(table_spacing=0.8137)
+    first, info = levels(2., gsp)
+    assert 0 < first <= 16
+    assert levels(2., gsp)[0] == 0
+    more, _ = levels(5., gsp)
+    assert 0 < more <= 16
+    assert levels(4., gsp)[0] == 0
+    again, info2 = levels(2., gsp)
+    assert again == 0 and np.array_equal(info, info2)
+    # an accuracy whose nodes ask for more levels than the rule expects gets them
+    _, info = levels(2., galsim.GSParams(table_spacing=0.8137, integration_relerr=1e-10, integration_abserr=1e-13))
+    assert info[H['STATUS']] == 0 and info[H['NUSED']] == info2[H['NUSED']]
