@@ -234,36 +234,19 @@ __device__ __forceinline__ double2 sersic_sample(double y, double invn, double d
     return make_double2(f, f * u * invn * (v + dnc));
 }
 
-// acc[r] += sum_q A[q] g[q - p (m + r)] (and the same with gd for DN), q = qlo .. qhi; g points at
-// the sample of d = 0, and samples from top on are 0.  With p = 1 the array is padded with them and the R nodes of a thread share each sample through a window in
-// registers: one shared-memory read (lane stride R doubles, R odd: no bank conflicts) and one
-// broadcast read feed R multiply-adds.
+// acc[c][r] += sum_q A[q] g[q - p (m + r)] (and the same with gd for DN) over q = qlo .. qhi, in the class c = (q - qlo)
+// mod kLogSums: several sums, so that the chain of one node's multiply-adds is not the time, counted from the
+// level's first point (qlo is a multiple of kLogSums from it), so that a node's value does not depend on how many
+// nodes a thread takes.  g points at the sample of d = 0, and samples from top on are 0.  With p = 1 the array is
+// padded with them and the R nodes of a thread share each sample through a window in registers: one
+// shared-memory read (lane stride R doubles, R odd: no bank conflicts) and one broadcast read feed R
+// multiply-adds.
+constexpr int kLogSums = 2;
 template <int R, bool DN, bool P1>
 __device__ __forceinline__ void correlate(const double* __restrict__ A, int qlo, int qhi, const double* g,
-                                          const double* gd, int m, int p, int top, double (&acc)[R],
-                                          double (&dacc)[R])
+                                          const double* gd, int m, int p, int top, double (&acc)[kLogSums][R],
+                                          double (&dacc)[kLogSums][R])
 {
-    if constexpr (R == 1 && P1) {
-        // four partial sums, so that the chain of one node's multiply-adds is not the time
-        double s[4] = {0., 0., 0., 0.}, sd[4] = {0., 0., 0., 0.};
-        int q = qlo;
-#pragma unroll 2
-        for (; q + 3 <= qhi; q += 4) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const double a = A[q + i];
-                s[i] = fma(a, g[q + i - m], s[i]);
-                if (DN) sd[i] = fma(a, gd[q + i - m], sd[i]);
-            }
-        }
-        for (; q <= qhi; ++q) {
-            s[0] = fma(A[q], g[q - m], s[0]);
-            if (DN) sd[0] = fma(A[q], gd[q - m], sd[0]);
-        }
-        acc[0] += (s[0] + s[1]) + (s[2] + s[3]);
-        if (DN) dacc[0] += (sd[0] + sd[1]) + (sd[2] + sd[3]);
-        return;
-    }
     double w[R], wd[R];
     if (P1) {
 #pragma unroll
@@ -272,16 +255,15 @@ __device__ __forceinline__ void correlate(const double* __restrict__ A, int qlo,
             if (DN) wd[r] = gd[qlo - m - r];
         }
     }
-#pragma unroll 6
-    for (int q = qlo; q <= qhi; ++q) {
+    auto step = [&](int c, int q) {
         const double a = A[q];
         if (P1) {
             w[0] = g[q - m];
             if (DN) wd[0] = gd[q - m];
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                acc[r] = fma(a, w[r], acc[r]);
-                if (DN) dacc[r] = fma(a, wd[r], dacc[r]);
+                acc[c][r] = fma(a, w[r], acc[c][r]);
+                if (DN) dacc[c][r] = fma(a, wd[r], dacc[c][r]);
             }
 #pragma unroll
             for (int r = R - 1; r > 0; --r) {
@@ -292,11 +274,20 @@ __device__ __forceinline__ void correlate(const double* __restrict__ A, int qlo,
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 const int d = min(q - p * (m + r), top);
-                acc[r] = fma(a, g[d], acc[r]);
-                if (DN) dacc[r] = fma(a, gd[d], dacc[r]);
+                acc[c][r] = fma(a, g[d], acc[c][r]);
+                if (DN) dacc[c][r] = fma(a, gd[d], dacc[c][r]);
             }
         }
+    };
+    int q = qlo;
+#pragma unroll (R == 1 ? 4 : 3)
+    for (; q + kLogSums - 1 <= qhi; q += kLogSums) {
+#pragma unroll
+        for (int c = 0; c < kLogSums; ++c) step(c, q + c);
     }
+#pragma unroll
+    for (int c = 0; c < kLogSums - 1; ++c)
+        if (q + c <= qhi) step(c, q + c);
 }
 
 // Truncated Hankel transform (math::hankel_trunc, src/math/Hankel.cpp:249-255) of a radial
@@ -809,27 +800,34 @@ __global__ void __launch_bounds__(THREADS, THREADS > 64 ? 1 : 8) sersic_table_ke
                 const int qhi = min(qmin + lg.len[j] - 1, p * mhi + dmax);
                 // samples below d0 (levels far beyond the usual) are formed on the fly
                 const int qlo = max(qmin, d0 + p * mlast + (R - 1) * p);
-                double acc[R], dacc[R];
+                double acc[kLogSums][R], dacc[kLogSums][R];
 #pragma unroll
-                for (int r = 0; r < R; ++r) acc[r] = dacc[r] = 0.;
-                for (int q = qmin; q < min(qlo, qhi + 1); ++q) {
-                    const double a = A[q];
+                for (int c = 0; c < kLogSums; ++c)
 #pragma unroll
-                    for (int r = 0; r < R; ++r) {
-                        const double2 v = sersic_sample((q - p * (m + r)) * lg.h - front, invn, dnc);
-                        acc[r] = fma(a, v.x, acc[r]);
-                        if (DN) dacc[r] = fma(a, v.y, dacc[r]);
+                    for (int r = 0; r < R; ++r) acc[c][r] = dacc[c][r] = 0.;
+                int q = qmin;
+                for (; q < min(qlo, qhi + 1); q += kLogSums) {
+#pragma unroll
+                    for (int c = 0; c < kLogSums; ++c) {
+                        if (q + c > qhi) continue;
+                        const double a = A[q + c];
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            const double2 v = sersic_sample((q + c - p * (m + r)) * lg.h - front, invn, dnc);
+                            acc[c][r] = fma(a, v.x, acc[c][r]);
+                            if (DN) dacc[c][r] = fma(a, v.y, dacc[c][r]);
+                        }
                     }
                 }
                 // (lanes past mlast read other samples of the array, or its zero padding)
-                if (qlo <= qhi)
-                    correlate<R, DN, P1>(A, qlo, qhi, g - d0, gd - d0, min(m, mlast), p, dmax + 1, acc, dacc);
+                if (q <= qhi)
+                    correlate<R, DN, P1>(A, q, qhi, g - d0, gd - d0, min(m, mlast), p, dmax + 1, acc, dacc);
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     if (!(run >> r & 1u) || l < lev[r]) continue;
                     prev[r] = cur[r];
-                    cur[r] = acc[r] / ksq[r];
-                    if (DN) dcur[r] = dacc[r] / ksq[r];
+                    cur[r] = (acc[0][r] + acc[1][r]) / ksq[r];
+                    if (DN) dcur[r] = (dacc[0][r] + dacc[1][r]) / ksq[r];
                     if (l == lev[r]) continue;
                     const double err = fabs(cur[r] - prev[r]);
                     const bool more = (err > gsp.integration_relerr * cur[r] &&

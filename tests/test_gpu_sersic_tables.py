@@ -88,3 +88,26 @@ def test_levels_are_resampled_as_builds_need_them():
     # an accuracy whose nodes ask for more levels than the rule expects gets them
     _, info = levels(2., galsim.GSParams(table_spacing=0.8137, integration_relerr=1e-10, integration_abserr=1e-13))
     assert info[H['STATUS']] == 0 and info[H['NUSED']] == info2[H['NUSED']]
+
+
+@pytest.mark.parametrize('spacing', [1., 0.3, 2.5])
+def test_a_table_does_not_depend_on_the_others_of_its_build(spacing):
+    """Small builds take one node a thread and large ones three: the same numbers, in the tables' constants and in
+    double-precision stamps drawn from them."""
+    from galsim_b200 import _lib
+    gsp = galsim.GSParams(table_spacing=spacing)
+    few = np.array([0.5, 1.3, 2.6, 4., 6.1])
+    many = np.unique(np.concatenate([few, np.linspace(0.4, 3.9, 800)]))
+    heads = []
+    for n in (few, many):
+        t = _lib.Tables()
+        t.build_sersic(n, gsp, with_dn=True)
+        heads.append(t.sersic_info()[[int(np.flatnonzero(n == v)[0]) for v in few]])
+    assert np.array_equal(heads[0], heads[1])
+    stamps = []
+    for n in (few[:4], many[many < 4.01]):
+        obj = galsim.Convolve(galsim.Sersic(n=n, half_light_radius=np.full(len(n), 0.6), gsparams=gsp), galsim.Gaussian(sigma=0.3))
+        sb = galsim.draw_batch(obj, nx=24, ny=24, scale=0.2, dtype=np.float64, precision='fp64')
+        a = sb.host(copy=True).reshape(len(n), 24, 24)
+        stamps.append(a[[int(np.flatnonzero(n == v)[0]) for v in few[:4]]])
+    assert np.array_equal(stamps[0], stamps[1])
