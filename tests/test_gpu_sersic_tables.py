@@ -111,3 +111,10 @@ def test_a_table_does_not_depend_on_the_others_of_its_build(spacing):
         a = sb.host(copy=True).reshape(len(n), 24, 24)
         stamps.append(a[[int(np.flatnonzero(n == v)[0]) for v in few[:4]]])
     assert np.array_equal(stamps[0], stamps[1])
+
+
+@pytest.mark.parametrize('count', [3, 700])
+@pytest.mark.parametrize('spacing', [0.3, 0.55])
+def test_fine_tables_against_the_oracle(count, spacing):
+    """ln k grids finer than the resampled levels' spacing: one level point in three or one in one node."""
+    test_tables_against_the_oracle(count, spacing, False)
