@@ -227,6 +227,8 @@ size_t adj_slab_bytes(int N) { return sizeof(Cx<T>) * (size_t)(N / 2 + 1) * N; }
 template <typename T, int ROW_THREADS, int COL_THREADS>
 int launch_adj_large_t(const AdjArgs& args, int N, void* work, size_t work_bytes, cudaStream_t stream)
 {
+    if (!block_fft_has(N, ROW_THREADS) || !block_fft_has(N, COL_THREADS))
+        return set_error(GSB_ERR_UNSUPPORTED, "FFT size not built");
     const size_t slab = adj_slab_bytes<T>(N);
     if (!work || work_bytes < slab) return set_error(GSB_ERR_INVALID, "adjoint workspace too small");
     const size_t row_sm = sizeof(Cx<T>) * fft_buf_len<T>(N);

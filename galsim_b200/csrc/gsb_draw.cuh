@@ -1287,7 +1287,9 @@ __global__ void __launch_bounds__(fused_warps<T, N>() * 32, fused_min_blocks<T, 
                     const T px = (r ? v.y : v.x) * inv_n2;
                     store_pixel<T>(a.out, a.out_dtype, a.add, row1 + (r ? G.nx : 0) + i, px);
                     const double d = double(px);
-                    if (sizeof(T) == 4) {          // (float pixels: exact to ~1e-13 in a plain FP64 sum)
+                    // (a lane's ~100 float pixels add up exactly in FP64 but for a range beyond 2^22: the float
+                    // fluxes are within 4e-16 of the exact sum of the pixels, as with compensation)
+                    if (sizeof(T) == 4) {
                         fsum += d;
                     } else {                       // Neumaier compensated sum in FP64
                         const double tsum = fsum + d;

@@ -291,6 +291,7 @@ int launch_rows(const LargeArgs& la, int N, dim3 grid, cudaStream_t stream)
 template <typename T, int THREADS>
 int launch_large_t(const DrawArgs& args, int N, void* work, size_t work_bytes, cudaStream_t stream)
 {
+    if (!block_fft_has(N, THREADS)) return set_error(GSB_ERR_UNSUPPORTED, "FFT size not built");
     const size_t slab = slab_bytes<T>(N);
     if (!work || work_bytes < slab) return set_error(GSB_ERR_INVALID, "draw workspace too small");
     const size_t base = large_smem<T>() + sizeof(Cx<T>) * ((fft_buf_len<T>(N) + 1) & ~size_t(1));

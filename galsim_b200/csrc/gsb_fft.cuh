@@ -165,12 +165,13 @@ __device__ inline void fill_twiddles(Cx<T>* tw, int N)
 // Block-wide length-N DFT (N = 2^a or 3 * 2^a) in shared memory, Stockham order, N and the thread
 // count known at compile time so that every index is a shift or a constant: radix 8 (4 and 2 for the
 // rest of the power of two), the factor 3 last.  Up to N = 1024, where a bucket may also run the fused
-// kernel, warp_fft_io's radix plan and twiddles, so that both give the same bits.  The first pass takes its inputs from load(i) and
-// the last hands its outputs to store(i, value), so that a caller can read from or write to memory
-// without a trip through the buffer.  tw: exp(+2 pi i m / N), m < N, in T (global).  A radix-8
-// butterfly reads all seven twiddles: three read and the others multiplied from them are 8 % faster
-// (six stamps of N = 4096 .. 8192: device time 5.7 ms against 6.2) but lose accuracy (float, N = 4096:
-// rms error against double 6.0e-9 of the peak against 4.1e-9).
+// kernel, warp_fft_io's radix plan and twiddles, so that both give the same bits.  The first pass takes
+// its inputs from load(i) and the last hands its outputs to store(i, value), so that a caller can read from
+// or write to memory without a trip through the buffer.  tw: exp(+2 pi i m / N), m < N, in T (global).  A
+// radix-8 butterfly reads all seven twiddles: three read and the others multiplied from them are 8 % faster
+// (six stamps of N = 4096 .. 8192: device time 5.7 ms against 6.2) but half as exact again (float).  As it is
+// the transform is as exact as the radix-4 plan: rms error of a float transform 1.17e-7 .. 1.28e-7 of its rms
+// at N = 2048 .. 8192, against 1.15e-7 .. 1.26e-7 (emulated, random and decaying inputs).
 // Between passes the values lie padded by one in 16 (8 in double), which spreads a radix-8 butterfly's
 // adjacent outputs over the banks (16 lanes would share one otherwise): buf holds fft_buf_len values.
 // LOAD_BUF / STORE_BUF: load / store address `buf` itself (their pass then waits for the block
@@ -250,6 +251,15 @@ __device__ __noinline__ void block_fft_out(Cx<T>* buf, const Cx<T>* __restrict__
     block_fft_pass<T, N, THREADS, 1, +1, true, false>(buf, tw, [&](int i) { return buf[i]; },
                                                       [&](int i, Cx<T> z) { out[i] = z; });
     __syncthreads();
+}
+
+// Whether block_fft_any transforms length N with that many threads (asked on the host before a launch).
+__host__ __device__ constexpr bool block_fft_has(int N, int threads)
+{
+    int m = N;
+    while (m > 1 && m % 2 == 0) m /= 2;
+    if (m != 1 && m != 3) return false;
+    return threads == 256 ? N >= 192 && N <= 1024 : threads == 512 ? N >= 1536 && N <= 8192 : threads == 1024 && N >= 1536 && N <= 16384;
 }
 
 // The sizes of the split path, one instantiation each (N uniform over the block).  OUT: to `out`.

@@ -124,13 +124,6 @@ __device__ __forceinline__ double exp_tab(double x)
     return exp_tab_core(x);
 }
 
-// exp(x) for x <= 0 without a branch: arguments below -708 give exp(-708) ~ 3e-308 instead
-// of 0 (the quadrature's terms that reach them are far below its stopping threshold).
-__device__ __forceinline__ double exp_tab_neg(double x, const double* tab = kExp2Tab)
-{
-    return exp_tab_core(fmax(x, -708.), tab);
-}
-
 // ---------------------------------------------------------------------------------------
 // Digamma psi(x) = d ln Gamma / dx for x > 0: the recurrence psi(x) = psi(x + 1) - 1/x
 // (A&S 6.3.5) up to x >= 10, then the asymptotic series

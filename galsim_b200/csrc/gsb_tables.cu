@@ -31,13 +31,13 @@ constexpr int kLevMax = 20;
 constexpr long long kNroot = 1000000;
 
 // 2^(j/256), j = 0..255, correctly rounded (computed on the host in extended precision by
-// ogata_init): the exponential table of the quadrature kernels' exp_tab256_core.
+// ogata_init): the table of exp_tab256_core.
 __device__ double g_exp2_256[256];
 
 // The same method with a 256-entry table 2^(j/256) (`tab`, correctly rounded, filled by the
 // caller): |r| <= ln2/512, so the degree-4 Taylor polynomial of e^r suffices (truncation
-// < 4e-17 relative), two fused multiply-adds fewer than exp_tab_core.  For the quadrature
-// kernels, which evaluate billions of exponentials per table build.
+// < 4e-17 relative), two fused multiply-adds fewer than exp_tab_core.  Evaluated through
+// gsb_exp_fp64_ex alone.
 __device__ __forceinline__ double exp_tab256_core(double x, const double* tab)
 {
     const double kShift = 6755399441055744.0;               // 1.5 * 2^52
@@ -157,6 +157,7 @@ __device__ double warp_hankel(const OgataTables& og, const F& f, double k, doubl
 // samples a smooth G at the scattered ln x_i.  With G band-limited well below pi / h, its value
 // between the points of a grid of spacing h is the windowed-sinc sum
 //     G(u h) = sum_q phi(u - q) G(q h),   phi(t) = sinc(t) exp(beta (sqrt(1 - (2 t / W)^2) - 1)),
+// (the "exponential of semicircle" window of Barnett, Magland and af Klinteberg, SIAM J. Sci. Comput. 41, 2019)
 // so the nodes can be spread onto the grid once and for all, A_l[q] = sum_i w_i phi(ln x_i / h - q),
 // and S_l(k) = sum_q A_l[q] G(q h - ln k): one array of G per profile serves every ln k on the
 // grid and every level, and a term costs one multiply-add instead of an exponential.  The A_l
