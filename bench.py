@@ -557,13 +557,13 @@ def gpu_object(galsim, p):
 # DRAM bytes of one step's draw kernels (ncu, one-pass metrics, this workload at its own
 # automatic sizes; profiles/draw_fused_kernel_dram_bench_step_4096.md): reads, writes, and the
 # global stores the SMs issue (stamps plus the N >= 256 buckets' W slabs, which stay in L2).
-DRAW_STEP_DRAM_READ = 37439488
-DRAW_STEP_DRAM_WRITE = 63917824
+DRAW_STEP_DRAM_READ = 35580160
+DRAW_STEP_DRAM_WRITE = 67625472
 DRAW_STEP_STORES = 285221408
 # FP64 pipe and issue utilisation of the Sersic table kernel (ncu, a 4096-table build;
 # profiles/sersic_table_kernel_4096_tables.md)
-TABLES_FP64_PIPE = 0.276
-TABLES_ISSUE_ACTIVE = 0.340
+TABLES_FP64_PIPE = 0.261
+TABLES_ISSUE_ACTIVE = 0.329
 
 
 TABLE_BUILD_LAUNCHES = 2     # of an untruncated Sersic table build: set-up and tables
