@@ -738,7 +738,7 @@ __device__ __forceinline__ void sersic_points(const LeafT<float>& L, const unsig
         const float lin = fmaf(s, n0.y - n1.y, n1.y);
         float r = quotient(fmaf(s * bb * (-1.f / 6.f), fmaf(aa + h, n0.z, mul_rn(bb + h, n1.z)), lin), k2, inv);
         if (!(k2 >= kmin && k2 < kmax)) {
-            if (k2 >= kmax) r = quotient(fmaf(L.q[5], refined_rsqrt(k2), L.q[4]), k2, inv);
+            if (k2 >= kmax) r = k2 <= 3e38f ? quotient(fmaf(L.q[5], refined_rsqrt(k2), L.q[4]), k2, inv) : 0.f;
             else r = fmaf(k2, fmaf(k2, L.q[3], L.q[2]), 1.f);
         }
         out[v] = r;
@@ -852,10 +852,10 @@ __device__ __forceinline__ T leaf_points(const StampSmem& S, const unsigned char
         } else if (kind == kLeafKolm) {
             // exp(-(k^2)^(5/6)), the power as k^2 times its -1/6th power r, whose error is a sixth of the
             // logarithm's and is then taken out by a Newton step on r^6 k^2 = 1 (the general form's power
-            // has 5/6 of the logarithm's: 1e-7 at k^2 = 4).  Below 1e-30 the value is 1.
+            // has 5/6 of the logarithm's: 1e-7 at k^2 = 4).  Below 1e-30 the value is 1, above 1e30 0; a NaN stays.
 #pragma unroll
             for (int v = 0; v < V; ++v) {
-                const float x = fmaxf(ksq[v], 1e-30f);
+                const float k2 = ksq[v], x = k2 < 1e-30f ? 1e-30f : k2 > 1e30f ? 1e30f : k2;
                 const float r = fast_exp2(fast_log2(x) * (-1.f / 6.f)), r3 = mul_rn(mul_rn(r, r), r);
                 const float y = mul_rn(x, fmaf(mul_rn(r, 1.f / 6.f), fmaf(-mul_rn(x, r3), r3, 1.f), r));
                 out[v] = expf(-y);

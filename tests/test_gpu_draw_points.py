@@ -141,3 +141,19 @@ def test_float_forms_are_as_exact_as_the_general_ones(kind):
                                 for q, d in (('fp32', np.float32), ('fp32', np.float64), ('fp64', np.float64))]
         ratio.append(np.sqrt(np.mean((fast - exact) ** 2) / np.mean((general.astype(np.float32) - exact) ** 2)))
     assert np.exp(np.mean(np.log(ratio))) <= 1.1, ratio
+
+
+@pytest.mark.parametrize('kind', ['kolmogorov', 'sersic', 'exponential'])
+def test_wave_vectors_whose_square_overflows(kind):
+    """A profile so large that k^2 in its units is beyond float's range: its value there is 0, as in double."""
+    from galsim_b200 import _lib
+    big = np.full(2, 1e22)
+    obj = {'kolmogorov': lambda: galsim.Kolmogorov(fwhm=big), 'sersic': lambda: galsim.Sersic(n=1.5, half_light_radius=big),
+           'exponential': lambda: galsim.Exponential(half_light_radius=big)}[kind]()
+    img = []
+    for precision, dt in ((_lib.F32, _lib.F32), (_lib.F64, _lib.F64)):
+        prog = galsim.plan_batch(obj, nx=20, ny=20, scale=0.2).prog
+        n = np.full(2, 64)
+        img.append(prog.draw_stamps(n, n, -10, -10, 20, 20, dt, precision=precision)[0].double().cpu().numpy())
+    assert np.all(np.isfinite(img[0])) and img[1].max() > 0.
+    assert np.abs(img[0] - img[1]).max() <= 1e-6 * img[1].max()
