@@ -297,6 +297,13 @@ def plan_batch(obj, nx=None, ny=None, scale=None, dtype=np.float32, method='fft'
     """Host set-up of draw_batch: drawImage's argument handling and world-to-image transform
     (gsobject.py:1647-1764) applied to the batched object, flattened into a device program.
     `tables` (a galsim_b200._lib.Tables) is reused for the Sersic tables when given."""
+    plan = _plan(obj, nx, ny, scale, dtype, method, area, exptime, gain, offset, use_true_center, precision, tables)
+    plan.prog.upload_ahead()
+    return plan
+
+
+def _plan(obj, nx, ny, scale, dtype, method, area, exptime, gain, offset, use_true_center, precision, tables=None):
+    """plan_batch for a run at once: its records are uploaded by the run."""
     from . import box, compound
     from .compound import _Transform
     from .program import Program
@@ -328,7 +335,6 @@ def plan_batch(obj, nx=None, ny=None, scale=None, dtype=np.float32, method='fft'
         prof = compound.Convolve(prof, box.Pixel(scale=1.0, gsparams=obj.gsparams),
                                  real_space=False, gsparams=obj.gsparams)
     prog = Program(prof, tables=tables)
-    prog.upload_ahead()
     plan = BatchPlan(prog, nx, ny, nx is not None, flux_scale, dtype, scale, precision)
     # 'no_pixel' / 'sb' on a profile analytic in real space is drawn in real space, as
     # drawImage does (gsobject.py:1810-1811)
@@ -414,8 +420,7 @@ def draw_batch(obj, nx=None, ny=None, scale=None, dtype=np.float32, method='fft'
                                                 bandpass=bandpass)
         return draw_batch_chromatic(obj, bandpass, nx, ny, scale, dtype, method, area, exptime, gain,
                                     offset, use_true_center, precision, integrator)
-    return run_batch(plan_batch(obj, nx, ny, scale, dtype, method, area, exptime, gain, offset,
-                                use_true_center, precision))
+    return run_batch(_plan(obj, nx, ny, scale, dtype, method, area, exptime, gain, offset, use_true_center, precision))
 
 
 def draw_batches(objects, nx=None, ny=None, scale=None, dtype=np.float32, method='fft', area=1.,
